@@ -58,6 +58,10 @@ extern "C" {
 #define LBMAN_FP32 1 /* FP32 compute, populations stored as f_i - w_i*rho0    */
 #define LBMAN_FP16 2 /* FP32 compute, populations stored as FP16 deviations   */
 /* Kernel organisation. */
+/* AUTO: the split organisation (two points per thread where its 30-wide tiles
+ * fit); a whole box in the size range where they are faster is stepped with
+ * the shared-memory-free kernels, which do the same arithmetic bit for bit,
+ * until a shape is set.                                                     */
 #define LBMAN_KERNELS_AUTO 0
 #define LBMAN_KERNELS_SPLIT 1 /* Q+force kernel, then LBM kernel               */
 #define LBMAN_KERNELS_FUSED 2 /* one kernel per time step                      */
@@ -228,8 +232,10 @@ int lbman_get_shape(lbman_solver* s, lbman_shape* out);
  * zchunk >= -8).                                                           */
 int lbman_set_shape(lbman_solver* s, const lbman_shape* shape);
 /* Autotuner (no counterpart in the reference): times steps_per_trial steps
- * of every kernel organisation x compiled tile x z-chunk candidate on the
- * current state with CUDA events, keeps the fastest and restores the state
+ * of every kernel organisation x compiled tile x z-chunk candidate, and of the
+ * shared-memory-free kernels of an AUTO handle (for which best holds the
+ * handle's own shape), on the current state with CUDA events, keeps the
+ * fastest and restores the state
  * it started from bit for bit (a temporary device copy of the fields is
  * taken for that).  ntrials (may be NULL) receives the number of candidates
  * timed.                                                                    */

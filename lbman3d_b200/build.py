@@ -6,6 +6,7 @@ Translation units and their flags:
   kernels_f64.cu  --fmad=false  (FP64 path, bitwise parity with the reference)
   kernels_f32.cu  default contraction (FP32 path)
   kernels_f16.cu  default contraction (FP16 population storage)
+  kernels_point*.cu  the shared-memory-free time step, per precision
   api.cu          host C ABI
   ens_api.cu      ensemble runner
   noalloc.cu      allocation-free flow diagnostics
@@ -36,6 +37,9 @@ UNITS = {
     "kernels_f64.cu": ["--fmad=false"],
     "kernels_f32.cu": [],
     "kernels_f16.cu": [],
+    "kernels_point.cu": [],
+    "kernels_point_f16.cu": [],
+    "kernels_point_f64.cu": ["--fmad=false"],
     "kernels_ens.cu": [],
     "kernels_ens_f64.cu": ["--fmad=false"],
     "api.cu": [],

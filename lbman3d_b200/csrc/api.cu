@@ -68,13 +68,17 @@ struct Ops {
     decltype(&launch_seeded_init_f64) seeded_init;
     decltype(&launch_qsetup_f64) qsetup;
     decltype(&launch_active_force_f64) active_force;
+    decltype(&launch_qpoint_f64) qpoint;
+    decltype(&launch_point_force_f64) point_force;
+    decltype(&launch_lbm_aa_point_f64) lbm_aa_point;
     decltype(&qforce_smem_f64) qforce_smem;
     decltype(&qforce_threads_f64) qforce_threads;
     decltype(&march_blocks_f64) march_blocks;
     decltype(&prepare_f64) prepare;
 };
 
-#define LBMAN_OPS(SUF)                                                                                 \
+// QSUF: the suffix of the Q stage's point kernels (FP16 storage computes in FP32)
+#define LBMAN_OPS(SUF, QSUF)                                                                               \
     Ops {                                                                                              \
         launch_qforce_##SUF, launch_fused_##SUF, launch_lbm_##SUF, launch_stream_only_##SUF,           \
             launch_lbm_aa_##SUF, launch_aa_pop_out_##SUF, launch_swap_pairs_##SUF,                     \
@@ -83,10 +87,11 @@ struct Ops {
             launch_real_out_##SUF, launch_flow_reduce_##SUF, launch_energy_reduce_##SUF,               \
             launch_director_##SUF, launch_defect_count_##SUF, launch_defect_flags_##SUF,              \
             launch_seeded_init_##SUF, launch_qsetup_##SUF, launch_active_force_##SUF,                  \
+            launch_qpoint_##QSUF, launch_point_force_##QSUF, launch_lbm_aa_point_##SUF,                \
             qforce_smem_##SUF, qforce_threads_##SUF, march_blocks_##SUF, prepare_##SUF                 \
     }
 
-const Ops kOps[3] = {LBMAN_OPS(f64), LBMAN_OPS(f32), LBMAN_OPS(f16)};
+const Ops kOps[3] = {LBMAN_OPS(f64, f64), LBMAN_OPS(f32, f32), LBMAN_OPS(f16, f32)};
 
 // AnchoredQ (src/boundary_handler.h:232-251), evaluated on the host.
 void anchored_q(const lbman_face& f, double out[5]) {
@@ -160,6 +165,10 @@ struct lbman_solver {
     void* u[2] = {nullptr, nullptr};
     void* rho = nullptr;
     void* F = nullptr;
+    // Point organisation (qpoint.cuh): steps run without the z-marching Q
+    // kernel; pstress holds the stress between its two kernels.
+    bool point = false;
+    void* pstress = nullptr;
     void* stress = nullptr;  // Sigma (5) and tau (3) of the two-phase Q stage, allocated on first use
     double* staging = nullptr;
     double* partials = nullptr;
@@ -219,6 +228,24 @@ int default_zchunk(int nx, int ny, int nz, int tcx, int tcy, int num_sms) {
     nchunks = std::max(nchunks, (long)((nz + 255) / 256));
     return (int)((nz + nchunks - 1) / nchunks);
 }
+
+// Largest box (cells) an untuned AUTO handle steps with the point kernels
+// (qpoint.cuh), whole steps timed on B200 against the z-marching kernels:
+//   FP64             faster at every size tried (32^3 67 -> 12 us, 256^3 2865 ->
+//                    2100 us); the kernels index 15 V in 32 bits
+//   FP32, one point  64x256x256 slit 280 -> 248 us, 256^3 939 -> 969 us
+//   FP32, packed     120x128x128 Q stage 102 -> 80 us; 256^3 541 -> 512 us alone,
+//                    but the FP16 step there 1.00 -> 1.02 ms (the stress is 72 B
+//                    of HBM traffic per cell)
+int64_t point_limit(int prec) {
+    if (prec == LBMAN_FP64) return (((int64_t)1 << 31) - 1) / 15;
+    return (int64_t)8 << 20;
+}
+
+// Up to this size the LBM kernel forms the body force itself (one launch and
+// the force's round trip less); above it a force kernel runs before the LBM
+// step (FP32 64x256x256: 248 us fused, 264 us apart; 256^3: 995 and 969 us).
+constexpr int64_t kPointFusedCells = (int64_t)6 << 20;
 
 // Default z-marching tile before any autotuning: the widest compiled tile
 // up to 32 cells whose last partial tile pads x by at most 10% (wide rows
@@ -444,6 +471,16 @@ int lbman_create(const lbman_config* cfg, lbman_solver** out) {
         if (int st = alloc(&s->q[b], 5 * V * s->rbytes)) return bail(st);
         if (int st = alloc(&s->u[b], 3 * V * s->rbytes)) return bail(st);
     }
+    if (cfg->kernels == LBMAN_KERNELS_AUTO && cfg->tile_x == 0 && cfg->tile_y == 0 && cfg->zchunk == 0 &&
+        V <= point_limit(s->prec)) {
+        // 9 row-stress words (FP32) or Sigma and tau (FP64) per cell; a box that
+        // has no room for them keeps the z-marching kernels
+        s->point = cudaMalloc(&s->pstress, (s->prec == LBMAN_FP64 ? 8 : 9) * V * s->rbytes) == cudaSuccess;
+        if (!s->point) {
+            cudaGetLastError();
+            s->pstress = nullptr;
+        }
+    }
     if (int st = alloc(&s->rho, V * s->rbytes)) return bail(st);
     if (int st = alloc(&s->F, 3 * V * s->rbytes)) return bail(st);
     // FP64 host staging too: downloads of an in-place-layout state gather
@@ -467,7 +504,7 @@ int lbman_destroy(lbman_solver* s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     for (int b = 0; b < 2; ++b) { cudaFree(s->f[b]); cudaFree(s->q[b]); cudaFree(s->u[b]); }
     cudaFree(s->rho); cudaFree(s->F); cudaFree(s->staging); cudaFree(s->partials); cudaFree(s->red_dev);
-    cudaFree(s->upast); cudaFree(s->dirbuf); cudaFree(s->stress); cudaFree(s->fstage);
+    cudaFree(s->upast); cudaFree(s->dirbuf); cudaFree(s->stress); cudaFree(s->pstress); cudaFree(s->fstage);
     if (s->ev_ready) cudaEventDestroy(s->ev_ready);
     if (s->ev_done) cudaEventDestroy(s->ev_done);
     lbman::stats::destroy(s->stats);
@@ -642,17 +679,42 @@ static int ensure_f1(lbman_solver* s) {
     return LBMAN_OK;
 }
 
-// In-place LBM step (AA pattern): even from F_PRE, odd from F_SWAP; a
-// two-buffer post-collision state is first put in the in-place layout.
-static int aa_step(lbman_solver* s, bool last) {
-    const Ops& o = s->ops();
+// A two-buffer post-collision state is put in the in-place layout.
+static int aa_layout(lbman_solver* s) {
     if (s->fphase == F_POST) {
-        LB_TRY(check_launch(s, o.swap_pairs(s->P, s->f[s->fcur], s->stream), "swap_pairs"));
+        LB_TRY(check_launch(s, s->ops().swap_pairs(s->P, s->f[s->fcur], s->stream), "swap_pairs"));
         s->fphase = F_SWAP;
     }
+    return LBMAN_OK;
+}
+
+// In-place LBM step (AA pattern): even from F_PRE, odd from F_SWAP.
+static int aa_step(lbman_solver* s, bool last) {
+    const Ops& o = s->ops();
+    LB_TRY(aa_layout(s));
     const bool odd = s->fphase == F_SWAP;
     LB_TRY(check_launch(s, o.lbm_aa(s->P, odd, last, s->f[s->fcur], s->F, s->rho, s->u[s->ucur], s->stream), "lbm_aa"));
     s->fphase = odd ? F_PRE : F_SWAP;
+    return LBMAN_OK;
+}
+
+// The Q stage: Q_new, and the body force in s->F (force: formed here rather
+// than by the LBM step that follows).
+static int q_stage(lbman_solver* s, bool force) {
+    const Ops& o = s->ops();
+    if (s->point) {
+        const bool pair = s->kernels == LBMAN_KERNELS_SPLIT_PAIR;
+        LB_TRY(check_launch(s, o.qpoint(s->P, pair, s->num_sms, s->q[s->qcur], s->u[s->ucur], s->q[1 - s->qcur],
+                                        s->pstress, s->F, s->stream),
+                            "qpoint"));
+        if (force)
+            LB_TRY(check_launch(s, o.point_force(s->P, pair, s->q[1 - s->qcur], s->pstress, s->u[s->ucur], s->F, s->stream),
+                                "point_force"));
+    } else {
+        LB_TRY(check_launch(s, o.qforce(s->P, s->shape, s->q[s->qcur], s->u[s->ucur], s->q[1 - s->qcur], s->F, s->stream),
+                            "qforce"));
+    }
+    s->qcur ^= 1;
     return LBMAN_OK;
 }
 
@@ -674,10 +736,16 @@ static int one_step(lbman_solver* s, bool last) {
         s->ucur ^= 1;
         s->fcur ^= 1;
         s->fphase = F_POST;
+    } else if (s->point && s->P.V <= kPointFusedCells) {
+        LB_TRY(q_stage(s, false));
+        LB_TRY(aa_layout(s));
+        const bool odd = s->fphase == F_SWAP;
+        LB_TRY(check_launch(s, o.lbm_aa_point(s->P, s->kernels == LBMAN_KERNELS_SPLIT_PAIR, odd, last, s->f[s->fcur],
+                                              s->q[s->qcur], s->pstress, s->F, s->rho, s->u[s->ucur], s->stream),
+                            "lbm_aa_point"));
+        s->fphase = odd ? F_PRE : F_SWAP;
     } else {
-        LB_TRY(check_launch(s, o.qforce(s->P, s->shape, s->q[s->qcur], s->u[s->ucur], s->q[1 - s->qcur], s->F, s->stream),
-                            "qforce"));
-        s->qcur ^= 1;
+        LB_TRY(q_stage(s, true));
         LB_TRY(aa_step(s, last));
     }
     ++s->steps;
@@ -701,9 +769,7 @@ int lbman_qtensor_step(lbman_solver* s) {
         return fail(LBMAN_ERR_STATE, s->fout_pending ? "exchange LBMAN_HALO_F_OUT after the odd LBM step first"
                                                      : "exchange LBMAN_HALO_QU before the Q stage of a slab");
     LB_TRY(set_device(s));
-    LB_TRY(check_launch(s, s->ops().qforce(s->P, s->shape, s->q[s->qcur], s->u[s->ucur], s->q[1 - s->qcur], s->F, s->stream),
-                        "qforce"));
-    s->qcur ^= 1;
+    LB_TRY(q_stage(s, true));
     s->qu_fresh = false;
     return LBMAN_OK;
 }
@@ -942,6 +1008,7 @@ int lbman_set_shape(lbman_solver* s, const lbman_shape* sh) {
         return fail(LBMAN_ERR_ARG, "tile %dx%d is not compiled for this precision%s", sh->tile_x, sh->tile_y,
                     t.pair ? " and organisation" : "");
     s->kernels = sh->kernels;
+    s->point = false;  // a shape names a z-marching launch
     s->shape.tile = t;
     s->shape.qthreads = s->ops().qforce_threads(t);
     return LBMAN_OK;
@@ -989,13 +1056,20 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
     int status = LBMAN_OK, count = 0;
     lbman_shape orig, cur{}, win{};
     std::vector<lbman_shape> trials;
+    const bool point0 = s->point;
+    double point_ms = 1e30;
     lbman_get_shape(s, &orig);
     win = orig;
     win.ms_per_step = 1e30;
     if (copy_state(true) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
         status = fail(LBMAN_ERR_CUDA, "autotune set-up failed");
     } else {
+        if (point0) {  // the point kernels have no shape: one trial, at the length of the final ones
+            status = time_trial(s, 3 * steps_per_trial, e0, e1, &point_ms);
+            ++count;
+        }
         for (int k : {LBMAN_KERNELS_SPLIT, LBMAN_KERNELS_FUSED, LBMAN_KERNELS_SPLIT_PAIR}) {
+            if (status != LBMAN_OK) break;
             if (k == LBMAN_KERNELS_SPLIT_PAIR && (s->prec == LBMAN_FP64 || (s->P.nx & 3) != 0)) continue;
             // the fused organisation needs a second population buffer; a box
             // too large for it is tuned over the in-place organisations only
@@ -1046,9 +1120,15 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
     cudaFree(snap);
     if (status != LBMAN_OK) {
         lbman_set_shape(s, &orig);
+        s->point = point0;
         return status;
     }
+    if (point_ms <= win.ms_per_step) {
+        win = orig;
+        win.ms_per_step = point_ms;
+    }
     lbman_set_shape(s, &win);
+    s->point = point_ms <= win.ms_per_step;
     lbman_get_shape(s, best);
     best->ms_per_step = win.ms_per_step;
     if (ntrials) *ntrials = count;
@@ -1077,6 +1157,9 @@ int lbman_create_slab(const lbman_config* cfg, int nz_global, int z_offset, lbma
     lbman_solver* s = nullptr;
     LB_TRY(lbman_create(&c, &s));
     s->slab = true;
+    s->point = false;  // the point kernels cover whole boxes
+    cudaFree(s->pstress);
+    s->pstress = nullptr;
     s->nz_global = nz_global;
     s->z_offset = z_offset;
     SimParams& P = s->P;

@@ -61,6 +61,14 @@ struct LaunchShape {
                                     void* sig, void* tau, void* F, cudaStream_t st);                   \
     cudaError_t launch_active_force_##SUF(const SimParams& P, const void* q, const void* sig,           \
                                           const void* tau, const void* u, void* F, cudaStream_t st);   \
+    cudaError_t launch_qpoint_##SUF(const SimParams& P, bool pair, int num_sms, const void* qin,        \
+                                    const void* uin, void* qout, void* stress, void* F,                \
+                                    cudaStream_t st);                                                  \
+    cudaError_t launch_point_force_##SUF(const SimParams& P, bool pair, const void* qn,                 \
+                                         const void* stress, const void* u, void* F, cudaStream_t st); \
+    cudaError_t launch_lbm_aa_point_##SUF(const SimParams& P, bool pair, bool odd, bool last, void* f,  \
+                                          const void* qn, const void* stress, void* F, void* rho,      \
+                                          void* u, cudaStream_t st);                                   \
     size_t qforce_smem_##SUF(const QTile& T);                                                          \
     int qforce_threads_##SUF(const QTile& T);                                                          \
     int march_blocks_##SUF(const SimParams& P, const LaunchShape& shape, bool fused_org);              \

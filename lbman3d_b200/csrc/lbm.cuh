@@ -401,22 +401,49 @@ __device__ __forceinline__ void crossing(const SimParams& P, const AxisOff<I>& o
     cz = (WM & 4) && ez_(j) != 0 && !P.uper[4] && ((ez_(j) > 0 && o.loz) || (ez_(j) < 0 && o.hiz));
 }
 
-template <class R, class S, bool DEV, int WM, class I>
-__global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
-    lbm_aa_even_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, S* F, const R* __restrict__ Fb,
-                       R* __restrict__ rho_buf, R* __restrict__ uout, int write_rho_all) {
-    const I c = (I)P.c0 + (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
-    if (c >= (I)P.c1) return;
+// The body force of a cell read from its array.
+template <class R, class I>
+struct LoadForce {
+    static constexpr bool kNeedsPos = false;
+    const R* __restrict__ Fb;
+    I V;
+    __device__ __forceinline__ void operator()(I c, const CellPos&, R F[3]) const {
+        F[0] = Fb[c];
+        F[1] = Fb[V + c];
+        F[2] = Fb[2 * V + c];
+    }
+};
+
+template <class I>
+__device__ __forceinline__ CellPos cell_pos(const SimParams& P, I c, const FastDiv& dnx, const FastDiv& dnxy) {
+    CellPos q;
+    q.z = (int)fdiv((uint32_t)c, dnxy);
+    const uint32_t r = (uint32_t)((int64_t)c - (int64_t)q.z * P.nxy);
+    q.y = (int)fdiv(r, dnx);
+    q.x = (int)(r - (uint32_t)q.y * (uint32_t)P.nx);
+    return q;
+}
+
+// Even and odd in-place step of cell c; force(c, position, F) gives the body
+// force (read from memory, or formed from the stress in qpoint.cuh).
+template <class R, class S, bool DEV, int WM, class I, class Force>
+__device__ __forceinline__ void aa_even_cell(const SimParams& P, const FastDiv& dnx, const FastDiv& dnxy, I c, S* F,
+                                             const Force& force, R* __restrict__ rho_buf, R* __restrict__ uout,
+                                             int write_rho_all) {
     const I V = (I)P.V;
     const Phys<R>& K = phys_ref<R>(P);
     S raw[15];
 #pragma unroll
     for (int j = 0; j < 15; ++j) raw[j] = F[j * V + c];
+    CellPos q{0, 0, 0};
+    if constexpr (Force::kNeedsPos) q = cell_pos<I>(P, c, dnx, dnxy);
+    R Fc[3];
+    force(c, q, Fc);
     R f[15];
 #pragma unroll
     for (int j = 0; j < 15; ++j) f[j] = Store<S>::widen(raw[j]);
     R rho, ux, uy, uz;
-    collide<R, DEV>(K, f, Fb[c], Fb[V + c], Fb[2 * V + c], rho, ux, uy, uz);
+    collide<R, DEV>(K, f, Fc[0], Fc[1], Fc[2], rho, ux, uy, uz);
 #pragma unroll
     for (int j = 0; j < 15; ++j) Store<S>::st(F + opp_(j) * V + c, f[j]);
     uout[c] = ux;
@@ -424,29 +451,19 @@ __global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
     uout[2 * V + c] = uz;
     bool mv = false;
     if (WM != 0 && P.moving_any && !write_rho_all) {
-        CellPos q;
-        q.z = (int)fdiv((uint32_t)c, dnxy);
-        const uint32_t r = (uint32_t)((int64_t)c - (int64_t)q.z * P.nxy);
-        q.y = (int)fdiv(r, dnx);
-        q.x = (int)(r - (uint32_t)q.y * (uint32_t)P.nx);
+        if constexpr (!Force::kNeedsPos) q = cell_pos<I>(P, c, dnx, dnxy);
         mv = touches_moving(P, q.x, q.y, q.z);
     }
     if (write_rho_all || mv) rho_buf[c] = rho;
 }
 
-template <class R, class S, bool DEV, int WM, class I>
-__global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
-    lbm_aa_odd_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, S* F, const R* __restrict__ Fb,
-                      R* __restrict__ rho_buf, R* __restrict__ uout, int write_rho_all) {
-    const I c = (I)P.c0 + (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
-    if (c >= (I)P.c1) return;
+template <class R, class S, bool DEV, int WM, class I, class Force>
+__device__ __forceinline__ void aa_odd_cell(const SimParams& P, const FastDiv& dnx, const FastDiv& dnxy, I c, S* F,
+                                            const Force& force, R* __restrict__ rho_buf, R* __restrict__ uout,
+                                            int write_rho_all) {
     const I V = (I)P.V;
     const Phys<R>& K = phys_ref<R>(P);
-    CellPos q;
-    q.z = (int)fdiv((uint32_t)c, dnxy);
-    const uint32_t r = (uint32_t)((int64_t)c - (int64_t)q.z * P.nxy);
-    q.y = (int)fdiv(r, dnx);
-    q.x = (int)(r - (uint32_t)q.y * (uint32_t)P.nx);
+    const CellPos q = cell_pos<I>(P, c, dnx, dnxy);
     const AxisOff<I> o = axis_off<I>(P, q);
     constexpr bool WALLS = WM != 0;
     const bool mv = WALLS && P.moving_any && touches_moving(P, q.x, q.y, q.z);
@@ -466,6 +483,8 @@ __global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
             raw[j] = F[src];
         }
     }
+    R Fc[3];
+    force(c, q, Fc);
     R f[15];
 #pragma unroll
     for (int j = 0; j < 15; ++j) f[j] = Store<S>::widen(raw[j]);
@@ -481,7 +500,7 @@ __global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
         }
     }
     R rho, ux, uy, uz;
-    collide<R, DEV>(K, f, Fb[c], Fb[V + c], Fb[2 * V + c], rho, ux, uy, uz);
+    collide<R, DEV>(K, f, Fc[0], Fc[1], Fc[2], rho, ux, uy, uz);
     // scatter
 #pragma unroll
     for (int k = 0; k < 15; ++k) {
@@ -514,6 +533,24 @@ __global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
     uout[V + c] = uy;
     uout[2 * V + c] = uz;
     if (write_rho_all || mv) rho_buf[c] = rho;
+}
+
+template <class R, class S, bool DEV, int WM, class I>
+__global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
+    lbm_aa_even_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, S* F, const R* __restrict__ Fb,
+                       R* __restrict__ rho_buf, R* __restrict__ uout, int write_rho_all) {
+    const I c = (I)P.c0 + (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
+    if (c >= (I)P.c1) return;
+    aa_even_cell<R, S, DEV, WM, I>(P, dnx, dnxy, c, F, LoadForce<R, I>{Fb, (I)P.V}, rho_buf, uout, write_rho_all);
+}
+
+template <class R, class S, bool DEV, int WM, class I>
+__global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
+    lbm_aa_odd_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, S* F, const R* __restrict__ Fb,
+                      R* __restrict__ rho_buf, R* __restrict__ uout, int write_rho_all) {
+    const I c = (I)P.c0 + (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
+    if (c >= (I)P.c1) return;
+    aa_odd_cell<R, S, DEV, WM, I>(P, dnx, dnxy, c, F, LoadForce<R, I>{Fb, (I)P.V}, rho_buf, uout, write_rho_all);
 }
 
 // ---- in-place streaming, FP16 storage, two cells per thread ---------------

@@ -1,0 +1,131 @@
+// point_launch.cuh -- launchers of the qpoint.cuh kernels, instantiated by
+// kernels_point.cu (FP32), kernels_point_f16.cu (FP16 storage: the LBM step
+// only) and kernels_point_f64.cu.
+#pragma once
+
+#include "launch.h"
+#include "qpoint.cuh"
+
+#include <algorithm>
+
+namespace lbman {
+namespace impl {
+
+// The compiled wall-rule masks, each a superset of the ones before: none, x
+// walls (slit), x and y walls (channel), everything.
+inline int point_mask(const SimParams& P) {
+    int m = 0;
+    for (int ax = 0; ax < 3; ++ax) {
+        if (!(P.qper[2 * ax] && P.qper[2 * ax + 1] && P.uper[2 * ax] && P.uper[2 * ax + 1])) m |= 1 << ax;
+        for (int f = 2 * ax; f < 2 * ax + 2; ++f)
+            if (P.face[f].qbc == Q_ANCHORING) m |= QW_ANCHOR;
+    }
+    return m == 0 ? 0 : m == QW_X ? QW_X : (m & ~(QW_X | QW_Y)) == 0 ? QW_X | QW_Y : 15;
+}
+template <class F>
+void with_mask(int m, F&& f) {
+    if (m == 0) f(std::integral_constant<int, 0>{});
+    else if (m == QW_X) f(std::integral_constant<int, QW_X>{});
+    else if (m == (QW_X | QW_Y)) f(std::integral_constant<int, QW_X | QW_Y>{});
+    else f(std::integral_constant<int, 15>{});
+}
+
+// Planes per thread: the longest walk (at most 4, where the gain ends) that
+// still gives 16 blocks per SM.
+inline int point_walk(int64_t nxy, int nz, int cells_per_block, int num_sms) {
+    const int64_t cols = (nxy + cells_per_block - 1) / cells_per_block;
+    int zc = 4;
+    while (zc > 1 && cols * ((nz + zc - 1) / zc) < (int64_t)16 * num_sms) zc /= 2;
+    return std::min(zc, nz);
+}
+
+template <class R>
+cudaError_t qpoint(const SimParams& P, bool pair, int num_sms, const void* qin, const void* uin, void* qout,
+                   void* stress, void* F, cudaStream_t st) {
+    const FastDiv dnx = make_fastdiv((uint32_t)P.nx);
+    const int per_block = kPointThreads * (pair ? 2 : 1);
+    const int zc = point_walk(P.nxy, P.nz, per_block, num_sms);
+    const dim3 g((unsigned)((P.nxy + per_block - 1) / per_block), (unsigned)((P.nz + zc - 1) / zc));
+    auto launch = [&](auto k) {
+        k<<<g, kPointThreads, 0, st>>>(P, dnx, zc, (const R*)qin, (const R*)uin, (R*)qout, (R*)stress, (R*)F);
+    };
+    with_mask(point_mask(P), [&](auto m) {
+        constexpr int QW = decltype(m)::value;
+        if constexpr (sizeof(R) == 4) {
+            if (pair) {
+                if (P.upwind) launch(qpoint2_kernel<true, QW>);
+                else launch(qpoint2_kernel<false, QW>);
+                return;
+            }
+        }
+        if (P.upwind) launch(qpoint_kernel<R, true, QW>);
+        else launch(qpoint_kernel<R, false, QW>);
+    });
+    return cudaGetLastError();
+}
+
+template <class R>
+cudaError_t point_force(const SimParams& P, bool pair, const void* qn, const void* stress, const void* u, void* F,
+                        cudaStream_t st) {
+    const FastDiv dnx = make_fastdiv((uint32_t)P.nx), dnxy = make_fastdiv((uint32_t)P.nxy);
+    const unsigned nb = (unsigned)((P.V + 255) / 256);
+    with_mask(point_mask(P), [&](auto m) {
+        constexpr int QW = decltype(m)::value;
+        if constexpr (sizeof(R) == 4) {
+            if (pair) {
+                point_force_kernel<R, QW, true><<<nb, 256, 0, st>>>(P, dnx, dnxy, (const R*)qn, (const R*)stress,
+                                                                    (const R*)u, (R*)F);
+                return;
+            }
+        }
+        point_force_kernel<R, QW><<<nb, 256, 0, st>>>(P, dnx, dnxy, (const R*)qn, (const R*)stress, (const R*)u, (R*)F);
+    });
+    return cudaGetLastError();
+}
+
+template <class R, class S, bool DEV>
+cudaError_t lbm_aa_point(const SimParams& P, bool pair, bool odd, bool last, void* f, const void* qn,
+                         const void* stress, void* F, void* rho, void* u, cudaStream_t st) {
+    const FastDiv dnx = make_fastdiv((uint32_t)P.nx), dnxy = make_fastdiv((uint32_t)P.nxy);
+    const unsigned nb = (unsigned)((P.V + kPointThreads - 1) / kPointThreads);
+    auto launch = [&](auto k) {
+        k<<<nb, kPointThreads, 0, st>>>(P, dnx, dnxy, (S*)f, (const R*)qn, (const R*)stress, (R*)F, (R*)rho, (R*)u,
+                                        last ? 1 : 0);
+    };
+    with_mask(point_mask(P), [&](auto m) {
+        constexpr int QW = decltype(m)::value, WM = QW & 7;
+        if constexpr (sizeof(R) == 4) {
+            if (pair) {
+                if (odd) launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, true, true>);
+                else launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, false, true>);
+                return;
+            }
+        }
+        if (odd) launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, true>);
+        else launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, false>);
+    });
+    return cudaGetLastError();
+}
+
+}  // namespace impl
+}  // namespace lbman
+
+#define LBMAN_DEFINE_POINT_Q(SUF, R)                                                                              \
+    namespace lbman {                                                                                             \
+    cudaError_t launch_qpoint_##SUF(const SimParams& P, bool pair, int num_sms, const void* qin, const void* uin, \
+                                    void* qout, void* stress, void* F, cudaStream_t st) {                         \
+        return impl::qpoint<R>(P, pair, num_sms, qin, uin, qout, stress, F, st);                                  \
+    }                                                                                                             \
+    cudaError_t launch_point_force_##SUF(const SimParams& P, bool pair, const void* qn, const void* stress,       \
+                                         const void* u, void* F, cudaStream_t st) {                               \
+        return impl::point_force<R>(P, pair, qn, stress, u, F, st);                                               \
+    }                                                                                                             \
+    }
+#define LBMAN_DEFINE_POINT_LBM(SUF, R, S, DEV)                                                                    \
+    namespace lbman {                                                                                             \
+    cudaError_t launch_lbm_aa_point_##SUF(const SimParams& P, bool pair, bool odd, bool last, void* f,            \
+                                          const void* qn, const void* stress, void* F, void* rho, void* u,        \
+                                          cudaStream_t st) {                                                      \
+        return impl::lbm_aa_point<R, S, DEV>(P, pair, odd, last, f, qn, stress, F, rho, u, st);                   \
+    }                                                                                                             \
+    }
