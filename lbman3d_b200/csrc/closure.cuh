@@ -36,6 +36,7 @@ namespace cl {
 
 constexpr int kTileM = 128;
 constexpr int kThreads = 128;
+constexpr int kOutChannels = 8;  // of the network; its output is channel-major, [8][V]
 constexpr int kStages = 4;  // A-operand stages of the convolution pipeline
 
 struct Grid3 {
@@ -58,12 +59,18 @@ __device__ __forceinline__ float gelu_grad(float x) {
 }
 
 // Byte size of the B image of one convolution: 27 taps x CIN/16 k-steps of
-// COUT x 16 K-major BF16 (core matrices: n-group stride 256, k-group 128).
+// COUT x 16 K-major BF16 blocks (core matrices: n-group stride 256, k-group 128).
 __host__ __device__ constexpr int bimg_bytes(int cin, int cout) { return 27 * (cin / 16) * cout * 32; }
+
+// Byte offset in the B image of the COUT x 16 block of (dy, dx) index yx, k-step
+// kb and dz: the three dz of a (yx, kb) are consecutive, +1 first.
+__host__ __device__ constexpr int bimg_off(int cin, int cout, int yx, int kb, int dz) {
+    return ((yx * (cin / 16) + kb) * 3 + (1 - dz)) * cout * 32;
+}
 
 enum ConvMode : int {
     kFwdHidden = 0,  // + bias, store pre (BF16) and GELU(pre) (BF16)
-    kFwdLast = 1,    // + bias, store FP32
+    kFwdLast = 1,    // + bias, store FP32 channel-major
     kBwdData = 2     // times GELU'(pre of the layer below), store BF16
 };
 
@@ -177,7 +184,7 @@ __global__ void __launch_bounds__(kThreads) conv_kernel(Grid3 g, const __nv_bflo
 #pragma unroll
                 for (int kb = 0; kb < KS; ++kb) {
                     const uint64_t da = tc::smem_desc(a0 + s * ABYTES + kb * 4096, 128, 256);
-                    const uint64_t db = tc::smem_desc(b0 + (tap * KS + kb) * COUT * 32, 128, 256);
+                    const uint64_t db = tc::smem_desc(b0 + bimg_off(CIN, COUT, tap % 9, kb, tap / 9 - 1), 128, 256);
                     tc::mma_bf16(tmem, da, db, idesc, (tap > 0 || kb > 0) ? 1u : 0u);
                 }
                 tc::mma_commit(&bar[s]);
@@ -213,10 +220,7 @@ __global__ void __launch_bounds__(kThreads) conv_kernel(Grid3 g, const __nv_bflo
                 }
             } else if constexpr (MODE == kFwdLast) {
 #pragma unroll
-                for (int j = 0; j < COUT; j += 4)
-                    reinterpret_cast<float4*>(out_f + c * COUT)[j / 4] =
-                        make_float4(acc[j] + bias[j], acc[j + 1] + bias[j + 1], acc[j + 2] + bias[j + 2],
-                                    acc[j + 3] + bias[j + 3]);
+                for (int j = 0; j < kOutChannels; ++j) out_f[j * g.V + c] = acc[j] + bias[j];
             } else {
                 __align__(16) __nv_bfloat16 pre[COUT], gb[COUT];
 #pragma unroll
@@ -247,41 +251,51 @@ __global__ void __launch_bounds__(kThreads) conv_kernel(Grid3 g, const __nv_bflo
 // Tile = 8 x-cells by 16 y-rows of one z plane (128 cells, M row m = 8*dy_row
 // + dx_cell).  A CTA takes a column of tiles (the same 8 x 16 block of every
 // plane of a z range) and marches it in z.  The column's neighbourhood is
-// staged plane by plane (10 x 18 cells per plane) in a ring of 5 plane slots,
+// staged plane by plane (10 x 18 cells per plane) in a ring of 3 plane slots,
 // as 16-byte units, one block per 8-channel group:
 //   unit(slot, kg, hy, hx) at slot*SLOT + (kg*18 + hy)*10 + hx,
-// which makes the A operand of every tap a K-major view of the ring: rows of
-// a core matrix are 8 consecutive x cells (16 bytes apart), the next y row is
-// SBO = 160 bytes on, the next 8 channels LBO = 2880 bytes on, and the tap
-// (dx, dy, dz) only picks the slot of plane z + dz and moves the start
-// address.  So each tile costs one new plane (the other two are the previous
-// tiles') and 27 x CIN/16 back-to-back MMAs with no operand copies; the copy
-// of a plane is issued two tiles before the tile that first reads it.  The
-// TMEM accumulator is double buffered.  Warps 0-7 copy planes and run the
-// epilogues (warps w and w + 4 read the same TMEM lanes, 32 (w % 4) ..,
-// and split the accumulator's columns); warp 8 issues the MMAs.  So while
-// the tensor core runs tile z, warps 0-7 start copying plane z + 3, finish
-// tile z - 1 and wait for plane z + 2, and warp 8 has queued tile z: one
-// block barrier per tile.
+// which makes the A operand of every (dx, dy) a K-major view of a slot: rows
+// of a core matrix are 8 consecutive x cells (16 bytes apart), the next y row
+// is SBO = 160 bytes on, the next 8 channels LBO = 2880 bytes on, and (dx, dy)
+// only moves the start address.
+//
+// A staged plane is multiplied once, by the weights of all three dz at once:
+// N = 3 COUT columns, the accumulators of the output planes z - 1, z and z + 1,
+// which lie side by side in a ring of plane accumulators in TMEM (NP planes; a
+// window that wraps is issued in two parts).  An MMA costs the same issue time
+// at N = 32 and 64 and little more at 96, so this halves the tensor time
+// against one MMA per tap (9 x CIN/16 instead of 27 x CIN/16 per tile).  The
+// order in which a plane's taps accumulate is that of the taps, (dz, dy, dx).
+//
+// Worker warps copy planes and run the epilogues (warps w, w + 4, .. read the
+// same TMEM lanes, 32 (w % 4) .., and take 8 of the accumulator's columns each);
+// one more warp issues the MMAs.  So while the tensor core runs input plane s,
+// the workers start copying plane s + 2, finish the output plane that plane
+// s - 1 completed and wait for plane s + 1: one block barrier per plane.
 constexpr int kHX = 10, kHY = 18;
-constexpr int kZWorkers = 256;             // copy / epilogue threads
+constexpr int kZWorkers = 256;             // copy threads of the weight gradient
 constexpr int kZThreads = kZWorkers + 32;  // + the MMA warp
 constexpr int kZIssuer = kZWorkers;        // the thread that issues the MMAs
-constexpr int kSlots = 5;
-__host__ __device__ constexpr int ring_slot(int plane) { return (plane + kSlots) % kSlots; }  // plane >= -1
+constexpr int kEpiCols = 8;                // accumulator columns per worker thread
+__host__ __device__ constexpr int conv_workers(int cout) { return kTileM * (cout / kEpiCols); }
+__host__ __device__ constexpr int conv_threads(int cout) { return conv_workers(cout) + 32; }
+constexpr int kSlots = 3;
 __host__ __device__ constexpr int dhalo_slot_bytes(int cin) { return (cin / 8) * kHX * kHY * 16; }
 __host__ __device__ constexpr int dhalo_bytes(int cin) { return kSlots * dhalo_slot_bytes(cin); }
-
+// Accumulators in the TMEM ring: the three being summed and the one being read
+// need 4; 8 where two blocks per SM leave the columns for it (fewer wraps).
+__host__ __device__ constexpr int ring_planes(int cin, int cout) { return cin == 32 || cout == 16 ? 8 : 4; }
+__host__ __device__ constexpr int ring_cols(int cin, int cout) { return ring_planes(cin, cout) * cout; }
 __host__ __device__ inline bool dhalo_ok(int nx, int ny) { return nx % 8 == 0 && ny % 16 == 0; }
 
 // Copies plane zz (-1 <= zz <= nz, periodic) of the column at (x0, y0) into
 // its ring slot S (worker threads).
-template <int CIN>
+template <int CIN, int WORKERS>
 __device__ __forceinline__ void dhalo_load_plane(const Grid3& g, const __nv_bfloat16* __restrict__ in, int x0,
                                                  int y0, int zz, unsigned char* S) {
     constexpr int N = (CIN / 8) * kHX * kHY;
     const int64_t zoff = (int64_t)wrapi(zz, g.nz) * g.ny;
-    for (int i = threadIdx.x; i < N; i += kZWorkers) {
+    for (int i = threadIdx.x; i < N; i += WORKERS) {
         const int hx = i % kHX, hy = (i / kHX) % kHY, kg = i / (kHX * kHY);
         const int64_t cell = (zoff + wrapi(y0 - 1 + hy, g.ny)) * g.nx + wrapi(x0 - 1 + hx, g.nx);
         const uint4* src = reinterpret_cast<const uint4*>(in + cell * CIN) + kg;
@@ -290,20 +304,17 @@ __device__ __forceinline__ void dhalo_load_plane(const Grid3& g, const __nv_bflo
 }
 
 // Epilogue of one tile: this thread's cell c (TMEM lane = threadIdx % 128)
-// and its half of the COUT accumulator columns (bias: that half's biases).
+// and its kEpiCols accumulator columns (bias: their biases).
 template <int COUT, int MODE>
-__device__ __forceinline__ void conv_epilogue(uint32_t tacc, int64_t c, const float (&bias)[COUT / 2],
+__device__ __forceinline__ void conv_epilogue(uint32_t tacc, int64_t c, int64_t V, const float (&bias)[kEpiCols],
                                               const __nv_bfloat16* __restrict__ pre_below,
                                               __nv_bfloat16* __restrict__ out_pre, __nv_bfloat16* __restrict__ out_bf,
                                               float* __restrict__ out_f) {
-    constexpr int H = COUT / 2;
-    static_assert(H == 8 || H == 16, "16 or 32 output channels");
-    const int w = threadIdx.x >> 5, half = threadIdx.x >> 7;
-    const int j0 = half * H;
+    constexpr int H = kEpiCols;
+    static_assert(H == 8, "one 16-byte BF16 store per thread and cell");
+    const int w = threadIdx.x >> 5, j0 = (threadIdx.x >> 7) * H;
     float acc[H];
-    const uint32_t ta = tacc + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)j0;
-    if constexpr (H == 16) tc::tmem_ld16(ta, acc);
-    else tc::tmem_ld8(ta, acc);
+    tc::tmem_ld8(tacc + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)j0, acc);
     if constexpr (MODE == kFwdHidden) {
         __align__(16) __nv_bfloat16 pb[H], ab[H];
 #pragma unroll
@@ -312,34 +323,27 @@ __device__ __forceinline__ void conv_epilogue(uint32_t tacc, int64_t c, const fl
             pb[j] = __float2bfloat16(p);
             ab[j] = __float2bfloat16(gelu(p));
         }
-#pragma unroll
-        for (int q = 0; q < H / 8; ++q) {
-            reinterpret_cast<uint4*>(out_pre + c * COUT + j0)[q] = reinterpret_cast<const uint4*>(pb)[q];
-            reinterpret_cast<uint4*>(out_bf + c * COUT + j0)[q] = reinterpret_cast<const uint4*>(ab)[q];
-        }
+        *reinterpret_cast<uint4*>(out_pre + c * COUT + j0) = *reinterpret_cast<const uint4*>(pb);
+        *reinterpret_cast<uint4*>(out_bf + c * COUT + j0) = *reinterpret_cast<const uint4*>(ab);
     } else if constexpr (MODE == kFwdLast) {
+        static_assert(MODE != kFwdLast || H == kOutChannels, "the columns from kOutChannels on are padding");
+        if (j0 == 0) {
 #pragma unroll
-        for (int j = 0; j < H; j += 4)
-            reinterpret_cast<float4*>(out_f + c * COUT + j0)[j / 4] =
-                make_float4(acc[j] + bias[j], acc[j + 1] + bias[j + 1], acc[j + 2] + bias[j + 2],
-                            acc[j + 3] + bias[j + 3]);
+            for (int j = 0; j < H; ++j) out_f[j * V + c] = acc[j] + bias[j];
+        }
     } else {
         __align__(16) __nv_bfloat16 pre[H], gb[H];
-#pragma unroll
-        for (int q = 0; q < H / 8; ++q)
-            reinterpret_cast<uint4*>(pre)[q] = reinterpret_cast<const uint4*>(pre_below + c * COUT + j0)[q];
+        *reinterpret_cast<uint4*>(pre) = *reinterpret_cast<const uint4*>(pre_below + c * COUT + j0);
 #pragma unroll
         for (int j = 0; j < H; ++j) gb[j] = __float2bfloat16(acc[j] * gelu_grad(__bfloat162float(pre[j])));
-#pragma unroll
-        for (int q = 0; q < H / 8; ++q)
-            reinterpret_cast<uint4*>(out_bf + c * COUT + j0)[q] = reinterpret_cast<const uint4*>(gb)[q];
+        *reinterpret_cast<uint4*>(out_bf + c * COUT + j0) = *reinterpret_cast<const uint4*>(gb);
     }
 }
 
 // Block b marches column b % cols over planes [zc * (b / cols), + zc).
-// Smem: B image, then the plane ring.  TMEM: two 32-column accumulators.
+// Smem: B image, then the plane ring.
 template <int CIN, int COUT, int MODE>
-__global__ void __launch_bounds__(kZThreads) conv_dhalo_kernel(Grid3 g, int zc, const __nv_bfloat16* __restrict__ in,
+__global__ void __launch_bounds__(conv_threads(COUT)) conv_dhalo_kernel(Grid3 g, int zc, const __nv_bfloat16* __restrict__ in,
                                                                const uint4* __restrict__ bimg,
                                                                const float* __restrict__ bias,
                                                                const __nv_bfloat16* __restrict__ pre_below,
@@ -347,9 +351,11 @@ __global__ void __launch_bounds__(kZThreads) conv_dhalo_kernel(Grid3 g, int zc, 
                                                                __nv_bfloat16* __restrict__ out_bf,
                                                                float* __restrict__ out_f, int* __restrict__ err,
                                                                uint32_t wait_limit) {
+    constexpr int WORKERS = conv_workers(COUT), THREADS = conv_threads(COUT), ISSUER = WORKERS;
     constexpr int KS = CIN / 16;
     constexpr int BBYTES = bimg_bytes(CIN, COUT);
     constexpr int SLOT = dhalo_slot_bytes(CIN);
+    constexpr int NP = ring_planes(CIN, COUT), TCOLS = ring_cols(CIN, COUT);
     constexpr uint32_t KG = kHX * kHY;  // 16-byte units between 8-channel groups
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint64_t bar[2];
@@ -357,106 +363,120 @@ __global__ void __launch_bounds__(kZThreads) conv_dhalo_kernel(Grid3 g, int zc, 
     unsigned char* Bs = sm;
     unsigned char* Hs = sm + BBYTES;
     const int t = threadIdx.x;
-    for (int i = t; i < BBYTES / 16; i += kZThreads) reinterpret_cast<uint4*>(Bs)[i] = bimg[i];
+    const int bx = g.nx / 8, cols = bx * (g.ny / 16);
+    const int col = (int)(blockIdx.x % (unsigned)cols);
+    const int x0 = (col % bx) * 8, y0 = (col / bx) * 16;
+    const int za = (int)(blockIdx.x / (unsigned)cols) * zc, len = min(zc, g.nz - za);
+    const int last = len + 1;  // steps 0 .. last: input planes za - 1 .. za + len
+    const bool worker = t < WORKERS;
+    if (worker) {
+        dhalo_load_plane<CIN, WORKERS>(g, in, x0, y0, za - 1, Hs);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        dhalo_load_plane<CIN, WORKERS>(g, in, x0, y0, za, Hs + SLOT);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    for (int i = t; i < BBYTES / 16; i += THREADS) reinterpret_cast<uint4*>(Bs)[i] = bimg[i];
     if (t == 0) {
         tc::mbar_init(&bar[0], 1);
         tc::mbar_init(&bar[1], 1);
         tc::mbar_fence_init();
     }
-    if (t < 32) tc::tmem_alloc(&tslot, 64);
-    const int bx = g.nx / 8, cols = bx * (g.ny / 16);
-    const int col = (int)(blockIdx.x % (unsigned)cols);
-    const int x0 = (col % bx) * 8, y0 = (col / bx) * 16;
-    const int za = (int)(blockIdx.x / (unsigned)cols) * zc, zb = min(za + zc, g.nz);
-    const bool worker = t < kZWorkers;
-    float bias_h[COUT / 2];  // this worker's half of the biases
+    if (t < 32) tc::tmem_alloc(&tslot, TCOLS);
+    float bias_h[kEpiCols];  // the biases of this worker's columns
 #pragma unroll
-    for (int j = 0; j < COUT / 2; ++j) bias_h[j] = worker ? bias[((t >> 7) & 1) * (COUT / 2) + j] : 0.0f;
-    if (worker) {
-        for (int zz = za - 1; zz <= za + 1 && za < zb; ++zz)
-            dhalo_load_plane<CIN>(g, in, x0, y0, zz, Hs + ring_slot(zz) * SLOT);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        if (za + 2 <= zb) dhalo_load_plane<CIN>(g, in, x0, y0, za + 2, Hs + ring_slot(za + 2) * SLOT);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // planes za-1 .. za+1 in; za+2 may be in flight
+    for (int j = 0; j < kEpiCols; ++j)
+        bias_h[j] = (MODE != kBwdData && worker) ? bias[(t >> 7) * kEpiCols + j] : 0.0f;
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // plane za - 1 in; za may be in flight
     tc::fence_smem_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tslot;
-    const uint32_t idesc = tc::idesc_bf16(kTileM, COUT, 0, 0);
     const uint32_t h0 = tc::smem_addr(Hs), b0 = tc::smem_addr(Bs);
     // a worker's cell in a tile of plane z: M row t % 128
+    const int64_t nxy = (int64_t)g.nx * g.ny;
     const int64_t cxy = (int64_t)(y0 + (t & 127) / 8) * g.nx + x0 + (t & 7);
-    uint32_t uses[2] = {0, 0};
     bool ok = true;
-    int n = 0;
-    for (int z = za; z < zb && ok; ++z, ++n) {
-        const int b = n & 1;
-        if (t == kZIssuer) {
-            // planes z-1 .. z+1 were copied before the last barrier, and the
-            // previous tile of accumulator b (z - 2) was read before it
-            const uint64_t db0 = tc::smem_desc(b0, 128, 256);
+    int n = 0;  // steps issued
+    for (int s = 0; s <= last && ok; ++s) {
+        if (t == ISSUER) {
+            // Input plane r (relative to za) feeds the output planes lo .. hi of
+            // r - 1 .. r + 1; the last of them, r + 1, starts with this plane.
+            const int r = s - 1, lo = max(r - 1, 0), hi = min(r + 1, len - 1);
+            const bool fresh = r + 1 <= len - 1;
+            // the window's accumulators: n0 planes at slot lo % NP, the rest (if
+            // it wraps) from slot 0 on
+            const int n0 = min(hi - lo + 1, NP - lo % NP), n1 = hi - lo + 1 - n0;
+            const uint32_t d0 = tmem + (uint32_t)(lo % NP) * COUT;
+            const uint32_t i0 = tc::idesc_bf16(kTileM, COUT, 0, 0) + (uint32_t)((n0 - 1) * (COUT / 8)) * (1u << 17);
+            const uint32_t i1 = tc::idesc_bf16(kTileM, COUT, 0, 0) + (uint32_t)((n1 - 1) * (COUT / 8)) * (1u << 17);
+            // descriptors: the start address is the low field (16-byte units,
+            // smem < 256 KB so no carry), offsets add directly
+            const uint64_t da0 = tc::smem_desc(h0 + (s % kSlots) * SLOT, KG * 16, kHX * 16);
+            const uint64_t db0 = tc::smem_desc(b0 + (uint32_t)(lo - (r - 1)) * COUT * 32, 128, 256);
 #pragma unroll
-            for (int tap = 0; tap < 27; ++tap) {
-                const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-                // the start address is the descriptor's low field (16-byte
-                // units, smem < 256 KB so no carry): offsets add directly
-                const uint64_t da = tc::smem_desc(h0 + ring_slot(z + dz) * SLOT, KG * 16, kHX * 16);
+            for (int yx = 0; yx < 9; ++yx) {
 #pragma unroll
                 for (int kb = 0; kb < KS; ++kb) {
-                    const uint32_t aoff = 2 * kb * KG + (uint32_t)((1 + dy) * kHX + 1 + dx);
-                    const uint32_t boff = (uint32_t)((tap * KS + kb) * COUT * 32 / 16);
-                    tc::mma_bf16(tmem + b * 32, da + aoff, db0 + boff, idesc, (tap > 0 || kb > 0) ? 1u : 0u);
+                    const uint64_t da = da0 + (uint32_t)(2 * kb * KG + (yx / 3) * kHX + yx % 3);
+                    const uint64_t db = db0 + (uint32_t)((yx * KS + kb) * 3 * COUT * 32 / 16);
+                    if (yx == 0 && kb == 0 && fresh) {
+                        // one plane at a time: plane r + 1 overwrites its slot
+                        for (int o = lo; o <= hi; ++o)
+                            tc::mma_bf16(tmem + (uint32_t)(o % NP) * COUT, da, db + (uint32_t)((o - lo) * COUT * 32 / 16),
+                                         tc::idesc_bf16(kTileM, COUT, 0, 0), o <= r ? 1u : 0u);
+                    } else {
+                        tc::mma_bf16(d0, da, db, i0, 1u);
+                        if (n1 > 0) tc::mma_bf16(tmem, da, db + (uint32_t)(n0 * COUT * 32 / 16), i1, 1u);
+                    }
                 }
             }
-            tc::mma_commit(&bar[b]);
+            tc::mma_commit(&bar[s & 1]);
         }
-        ++uses[b];
+        n = s + 1;
         bool lost = false;
         if (worker) {
-            // tile z - 1 done: its accumulator is final, and the slot of plane
-            // z - 2, which only it still read, takes plane z + 3
-            if (uses[b ^ 1] > 0) lost = !tc::mbar_wait(&bar[b ^ 1], (uses[b ^ 1] - 1) & 1, err, wait_limit);
+            // step s - 1 done: its plane's slot takes plane s + 2, and output
+            // plane s - 3 is final
+            if (s > 0) lost = !tc::mbar_wait(&bar[(s - 1) & 1], ((s - 1) >> 1) & 1, err, wait_limit);
             if (!lost) {
                 tc::fence_after_sync();
-                if (z + 3 <= zb) dhalo_load_plane<CIN>(g, in, x0, y0, z + 3, Hs + ring_slot(z + 3) * SLOT);
+                if (s + 2 <= last)
+                    dhalo_load_plane<CIN, WORKERS>(g, in, x0, y0, za + s + 1, Hs + ((s + 2) % kSlots) * SLOT);
                 asm volatile("cp.async.commit_group;\n" ::: "memory");
-                if (z > za)
-                    conv_epilogue<COUT, MODE>(tmem + (b ^ 1) * 32, (int64_t)(z - 1) * g.nx * g.ny + cxy, bias_h,
-                                              pre_below, out_pre, out_bf, out_f);
+                if (s >= 3)
+                    conv_epilogue<COUT, MODE>(tmem + (uint32_t)((s - 3) % NP) * COUT, (int64_t)(za + s - 3) * nxy + cxy,
+                                              g.V, bias_h, pre_below, out_pre, out_bf, out_f);
             }
-            // plane z + 2 in (tile z + 1 reads it); z + 3 may stay in flight
+            // plane s + 1 in; s + 2 may stay in flight
             if (lost) asm volatile("cp.async.wait_all;\n" ::: "memory");
             else asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             tc::fence_smem_async();
         }
         tc::fence_before_sync();
-        if (__syncthreads_or(lost)) {  // plane z + 2 visible; accumulator b^1 read
+        if (__syncthreads_or(lost)) {  // plane s + 1 visible; accumulator s - 3 read
             ok = false;
             break;
         }
         tc::fence_after_sync();
     }
-    if (ok && n > 0) {
-        const int b = (n - 1) & 1;
+    if (ok) {
         bool lost = false;
-        if (worker) lost = !tc::mbar_wait(&bar[b], (uses[b] - 1) & 1, err, wait_limit);
+        if (worker) lost = !tc::mbar_wait(&bar[last & 1], (last >> 1) & 1, err, wait_limit);
         if (!__syncthreads_or(lost) && worker) {
             tc::fence_after_sync();
-            conv_epilogue<COUT, MODE>(tmem + b * 32, (int64_t)(zb - 1) * g.nx * g.ny + cxy, bias_h, pre_below,
-                                      out_pre, out_bf, out_f);
+            conv_epilogue<COUT, MODE>(tmem + (uint32_t)((len - 1) % NP) * COUT, (int64_t)(za + len - 1) * nxy + cxy, g.V,
+                                      bias_h, pre_below, out_pre, out_bf, out_f);
         }
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");  // no copy outlives the block
-    if (t == 0) {
-        for (int s = 0; s < 2; ++s)
-            if (uses[s] > 0) tc::mbar_wait(&bar[s], (uses[s] - 1) & 1, err);
+    if (t == 0) {  // drain: the newest commit on each barrier
+        for (int k = 1; k <= 2; ++k)
+            if (n >= k) tc::mbar_wait(&bar[(n - k) & 1], ((n - k) >> 1) & 1, err);
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (t < 32) tc::tmem_dealloc(tmem, 64);
+    if (t < 32) tc::tmem_dealloc(tmem, TCOLS);
 }
 
 // Weight gradient dW[tap][ci][co] = sum_c act[c + off(tap)][ci] * grad[c][co]
@@ -598,166 +618,209 @@ __global__ void __launch_bounds__(kThreads) wgrad_kernel(Grid3 g, const __nv_bfl
     if (t < 32) tc::tmem_dealloc(tmem, WS::TCOLS);
 }
 
-// The weight gradient's per-tile halo: the 10 x 18 x 3 neighbourhood of an
-// 8 x 16 x 1 tile as 16-byte units, one block per 8-channel group:
-//   unit(kg, hz, hy, hx) at ((kg*3 + hz)*18 + hy)*10 + hx.
-constexpr int kHZ = 3;
-__host__ __device__ constexpr int whalo_bytes(int cin) { return (cin / 8) * kHX * kHY * kHZ * 16; }
-
-template <int CIN>
-__device__ __forceinline__ void whalo_load(const Grid3& g, const __nv_bfloat16* __restrict__ in, int x0, int y0,
-                                           int z0, unsigned char* H) {
-    constexpr int QU = CIN / 8;
-    constexpr int N = QU * kHX * kHY * kHZ;
-    for (int i = threadIdx.x; i < N; i += kThreads) {
-        const int hx = i % kHX, hy = (i / kHX) % kHY, hz = (i / (kHX * kHY)) % kHZ, kg = i / (kHX * kHY * kHZ);
-        const int64_t cell =
-            ((int64_t)wrapi(z0 - 1 + hz, g.nz) * g.ny + wrapi(y0 - 1 + hy, g.ny)) * g.nx + wrapi(x0 - 1 + hx, g.nx);
-        const uint4* src = reinterpret_cast<const uint4*>(in + cell * CIN) + kg;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(tc::smem_addr(H + i * 16)), "l"(src));
-    }
-}
-
-// Weight gradient on 8 x 16 x 1 tiles (nx % 8 == 0, ny % 16 == 0).  Per tile
-// the activation halo (above) and the tile's
-// output gradient are staged once; then for each group of TPG taps the
-// MN-major A operand (rows (tap, ci), K = the tile's 128 cells) is assembled
-// from the halo by 16-byte copies -- cell k of the tile is row k of every
-// 8-channel plane, so K-groups are 128 bytes apart and channel groups 2 KB --
-// and 8 K-steps of MMAs accumulate into the group's TMEM columns.  Two A
-// buffers let the copies of one group overlap the MMAs of the previous one.
+// Weight gradient on 8 x 16 x 1 tiles (nx % 8 == 0, ny % 16 == 0), marching z.
+//
+// dW[tap][ci][co] is a GEMM with M = (tap, ci), N = co and K = cells.  The
+// tensor core reads both operands where cp.async put them: an MN-major core
+// matrix holds 8 channels of 8 consecutive cells, 16 bytes per cell, which is
+// what 8 x-cells of a channel-last field are.  A staged plane holds three
+// copies of the column's 18 rows, shifted by dx = -1, 0, 1, each 8 cells wide
+// and one block per 8-channel group:
+//   unit(slot, g, hy, x) at slot*SLOT + (g*18 + hy)*8 + x,  g = (dx+1)*CIN/8 + kg,
+// so 16 consecutive groups at one stride are the M = 128 rows of an operand:
+// the 3 CIN rows of the three dx taps, a group whose channel 0 is the constant
+// 1 (its row of the product is the bias gradient), and groups of the next slot
+// whose rows are not read back.  dy moves the start by one row (128 bytes), dz
+// picks the slot, and the K groups (y rows) are 128 bytes apart.  A tile is 9
+// (dy, dz) x 8 K-steps of MMAs and costs one new plane and one gradient tile;
+// nothing is copied inside shared memory.  (Assembling a 32 KB operand per 4
+// taps in shared memory instead took 179 us per 32 -> 32 layer at 64^3, and the
+// bias gradient 25 us in kernels of its own.)
+//
+// One block per SM takes an equal share of the column-major sequence of tiles.
+// Warps 0-7 copy (two planes ahead, ring of 5 planes and 3 gradient tiles),
+// warp 8 issues the MMAs; one block barrier per tile.  The nine accumulators
+// (COUT columns each) stay in TMEM for the whole share.
+constexpr int kWRing = 5, kWGrads = 3;
 template <int CIN, int COUT>
-struct WGradHalo {
-    static constexpr int TPG = kTileM / CIN;
-    static constexpr int G = (27 + TPG - 1) / TPG;
-    static constexpr int TCOLS = WGradShape<CIN, COUT>::TCOLS;
-    static constexpr int HB = whalo_bytes(CIN);
-    static constexpr int BB = (COUT / 8) * 2048;  // output-gradient tile
-    static constexpr int AB = 16 * 2048;          // one A buffer (128 x 128 BF16)
-    static constexpr int SMEM = HB + BB + 2 * AB;
+struct WGradMarch {
+    static constexpr int KGN = CIN / 8;
+    static constexpr int GROUP = kHY * 8 * 16;             // bytes of one channel group
+    static constexpr int SLOTG = 3 * KGN + 1;              // groups per plane, the constant one last
+    static constexpr int SLOT = SLOTG * GROUP;
+    static constexpr int PAD = (16 - SLOTG) * GROUP;       // the last slot's operand ends here
+    static constexpr int GB = (COUT / 8) * 2048;           // output-gradient tile
+    static constexpr int SMEM = kWRing * SLOT + PAD + kWGrads * GB;
+    static constexpr int TCOLS = 9 * COUT <= 256 ? 256 : 512;
+    static constexpr int NOUT = 27 * CIN * COUT + COUT;    // weights, then biases
+    static_assert(SLOTG <= 16, "the constant group lies inside the 128 operand rows");
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads) wgrad_dhalo_kernel(Grid3 g, const __nv_bfloat16* __restrict__ act,
-                                                               const __nv_bfloat16* __restrict__ grad,
-                                                               float* __restrict__ partials, int* __restrict__ err,
-        uint32_t wait_limit) {
-    using WH = WGradHalo<CIN, COUT>;
-    constexpr int TPG = WH::TPG, G = WH::G, QU = CIN / 8;
+__global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const __nv_bfloat16* __restrict__ act,
+                                                                const __nv_bfloat16* __restrict__ grad,
+                                                                float* __restrict__ partials, int* __restrict__ err,
+                                                                uint32_t wait_limit) {
+    using WM = WGradMarch<CIN, COUT>;
+    constexpr int KGN = WM::KGN, SLOT = WM::SLOT;
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint64_t bar[2];
     __shared__ uint32_t tslot;
-    unsigned char* Hs = sm;
-    unsigned char* Bs = sm + WH::HB;
-    unsigned char* As = Bs + WH::BB;
+    unsigned char* Gs = sm + kWRing * SLOT + WM::PAD;
     const int t = threadIdx.x;
     if (t == 0) {
         tc::mbar_init(&bar[0], 1);
         tc::mbar_init(&bar[1], 1);
         tc::mbar_fence_init();
     }
-    if (t < 32) tc::tmem_alloc(&tslot, WH::TCOLS);
+    if (t < 32) tc::tmem_alloc(&tslot, WM::TCOLS);
+    for (int i = t; i < kWRing * kHY * 8; i += kZThreads) {  // channel 0 = 1.0 in BF16
+        const int slot = i / (kHY * 8), u = i % (kHY * 8);
+        *reinterpret_cast<uint4*>(sm + slot * SLOT + 3 * KGN * WM::GROUP + u * 16) = make_uint4(0x3F80u, 0, 0, 0);
+    }
+    tc::fence_smem_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tslot;
     const uint32_t idesc = tc::idesc_bf16(kTileM, COUT, 1, 1);
-    const uint32_t a0 = tc::smem_addr(As), b0 = tc::smem_addr(Bs);
-    const int bx = g.nx / 8, by = g.ny / 16;
-    const int64_t ntiles = (int64_t)bx * by * g.nz;
-    uint32_t uses[2] = {0, 0};
-    int kg_run = 0;  // groups issued so far (selects the A buffer)
-    int last_b = -1;
-    bool ok = true, any = false;
-    for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const int x0 = (int)(tile % bx) * 8, y0 = (int)((tile / bx) % by) * 16;
-        const int z0 = (int)(tile / ((int64_t)bx * by));
-        // the previous tile's MMAs read the gradient tile: let them finish
-        bool lost = last_b >= 0 && !tc::mbar_wait(&bar[last_b], (uses[last_b] - 1) & 1, err, wait_limit);
+    const uint32_t s0 = tc::smem_addr(sm), g0 = tc::smem_addr(Gs);
+    const bool worker = t < kZWorkers;
+    const int bx = g.nx / 8;
+    const int64_t ntiles = (int64_t)bx * (g.ny / 16) * g.nz;
+    int64_t tile = ntiles * blockIdx.x / gridDim.x;
+    const int64_t tile1 = ntiles * (blockIdx.x + 1) / gridDim.x;
+    int n = 0;  // tiles issued by this block
+    bool ok = true;
+    while (tile < tile1 && ok) {
+        // one column segment: planes [za, za + len)
+        const int64_t col = tile / g.nz;
+        const int za = (int)(tile - col * g.nz);
+        const int len = (int)min((int64_t)(g.nz - za), tile1 - tile);
+        const int x0 = (int)(col % bx) * 8, y0 = (int)(col / bx) * 16;
+        // plane za + r (-1 <= r <= len) into slot (r + 1) % ring, gradient tile
+        // za + r into slot r % 3
+        auto load_plane = [&](int r) {
+            unsigned char* S = sm + ((r + 1) % kWRing) * SLOT;
+            const int64_t zoff = (int64_t)wrapi(za + r, g.nz) * g.ny;
+            for (int i = t; i < 3 * KGN * kHY * 8; i += kZWorkers) {
+                const int x = i % 8, hy = (i / 8) % kHY, gr = i / (8 * kHY);
+                const int dx = gr / KGN - 1, kg = gr % KGN;
+                const int64_t cell = (zoff + wrapi(y0 - 1 + hy, g.ny)) * g.nx + wrapi(x0 + x + dx, g.nx);
+                const uint4* src = reinterpret_cast<const uint4*>(act + cell * CIN) + kg;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(tc::smem_addr(S + i * 16)), "l"(src));
+            }
+        };
+        auto load_grad = [&](int r) {
+            unsigned char* D = Gs + (r % kWGrads) * WM::GB;
+            for (int i = t; i < (COUT / 8) * 128; i += kZWorkers) {
+                const int k = i % 128, q = i / 128;
+                const int64_t cell = ((int64_t)(za + r) * g.ny + y0 + k / 8) * g.nx + x0 + k % 8;
+                const uint4* src = reinterpret_cast<const uint4*>(grad + cell * COUT) + q;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(tc::smem_addr(D + i * 16)), "l"(src));
+            }
+        };
+        bool lost = false;
+        if (worker) {
+            // the previous segment's MMAs read the slots refilled here
+            if (n > 0) lost = !tc::mbar_wait(&bar[(n - 1) & 1], ((n - 1) >> 1) & 1, err, wait_limit);
+            if (!lost) {
+                for (int r = -1; r <= 1; ++r) load_plane(r);
+                load_grad(0);
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+                if (len > 1) {
+                    load_plane(2);
+                    load_grad(1);
+                }
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            }
+            tc::fence_smem_async();
+        }
+        tc::fence_before_sync();
         if (__syncthreads_or(lost)) {
             ok = false;
             break;
         }
-        whalo_load<CIN>(g, act, x0, y0, z0, Hs);
-        for (int i = t; i < (COUT / 8) * 128; i += kThreads) {
-            const int k = i % 128, q = i / 128;
-            const int64_t cell = ((int64_t)z0 * g.ny + y0 + k / 8) * g.nx + x0 + k % 8;
-            const uint4* src = reinterpret_cast<const uint4*>(grad + cell * COUT) + q;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(tc::smem_addr(Bs + q * 2048 + k * 16)),
-                         "l"(src));
-        }
-        asm volatile("cp.async.wait_all;\n" ::: "memory");
-        __syncthreads();
-        for (int gi = 0; gi < G; ++gi, ++kg_run) {
-            const int b = kg_run & 1;
-            lost = uses[b] > 0 && !tc::mbar_wait(&bar[b], (uses[b] - 1) & 1, err, wait_limit);
+        tc::fence_after_sync();
+        for (int i = 0; i < len; ++i, ++n) {
+            if (t == kZIssuer) {
+                const uint64_t db0 = tc::smem_desc(g0 + (i % kWGrads) * WM::GB, 128, 2048);
+#pragma unroll
+                for (int gi = 0; gi < 9; ++gi) {
+                    const int dy = gi % 3 - 1, dz = gi / 3 - 1;
+                    const uint64_t da0 =
+                        tc::smem_desc(s0 + ((i + dz + 1) % kWRing) * SLOT + (1 + dy) * 128, 128, WM::GROUP);
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks)
+                        tc::mma_bf16(tmem + gi * COUT, da0 + (uint32_t)(ks * 256 / 16), db0 + (uint32_t)(ks * 256 / 16),
+                                     idesc, (n > 0 || ks > 0) ? 1u : 0u);
+                }
+                tc::mma_commit(&bar[n & 1]);
+            }
+            if (worker) {
+                // tile n - 1 done: plane i - 2 (its slot takes plane i + 3) and
+                // the gradient of tile i - 1 are no longer read
+                if (n > 0) lost = !tc::mbar_wait(&bar[(n - 1) & 1], ((n - 1) >> 1) & 1, err, wait_limit);
+                if (!lost) {
+                    if (i + 3 <= len) load_plane(i + 3);
+                    if (i + 2 < len) load_grad(i + 2);
+                    asm volatile("cp.async.commit_group;\n" ::: "memory");
+                    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // plane i + 2, gradient i + 1
+                } else {
+                    asm volatile("cp.async.wait_all;\n" ::: "memory");
+                }
+                tc::fence_smem_async();
+            }
+            tc::fence_before_sync();
             if (__syncthreads_or(lost)) {
                 ok = false;
+                ++n;
                 break;
             }
-            unsigned char* A = As + b * WH::AB;
-            for (int i = t; i < TPG * QU * 128; i += kThreads) {
-                const int k = i % 128, kg = (i / 128) % QU, j = i / (128 * QU);
-                const int tap = gi * TPG + j;
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (tap < 27) {
-                    const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-                    const int hu = ((kg * kHZ + 1 + dz) * kHY + 1 + dy + k / 8) * kHX + 1 + dx + k % 8;
-                    v = *reinterpret_cast<const uint4*>(Hs + hu * 16);
-                }
-                *reinterpret_cast<uint4*>(A + (j * QU + kg) * 2048 + k * 16) = v;
-            }
-            tc::fence_smem_async();
-            tc::fence_before_sync();
-            __syncthreads();
             tc::fence_after_sync();
-            if (t == 0) {
-                const uint64_t da0 = tc::smem_desc(a0 + b * WH::AB, 128, 2048);
-                const uint64_t db0 = tc::smem_desc(b0, 128, 2048);
-#pragma unroll
-                for (int ks = 0; ks < 8; ++ks)
-                    tc::mma_bf16(tmem + gi * COUT, da0 + (uint32_t)(ks * 256 / 16), db0 + (uint32_t)(ks * 256 / 16),
-                                 idesc, (any || ks > 0) ? 1u : 0u);
-                tc::mma_commit(&bar[b]);
-            }
-            ++uses[b];
-            last_b = b;
         }
-        any = true;
+        tile += len;
     }
-    if (ok && last_b >= 0) {
-        const bool lost = !tc::mbar_wait(&bar[last_b], (uses[last_b] - 1) & 1, err, wait_limit);
+    if (ok && n > 0) {
+        const bool lost = !tc::mbar_wait(&bar[(n - 1) & 1], ((n - 1) >> 1) & 1, err, wait_limit);
         ok = !__syncthreads_or(lost);
     }
     tc::fence_after_sync();
-    if (ok) {
-        const int w = t >> 5;
-        const int j = t / CIN, ci = t % CIN;
-        float* dst = partials + (int64_t)blockIdx.x * 27 * CIN * COUT;
-        for (int gi = 0; gi < G; ++gi) {
+    if (ok && worker) {
+        // lane m of an accumulator: channel group m / 8, channel m % 8; warps w
+        // and w + 4 read the same lanes and take alternate accumulators
+        const int w = t >> 5, m = t & 127, gr = m / 8;
+        const int dx = gr / KGN, ci = (gr % KGN) * 8 + m % 8;
+        float* dst = partials + (int64_t)blockIdx.x * WM::NOUT;
+        for (int gi = w >> 2; gi < 9; gi += 2) {
             float v[COUT];
-            if (!any) {
+            if (n == 0) {
 #pragma unroll
-                for (int co = 0; co < COUT; ++co) v[co] = 0.0f;
+                for (int co = 0; co < COUT; ++co) v[co] = 0.0f;  // no tiles: zero partial
             } else {
 #pragma unroll
                 for (int c0 = 0; c0 < COUT; c0 += 16)
-                    tc::tmem_ld16(tmem + ((uint32_t)(32 * w) << 16) + (uint32_t)(gi * COUT + c0), v + c0);
+                    tc::tmem_ld16(tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(gi * COUT + c0), v + c0);
             }
-            const int tap = gi * TPG + j;
-            if (tap < 27) {
+            float* o = nullptr;
+            if (gr < 3 * KGN) o = dst + ((gi * 3 + dx) * CIN + ci) * COUT;
+            else if (gi == 4 && m == 24 * KGN) o = dst + 27 * CIN * COUT;  // the constant row, undisplaced
+            if (o) {
 #pragma unroll
-                for (int co = 0; co < COUT; ++co) dst[((int64_t)tap * CIN + ci) * COUT + co] = v[co];
+                for (int co = 0; co < COUT; co += 4)
+                    *reinterpret_cast<float4*>(o + co) = make_float4(v[co], v[co + 1], v[co + 2], v[co + 3]);
             }
         }
     }
-    if (t == 0) {
-        for (int s = 0; s < 2; ++s)
-            if (uses[s] > 0) tc::mbar_wait(&bar[s], (uses[s] - 1) & 1, err);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");  // no copy outlives the block
+    if (t == 0) {  // drain: the newest commit on each barrier
+        for (int k = 1; k <= 2; ++k)
+            if (n >= k) tc::mbar_wait(&bar[(n - k) & 1], ((n - k) >> 1) & 1, err);
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (t < 32) tc::tmem_dealloc(tmem, WH::TCOLS);
+    if (t < 32) tc::tmem_dealloc(tmem, WM::TCOLS);
 }
 
 // out[j] = sum over p < P of partials[p * n + j] in a fixed order: a block
@@ -819,13 +882,12 @@ __global__ void pack_kernel(const float* __restrict__ W, __nv_bfloat16* __restri
         const int co = i % COUT, ci = (i / COUT) % CIN, tap = i / (CIN * COUT);
         const __nv_bfloat16 v = __float2bfloat16(W[i]);
         {  // forward: B[n = co][k = ci] of k-step (tap, ci/16)
-            const int s = tap * (CIN / 16) + ci / 16, k = ci % 16;
-            fwd[(s * COUT * 32 + tc::kmajor_off(co, k, 128, 256)) / 2] = v;
+            const int k = ci % 16;
+            fwd[(bimg_off(CIN, COUT, tap % 9, ci / 16, tap / 9 - 1) + tc::kmajor_off(co, k, 128, 256)) / 2] = v;
         }
         if (bwd) {  // backward data: tap' = 26 - tap, B[n = ci][k = co]
-            const int tp = 26 - tap;
-            const int s = tp * (COUT / 16) + co / 16, k = co % 16;
-            bwd[(s * CIN * 32 + tc::kmajor_off(ci, k, 128, 256)) / 2] = v;
+            const int tp = 26 - tap, k = co % 16;
+            bwd[(bimg_off(COUT, CIN, tp % 9, co / 16, tp / 9 - 1) + tc::kmajor_off(ci, k, 128, 256)) / 2] = v;
         }
     }
 }
@@ -903,7 +965,7 @@ __global__ void __launch_bounds__(kThreads) loss_kernel(const float* __restrict_
         for (int j = 0; j < 16; ++j) {
             float gj = 0.0f;
             if (j < 8) {
-                const float d = out[c * 16 + j] - tgt[j * V + c] * inv_scale[j];
+                const float d = out[j * V + c] - tgt[j * V + c] * inv_scale[j];
                 acc += (double)d * d;
                 gj = gscale * d;
             }
@@ -922,15 +984,15 @@ __global__ void __launch_bounds__(kThreads) loss_kernel(const float* __restrict_
     }
 }
 
-// Correction of a coarse state after its step: Q_k += gain out[c][k] s_k
-// (k < 5), u_d += gain out[c][5+d] s_{5+d}.
+// Correction of a coarse state after its step: Q_k += gain out[k][c] s_k
+// (k < 5), u_d += gain out[5+d][c] s_{5+d}.
 __global__ void apply_kernel(const float* __restrict__ out, const float* __restrict__ out_scale, int64_t V,
                              float gain, float* __restrict__ u3, float* __restrict__ q5) {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < V; c += (int64_t)gridDim.x * blockDim.x) {
 #pragma unroll
-        for (int k = 0; k < 5; ++k) q5[k * V + c] += gain * out[c * 16 + k] * out_scale[k];
+        for (int k = 0; k < 5; ++k) q5[k * V + c] += gain * out[k * V + c] * out_scale[k];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) u3[d * V + c] += gain * out[c * 16 + 5 + d] * out_scale[5 + d];
+        for (int d = 0; d < 3; ++d) u3[d * V + c] += gain * out[(5 + d) * V + c] * out_scale[5 + d];
     }
 }
 

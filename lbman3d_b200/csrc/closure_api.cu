@@ -120,11 +120,13 @@ struct lbman_closure {
     double* lpart = nullptr;
     double* loss_hist = nullptr;
     int loss_cap = 0;
+    float *x_in = nullptr, *t_in = nullptr;  // host arrays of forward / gradient calls
+    double* loss_out = nullptr;
     float* scales = nullptr;  // shift[9] inv_scale[9] out_scale[8] inv_out_scale[8]
     float h_shift[9], h_scale[9], h_out[8];
     int* err = nullptr;
     uint32_t wait_limit = lbman::tc::kWaitLimit;  // polls of a pipeline wait before it gives up
-    int Gw = 148, Gb = 296;
+    int Gw = 296, Gb = 1184;
     std::vector<float*> snaps;          // filtered fine states [9V] (rho, u, Q), in recording order
     std::vector<int> traj;              // trajectory id of each snapshot
     std::vector<float*> targets;        // training pairs: target [8V] ...
@@ -150,14 +152,15 @@ int run_conv(lbman_closure* c, cudaStream_t st, const __nv_bfloat16* in, const _
         CL_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         // one block per (column, z range): as many z ranges as keep every
         // column's blocks within one wave of resident blocks (counted from
-        // the SM's shared memory, registers and threads)
+        // the SM's shared memory, registers, threads and TMEM columns)
         const int cols = (c->nx / 8) * (c->ny / 16);
-        const int slots = fit_blocks<K>(c->device, cl::kZThreads, smem) * c->num_sms;
+        const int fit = std::min(fit_blocks<K>(c->device, cl::conv_threads(COUT), smem), 512 / cl::ring_cols(CIN, COUT));
+        const int slots = fit * c->num_sms;
         const int nch = std::max(1, std::min(c->nz, slots / cols));
         const int zc = (c->nz + nch - 1) / nch;
         const int grid = cols * ((c->nz + zc - 1) / zc);
         const cl::Grid3 gr{c->nx, c->ny, c->nz, c->V};
-        K<<<grid, cl::kZThreads, smem, st>>>(gr, zc, in, reinterpret_cast<const uint4*>(img), bias, pre_below,
+        K<<<grid, cl::conv_threads(COUT), smem, st>>>(gr, zc, in, reinterpret_cast<const uint4*>(img), bias, pre_below,
                                              out_pre, out_bf, out_f, c->err, c->wait_limit);
         CL_CUDA(cudaGetLastError());
         return LBMAN_OK;
@@ -176,32 +179,34 @@ int run_conv(lbman_closure* c, cudaStream_t st, const __nv_bfloat16* in, const _
     return LBMAN_OK;
 }
 
+// Weight and bias gradient of one layer into c->g (biases follow weights).
 template <int CIN, int COUT>
 int run_wgrad(lbman_closure* c, cudaStream_t st, const __nv_bfloat16* a, const __nv_bfloat16* gr, int layer) {
     const cl::Grid3 g3{c->nx, c->ny, c->nz, c->V};
+    constexpr int n = 27 * CIN * COUT;
     if (cl::dhalo_ok(c->nx, c->ny)) {
-        using WH = cl::WGradHalo<CIN, COUT>;
-        constexpr auto K = cl::wgrad_dhalo_kernel<CIN, COUT>;
-        CL_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, WH::SMEM));
-        K<<<c->Gw, cl::kThreads, WH::SMEM, st>>>(g3, a, gr, c->wpart, c->err, c->wait_limit);
-    } else {
-        using WS = cl::WGradShape<CIN, COUT>;
-        constexpr auto K = cl::wgrad_kernel<CIN, COUT>;
-        CL_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, WS::SMEM));
-        K<<<c->Gw, cl::kThreads, WS::SMEM, st>>>(g3, a, gr, c->wpart, c->err, c->wait_limit);
+        using WM = cl::WGradMarch<CIN, COUT>;
+        static_assert(WM::NOUT == n + COUT);
+        constexpr auto K = cl::wgrad_march_kernel<CIN, COUT>;
+        const int grid = (int)std::min<int64_t>(c->num_sms, c->V / cl::kTileM);
+        CL_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, WM::SMEM));
+        K<<<grid, cl::kZThreads, WM::SMEM, st>>>(g3, a, gr, c->wpart, c->err, c->wait_limit);
+        CL_CUDA(cudaGetLastError());
+        cl::sum_partials_kernel<<<(WM::NOUT + 31) / 32, cl::kFoldThreads, 0, st>>>(c->wpart, grid, WM::NOUT,
+                                                                                    c->g + w_off(layer));
+        CL_CUDA(cudaGetLastError());
+        return LBMAN_OK;
     }
+    using WS = cl::WGradShape<CIN, COUT>;
+    constexpr auto K = cl::wgrad_kernel<CIN, COUT>;
+    CL_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, WS::SMEM));
+    K<<<c->Gw, cl::kThreads, WS::SMEM, st>>>(g3, a, gr, c->wpart, c->err, c->wait_limit);
     CL_CUDA(cudaGetLastError());
-    const int n = 27 * CIN * COUT;
     cl::sum_partials_kernel<<<(n + 31) / 32, cl::kFoldThreads, 0, st>>>(c->wpart, c->Gw, n, c->g + w_off(layer));
     CL_CUDA(cudaGetLastError());
-    return LBMAN_OK;
-}
-
-template <int C>
-int run_bias_grad(lbman_closure* c, cudaStream_t st, const __nv_bfloat16* gr, int layer) {
-    cl::bias_grad_kernel<C><<<c->Gb, cl::kThreads, 0, st>>>(gr, c->V, c->bpart);
+    cl::bias_grad_kernel<COUT><<<c->Gb, cl::kThreads, 0, st>>>(gr, c->V, c->bpart);
     CL_CUDA(cudaGetLastError());
-    cl::sum_partials_kernel<<<(C + 31) / 32, cl::kFoldThreads, 0, st>>>(c->bpart, c->Gb, C, c->g + b_off(layer));
+    cl::sum_partials_kernel<<<(COUT + 31) / 32, cl::kFoldThreads, 0, st>>>(c->bpart, c->Gb, COUT, c->g + b_off(layer));
     CL_CUDA(cudaGetLastError());
     return LBMAN_OK;
 }
@@ -253,19 +258,15 @@ int forward(lbman_closure* c, cudaStream_t st) {
 // Loss gradient gout must be filled; fills c->g.
 int backward(lbman_closure* c, cudaStream_t st) {
     CL_TRY((run_wgrad<32, 16>(c, st, c->act[2], c->gout, 3)));
-    CL_TRY(run_bias_grad<16>(c, st, c->gout, 3));
     CL_TRY((run_conv<16, 32, cl::kBwdData>(c, st, c->gout, c->bimg[3], nullptr, c->pre[2], nullptr, c->gbuf[0],
                                            nullptr)));
     CL_TRY((run_wgrad<32, 32>(c, st, c->act[1], c->gbuf[0], 2)));
-    CL_TRY(run_bias_grad<32>(c, st, c->gbuf[0], 2));
     CL_TRY((run_conv<32, 32, cl::kBwdData>(c, st, c->gbuf[0], c->bimg[2], nullptr, c->pre[1], nullptr, c->gbuf[1],
                                            nullptr)));
     CL_TRY((run_wgrad<32, 32>(c, st, c->act[0], c->gbuf[1], 1)));
-    CL_TRY(run_bias_grad<32>(c, st, c->gbuf[1], 1));
     CL_TRY((run_conv<32, 32, cl::kBwdData>(c, st, c->gbuf[1], c->bimg[1], nullptr, c->pre[0], nullptr, c->gbuf[0],
                                            nullptr)));
     CL_TRY((run_wgrad<16, 32>(c, st, c->act0, c->gbuf[0], 0)));
-    CL_TRY(run_bias_grad<32>(c, st, c->gbuf[0], 0));
     return LBMAN_OK;
 }
 
@@ -275,12 +276,31 @@ int loss_grad(lbman_closure* c, cudaStream_t st, const float* tgt) {
     return LBMAN_OK;
 }
 
-__global__ void fold_loss_kernel(const double* partials, int G, double scale, double* dst) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int i = 0; i < G; ++i) s += partials[i];
-        *dst = s * scale;
+// Sum of the G block partials, in a fixed tree order.
+constexpr int kFoldLossThreads = 256;
+__global__ void __launch_bounds__(kFoldLossThreads) fold_loss_kernel(const double* partials, int G, double scale,
+                                                                     double* dst) {
+    __shared__ double sh[kFoldLossThreads];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < G; i += kFoldLossThreads) s += partials[i];
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = kFoldLossThreads / 2; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *dst = sh[0] * scale;
+}
+
+// Device copies of the host arrays of lbman_closure_forward / _gradient, kept
+// between calls (allocating and freeing them cost more than the kernels of a
+// 64^3 gradient).
+int ensure_io(lbman_closure* c) {
+    const size_t V = (size_t)c->V;
+    if (!c->x_in) CL_CUDA(cudaMalloc(&c->x_in, 9 * V * sizeof(float)));
+    if (!c->t_in) CL_CUDA(cudaMalloc(&c->t_in, 8 * V * sizeof(float)));
+    if (!c->loss_out) CL_CUDA(cudaMalloc(&c->loss_out, sizeof(double)));
+    return LBMAN_OK;
 }
 
 int check_err(lbman_closure* c) {
@@ -319,7 +339,9 @@ int lbman_closure_create(int device, int nx, int ny, int nz, uint64_t seed, lbma
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) c->num_sms = prop.multiProcessorCount;
     c->Gw = 2 * c->num_sms;  // weight-gradient CTAs (two fit per SM in the staged form)
-    c->Gb = 2 * c->num_sms;
+    // elementwise grids: 8 blocks per SM (at 2 the per-cell kernels of a 64^3 grid
+    // took 19 us each, most of it latency)
+    c->Gb = 8 * c->num_sms;
     for (int j = 0; j < 9; ++j) {
         c->h_shift[j] = j == 0 ? 1.0f : 0.0f;
         c->h_scale[j] = 1.0f;
@@ -339,7 +361,7 @@ int lbman_closure_create(int device, int nx, int ny, int nz, uint64_t seed, lbma
         {(void**)&c->act[0], VB * 32}, {(void**)&c->act[1], VB * 32}, {(void**)&c->act[2], VB * 32},
         {(void**)&c->pre[0], VB * 32}, {(void**)&c->pre[1], VB * 32}, {(void**)&c->pre[2], VB * 32},
         {(void**)&c->gbuf[0], VB * 32}, {(void**)&c->gbuf[1], VB * 32},
-        {(void**)&c->out, (size_t)c->V * 16 * 4},
+        {(void**)&c->out, (size_t)c->V * cl::kOutChannels * 4},
         {(void**)&c->wpart, (size_t)c->Gw * 27 * 32 * 32 * 4}, {(void**)&c->bpart, (size_t)c->Gb * 32 * 4},
         {(void**)&c->lpart, (size_t)c->Gb * 8}, {(void**)&c->scales, 34 * 4}, {(void**)&c->err, sizeof(int)},
     };
@@ -412,7 +434,7 @@ int lbman_closure_destroy(lbman_closure* c) {
     for (float* x : c->rollout_in) cudaFree(x);
     void* ptrs[] = {c->p, c->g, c->m, c->v, c->mask, c->act0, c->gout, c->act[0], c->act[1], c->act[2],
                     c->pre[0], c->pre[1], c->pre[2], c->gbuf[0], c->gbuf[1], c->out, c->wpart, c->bpart,
-                    c->lpart, c->loss_hist, c->scales, c->err};
+                    c->lpart, c->loss_hist, c->scales, c->err, c->x_in, c->t_in, c->loss_out};
     for (void* x : ptrs) cudaFree(x);
     for (int l = 0; l < 4; ++l) {
         cudaFree(c->fimg[l]);
@@ -467,55 +489,35 @@ int lbman_closure_forward(lbman_closure* c, const float* feat9, float* out8) {
     if (!c || !feat9 || !out8) return failc(LBMAN_ERR_ARG, "closure: null argument");
     CL_CUDA(cudaSetDevice(c->device));
     const int64_t V = c->V;
-    float* dx = nullptr;
-    CL_CUDA(cudaMalloc(&dx, 9 * V * sizeof(float)));
-    int s = LBMAN_OK;
-    if (cudaMemcpyAsync(dx, feat9, 9 * V * sizeof(float), cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
-        s = LBMAN_ERR_CUDA;
-    if (s == LBMAN_OK) s = features(c, c->stream, dx, dx + V, dx + 4 * V);
-    if (s == LBMAN_OK) s = forward(c, c->stream);
-    if (s == LBMAN_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) s = LBMAN_ERR_CUDA;
-    if (s == LBMAN_OK) s = check_err(c);
-    if (s == LBMAN_OK) {
-        std::vector<float> o((size_t)V * 16);
-        cudaMemcpy(o.data(), c->out, o.size() * 4, cudaMemcpyDeviceToHost);
-        for (int64_t i = 0; i < V; ++i)
-            for (int j = 0; j < 8; ++j) out8[j * V + i] = o[i * 16 + j];
-    }
-    cudaFree(dx);
-    return s == LBMAN_ERR_CUDA ? failc(s, "closure forward failed") : s;
+    CL_TRY(ensure_io(c));
+    float* dx = c->x_in;
+    CL_CUDA(cudaMemcpyAsync(dx, feat9, 9 * V * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    CL_TRY(features(c, c->stream, dx, dx + V, dx + 4 * V));
+    CL_TRY(forward(c, c->stream));
+    CL_CUDA(cudaStreamSynchronize(c->stream));
+    CL_TRY(check_err(c));
+    CL_CUDA(cudaMemcpy(out8, c->out, (size_t)V * cl::kOutChannels * sizeof(float), cudaMemcpyDeviceToHost));
+    return LBMAN_OK;
 }
 
 int lbman_closure_gradient(lbman_closure* c, const float* feat9, const float* target8, double* loss, float* grad) {
     if (!c || !feat9 || !target8) return failc(LBMAN_ERR_ARG, "closure: null argument");
     CL_CUDA(cudaSetDevice(c->device));
     const int64_t V = c->V;
-    float *dx = nullptr, *dt = nullptr;
-    double* dl = nullptr;
-    CL_CUDA(cudaMalloc(&dx, 9 * V * sizeof(float)));
-    int s = LBMAN_OK;
-    if (cudaMalloc(&dt, 8 * V * sizeof(float)) != cudaSuccess || cudaMalloc(&dl, sizeof(double)) != cudaSuccess)
-        s = LBMAN_ERR_NOMEM;
-    if (s == LBMAN_OK && (cudaMemcpyAsync(dx, feat9, 9 * V * 4, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
-                          cudaMemcpyAsync(dt, target8, 8 * V * 4, cudaMemcpyHostToDevice, c->stream) != cudaSuccess))
-        s = LBMAN_ERR_CUDA;
-    if (s == LBMAN_OK) s = features(c, c->stream, dx, dx + V, dx + 4 * V);
-    if (s == LBMAN_OK) s = forward(c, c->stream);
-    if (s == LBMAN_OK) s = loss_grad(c, c->stream, dt);
-    if (s == LBMAN_OK) {
-        fold_loss_kernel<<<1, 32, 0, c->stream>>>(c->lpart, c->Gb, 1.0 / (8.0 * (double)V), dl);
-        s = backward(c, c->stream);
-    }
-    if (s == LBMAN_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) s = LBMAN_ERR_CUDA;
-    if (s == LBMAN_OK) s = check_err(c);
-    if (s == LBMAN_OK) {
-        if (loss) cudaMemcpy(loss, dl, sizeof(double), cudaMemcpyDeviceToHost);
-        if (grad) cudaMemcpy(grad, c->g, kNParams * sizeof(float), cudaMemcpyDeviceToHost);
-    }
-    cudaFree(dx);
-    cudaFree(dt);
-    cudaFree(dl);
-    return s == LBMAN_ERR_CUDA ? failc(s, "closure gradient failed") : s;
+    CL_TRY(ensure_io(c));
+    float* dx = c->x_in;
+    CL_CUDA(cudaMemcpyAsync(dx, feat9, 9 * V * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    CL_TRY(features(c, c->stream, dx, dx + V, dx + 4 * V));
+    CL_TRY(forward(c, c->stream));
+    CL_CUDA(cudaMemcpyAsync(c->t_in, target8, 8 * V * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    CL_TRY(loss_grad(c, c->stream, c->t_in));
+    fold_loss_kernel<<<1, kFoldLossThreads, 0, c->stream>>>(c->lpart, c->Gb, 1.0 / (8.0 * (double)V), c->loss_out);
+    CL_TRY(backward(c, c->stream));
+    CL_CUDA(cudaStreamSynchronize(c->stream));
+    CL_TRY(check_err(c));
+    if (loss) CL_CUDA(cudaMemcpy(loss, c->loss_out, sizeof(double), cudaMemcpyDeviceToHost));
+    if (grad) CL_CUDA(cudaMemcpy(grad, c->g, kNParams * sizeof(float), cudaMemcpyDeviceToHost));
+    return LBMAN_OK;
 }
 
 // Box-filters the fine state of v onto the coarse grid as a new snapshot of
@@ -743,7 +745,8 @@ int lbman_closure_train(lbman_closure* c, int iters, float lr, uint64_t seed, do
         CL_TRY(features(c, c->stream, x, x + V, x + 4 * V, c->train_noise, st));
         CL_TRY(forward(c, c->stream));
         CL_TRY(loss_grad(c, c->stream, c->targets[pi]));
-        fold_loss_kernel<<<1, 32, 0, c->stream>>>(c->lpart, c->Gb, 1.0 / (8.0 * (double)V), c->loss_hist + it);
+        fold_loss_kernel<<<1, kFoldLossThreads, 0, c->stream>>>(c->lpart, c->Gb, 1.0 / (8.0 * (double)V),
+                                                              c->loss_hist + it);
         CL_TRY(backward(c, c->stream));
         ++c->adam_t;
         const float bc1 = 1.0f - std::pow(b1, (float)c->adam_t), bc2 = 1.0f - std::pow(b2, (float)c->adam_t);
