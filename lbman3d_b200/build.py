@@ -42,6 +42,8 @@ UNITS = {
     "kernels_point_f64.cu": ["--fmad=false"],
     "kernels_ens.cu": [],
     "kernels_ens_f64.cu": ["--fmad=false"],
+    "kernels_ens_point.cu": [],
+    "kernels_ens_point_f64.cu": ["--fmad=false"],
     "api.cu": [],
     "ens_api.cu": [],
     "noalloc.cu": [],

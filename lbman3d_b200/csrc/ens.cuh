@@ -2,18 +2,23 @@
 // boundary configurations and physical parameters advanced together.
 //
 // Every box is described by an EnsBox in device memory (its own SimParams
-// and field pointers).  The host flattens all boxes into work lists -- one
-// item per z-marching block of the Q+force kernel, one per 256-cell block of
-// the LBM kernel -- and each launch covers every box: a persistent grid of
-// blocks strides through the list, running the same march / gather-collide
-// code as the single-box kernels on the item's box.  A time step of the whole
-// ensemble is therefore one launch per kernel (two in the split organisation,
-// one fused), which the host replays from a CUDA graph.  There is no
+// and field pointers).  The host flattens all boxes into work lists, and each
+// launch covers every box, running the code of the single-box kernels on the
+// item's box, so the results are the single-box ones bit for bit.  There is no
 // communication between boxes.
+//
+//   split   ens_qpoint_kernel, then ens_lbm_point_kernel (the time step of
+//           qpoint.cuh, in-place streaming): one block per work item;
+//   fused   ens_fused_kernel (fused.cuh): a persistent grid of z-marching blocks
+//           strides through the list.
+//
+// A time step of the whole ensemble is therefore two launches (split) or one
+// (fused), which the host replays from a CUDA graph.
 #pragma once
 
 #include "fused.cuh"
 #include "lbm.cuh"
+#include "qpoint.cuh"
 
 namespace lbman {
 
@@ -22,52 +27,95 @@ struct EnsBox {
     FastDiv dnx, dnxy;
     void* q[2];   // Q, double buffered
     void* u[2];   // u, double buffered (fused); the split organisation uses u[0] only
-    void* f[2];   // populations, double buffered
+    void* f[2];   // populations; the second buffer only for the fused organisation
     void* rho;
     void* F;
-    int zc;       // z chunk of this box's Q work items
+    void* stress; // between the split organisation's two kernels
+    int zc;       // z chunk of this box's fused work items
+    int mask;     // wall-rule mask of the split kernels (point_mask)
 };
+static_assert(sizeof(EnsBox) % 4 == 0, "copied to shared memory as 32-bit words");
 
 struct EnsQWork {
     int box, bx, by, bz;
 };
+struct EnsPointWork {
+    int box, block, z0, z1;  // 128 columns of the planes [z0, z1)
+};
 struct EnsLbmWork {
-    int box, block;
+    int box, block;  // kEnsLbmCells cells
 };
 
-template <class TL, class R, bool UPWIND>
-__global__ void __launch_bounds__(TL::NT, (Stage<TL, R>::MINB)) ens_qforce_kernel(const EnsBox* __restrict__ boxes,
-                                                            const EnsQWork* __restrict__ work, int nwork,
-                                                            int par) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    // The item's box parameters, copied to shared memory once per item: the
-    // z march reads them throughout, and a global-memory copy would cost a
-    // load per use where a single-box launch reads its constant bank.  Every
-    // tile whose staging fits one block (227 KB) leaves room for the copy
-    // (largest: FP64 32x8, 216 672 B staging + 1 368 B of parameters).
-    static_assert(Stage<TL, R>::bytes + sizeof(SimParams) + 1024 <= 227 * 1024,
-                  "the box parameters must fit beside the tile's staging");
-    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
-        const EnsQWork it = work[w];
-        const EnsBox& B = boxes[it.box];
-        const int z0 = it.bz * B.zc;
-        __shared__ __align__(16) uint32_t pbuf[sizeof(SimParams) / 4];
-        const SimParams& Ps = *reinterpret_cast<const SimParams*>(pbuf);
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(&B.P);
-        for (int i = threadIdx.x; i < (int)(sizeof(SimParams) / 4); i += blockDim.x) pbuf[i] = src[i];
-        __syncthreads();
-        if (z0 < Ps.nz)
-            qf_march<TL, R, UPWIND>(Ps, it.bx * TL::TCX, it.by * TL::TCY, z0, min(z0 + B.zc, Ps.nz),
-                                    (const R*)B.q[par], (const R*)B.u[0], reinterpret_cast<R*>(smem_raw),
-                                    StoreQForce<R>{(R*)B.q[1 - par], (R*)B.F, Ps.V});
-        __syncthreads();  // the staging rings and the parameters are reused by the next item
-    }
+// A work item's box, copied to shared memory: a single-box launch reads its
+// parameters from the constant bank, a global-memory copy would cost a load
+// per use.
+__device__ __forceinline__ const EnsBox& ens_box(const EnsBox* __restrict__ boxes, int box, uint32_t* buf) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(boxes + box);
+    for (int i = threadIdx.x; i < (int)(sizeof(EnsBox) / 4); i += blockDim.x) buf[i] = src[i];
+    __syncthreads();
+    return *reinterpret_cast<const EnsBox*>(buf);
+}
+
+// Calls f with the compile-time mask that `mask` (block-uniform) names.
+template <class F>
+__device__ __forceinline__ void ens_with_mask(int mask, F&& f) {
+    if (mask == 0) f(std::integral_constant<int, 0>{});
+    else if (mask == QW_X) f(std::integral_constant<int, QW_X>{});
+    else if (mask == (QW_X | QW_Y)) f(std::integral_constant<int, QW_X | QW_Y>{});
+    else f(std::integral_constant<int, 15>{});
+}
+
+template <class R, bool UPWIND>
+__global__ void __launch_bounds__(kPointThreads, point_min_blocks<R>())
+    ens_qpoint_kernel(const EnsBox* __restrict__ boxes, const EnsPointWork* __restrict__ work, int par) {
+    __shared__ __align__(16) uint32_t buf[sizeof(EnsBox) / 4];
+    const EnsPointWork it = work[blockIdx.x];
+    const EnsBox& B = ens_box(boxes, it.box, buf);
+    const SimParams& P = B.P;
+    const int n = (int)P.nxy;
+    int col = it.block * kPointThreads + threadIdx.x;
+    const bool live = col < n;
+    if (!live) col = n - 1;
+    const int y = (int)fdiv((uint32_t)col, B.dnx), x = col - y * P.nx;
+    ens_with_mask(B.mask, [&](auto m) {
+        qpoint_column<R, UPWIND, decltype(m)::value>(P, x, y, col, it.z0, it.z1, live, (const R*)B.q[par],
+                                                     (const R*)B.u[0], (R*)B.q[1 - par], (R*)B.stress, (R*)B.F);
+    });
+}
+
+// Cells of an LBM work item: enough that the box's parameters are copied once
+// per 4 cells of a thread.
+constexpr int kEnsLbmCells = 4 * kPointThreads;
+
+// par: the buffer holding Q_new.
+template <class R, class S, bool DEV, bool ODD>
+__global__ void __launch_bounds__(kPointThreads)
+    ens_lbm_point_kernel(const EnsBox* __restrict__ boxes, const EnsLbmWork* __restrict__ work, int par, int fcur,
+                         int last) {
+    __shared__ __align__(16) uint32_t buf[sizeof(EnsBox) / 4];
+    const EnsLbmWork it = work[blockIdx.x];
+    const EnsBox& B = ens_box(boxes, it.box, buf);
+    const SimParams& P = B.P;
+    const int c0 = it.block * kEnsLbmCells + threadIdx.x, c1 = min((it.block + 1) * kEnsLbmCells, (int)P.V);
+    S* f = (S*)(fcur ? B.f[1] : B.f[0]);
+    const R* qn = (const R*)(par ? B.q[1] : B.q[0]);
+    ens_with_mask(B.mask, [&](auto m) {
+        constexpr int QW = decltype(m)::value, WM = QW & 7;
+        const KeptPointForce<R, QW, false> force{{P, qn, (const R*)B.stress, (const R*)B.u[0], (const R*)B.F}, (R*)B.F, last};
+#pragma unroll 1
+        for (int c = c0; c < c1; c += kPointThreads) {
+            if constexpr (ODD)
+                aa_odd_cell<R, S, DEV, WM, int>(P, B.dnx, B.dnxy, c, f, force, (R*)B.rho, (R*)B.u[0], last);
+            else
+                aa_even_cell<R, S, DEV, WM, int>(P, B.dnx, B.dnxy, c, f, force, (R*)B.rho, (R*)B.u[0], last);
+        }
+    });
 }
 
 template <class TL, class R, class S, bool DEV, bool UPWIND>
 __global__ void __launch_bounds__(TL::NT) ens_fused_kernel(const EnsBox* __restrict__ boxes,
                                                            const EnsQWork* __restrict__ work, int nwork, int par,
-                                                           int first, int write_rho_all) {
+                                                           int fcur, int first, int write_rho_all) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const EnsQWork it = work[w];
@@ -77,50 +125,9 @@ __global__ void __launch_bounds__(TL::NT) ens_fused_kernel(const EnsBox* __restr
             qf_march<TL, R, UPWIND>(B.P, it.bx * TL::TCX, it.by * TL::TCY, z0, min(z0 + B.zc, B.P.nz),
                                     (const R*)B.q[par], (const R*)B.u[par], reinterpret_cast<R*>(smem_raw),
                                     CollideCell<R, S, DEV>{B.P, phys_ref<R>(B.P), first, (R*)B.q[1 - par],
-                                                           (R*)B.u[1 - par], (const S*)B.f[par],
-                                                           (S*)B.f[1 - par], (R*)B.rho, nullptr, write_rho_all});
+                                                           (R*)B.u[1 - par], (const S*)B.f[fcur],
+                                                           (S*)B.f[1 - fcur], (R*)B.rho, nullptr, write_rho_all});
         __syncthreads();
-    }
-}
-
-// Held to the single-box walled LBM kernel's register budget (5 blocks per SM
-// for FP32 compute, 2 for FP64); each work item's box picks the periodic or the
-// walled gather (block-uniform).
-template <class R, class S, bool DEV>
-__global__ void __launch_bounds__(256, lbm_min_blocks<R, S, true>()) ens_lbm_kernel(const EnsBox* __restrict__ boxes,
-                                                      const EnsLbmWork* __restrict__ work, int nwork, int par,
-                                                      int first, int write_rho_all) {
-    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
-        const EnsLbmWork it = work[w];
-        const EnsBox& B = boxes[it.box];
-        const SimParams& P = B.P;
-        const int64_t c = (int64_t)it.block * blockDim.x + threadIdx.x;
-        if (c >= P.V) continue;
-        const int64_t V = P.V;
-        const Phys<R>& K = phys_ref<R>(P);
-        CellPos q;
-        q.z = (int)fdiv((uint32_t)c, B.dnxy);
-        const uint32_t r = (uint32_t)(c - (int64_t)q.z * P.nxy);
-        q.y = (int)fdiv(r, B.dnx);
-        q.x = (int)(r - (uint32_t)q.y * (uint32_t)P.nx);
-        const bool mv = P.moving_any && touches_moving(P, q.x, q.y, q.z);
-        R* rho_buf = (R*)B.rho;
-        const R* F = (const R*)B.F;
-        R f[15];
-        if (P.uper[0] && P.uper[2] && P.uper[4])
-            load_pre<R, S, false>(P, K, first != 0, (const S*)B.f[par], c, q, R(0), f);
-        else
-            load_pre<R, S, true>(P, K, first != 0, (const S*)B.f[par], c, q, (mv && !first) ? rho_buf[c] : R(0), f);
-        R rho, ux, uy, uz;
-        collide<R, DEV>(K, f, F[c], F[V + c], F[2 * V + c], rho, ux, uy, uz);
-        S* fout = (S*)B.f[1 - par];
-#pragma unroll
-        for (int j = 0; j < 15; ++j) Store<S>::st(fout + j * V + c, f[j]);
-        R* u = (R*)B.u[0];
-        u[c] = ux;
-        u[V + c] = uy;
-        u[2 * V + c] = uz;
-        if (write_rho_all || mv) rho_buf[c] = rho;
     }
 }
 

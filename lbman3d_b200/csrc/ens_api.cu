@@ -13,6 +13,7 @@
 #include "ens_launch.h"
 #include "solver_view.h"
 #include "launch.h"
+#include "point_launch.cuh"
 #include "tiles.h"
 
 namespace lbman {
@@ -40,8 +41,9 @@ int efail(int code, const char* msg) {
     } while (0)
 
 struct PrecOps {
-    decltype(&ens_qstep_f64) qstep;
-    decltype(&ens_lbm_f64) lbm;
+    decltype(&ens_qpoint_f64) qpoint;
+    decltype(&ens_lbm_point_f64) lbm_point;
+    decltype(&ens_fused_f64) fused;
     decltype(&ens_prepare_f64) prepare;
     decltype(&ens_blocks_per_sm_f64) blocks_per_sm;
     decltype(&launch_seeded_init_f64) seeded_init;
@@ -51,17 +53,24 @@ struct PrecOps {
     decltype(&launch_pop_in_f64) pop_in;
     decltype(&launch_pop_out_f64) pop_out;
     decltype(&launch_stream_only_f64) stream_only;
+    decltype(&launch_aa_pop_out_f64) aa_pop_out;
+    decltype(&launch_swap_pairs_f64) swap_pairs;
     decltype(&qforce_smem_f64) qforce_smem;
     decltype(&qforce_threads_f64) qforce_threads;
 };
-#define ENS_OPS(S)                                                                                          \
+// Q: the suffix of the Q stage's kernels (FP16 storage computes in FP32)
+#define ENS_OPS(S, Q)                                                                                       \
     PrecOps {                                                                                               \
-        ens_qstep_##S, ens_lbm_##S, ens_prepare_##S, ens_blocks_per_sm_##S, launch_seeded_init_##S,         \
-            launch_feq_init_##S, launch_real_in_##S, launch_real_out_##S, launch_pop_in_##S,                \
-            launch_pop_out_##S, launch_stream_only_##S, qforce_smem_##S, qforce_threads_##S                 \
+        ens_qpoint_##Q, ens_lbm_point_##S, ens_fused_##S, ens_prepare_##S, ens_blocks_per_sm_##S,           \
+            launch_seeded_init_##S, launch_feq_init_##S, launch_real_in_##S, launch_real_out_##S,           \
+            launch_pop_in_##S, launch_pop_out_##S, launch_stream_only_##S, launch_aa_pop_out_##S,           \
+            launch_swap_pairs_##S, qforce_smem_##S, qforce_threads_##S                                      \
     }
-const PrecOps kEnsOps[3] = {ENS_OPS(f64), ENS_OPS(f32), ENS_OPS(f16)};
+const PrecOps kEnsOps[3] = {ENS_OPS(f64, f64), ENS_OPS(f32, f32), ENS_OPS(f16, f32)};
 
+// Layout of the populations, as for a single box: pre-collision, post-collision
+// of the two-buffer (fused) kernels, post-collision in place.
+enum { F_PRE = 0, F_POST = 1, F_SWAP = 2 };
 
 }  // namespace
 
@@ -76,15 +85,17 @@ struct lbman_ensemble {
     int64_t maxV = 0, cells = 0;
     // launch shape, work lists
     int kernels = LBMAN_KERNELS_SPLIT, tcx = 32, tcy = 6, zc_target = 0;
-    EnsQWork* qwork = nullptr;
+    EnsQWork* qwork = nullptr;       // fused
+    EnsPointWork* pwork = nullptr;   // split
     EnsLbmWork* lwork = nullptr;
-    int nq = 0, nl = 0, qgrid = 0, lgrid = 0;
-    int par = 0;
-    bool uploaded = false, f_post = false;
+    int nq = 0, np = 0, nl = 0, qgrid = 0;
+    bool small = true;               // every box within the split kernels' 32-bit indices
+    int par = 0, fcur = 0, fphase = F_PRE;
+    bool uploaded = false, stepped = false;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaGraphExec_t graph = nullptr;
-    int graph_steps = 0, graph_par = -1;
+    int graph_steps = 0, graph_par = -1, graph_fphase = -1;
     int64_t steps = 0, launches = 0;
     const PrecOps& ops() const { return kEnsOps[prec]; }
 };
@@ -98,13 +109,61 @@ void drop_graph(lbman_ensemble* e) {
     e->graph_par = -1;
 }
 
-// Work lists for the current tile: one Q item per z-marching block of each
-// box, one LBM item per 256-cell block of each box.
+// Second population and velocity buffers of the fused organisation, or the
+// stress of the split one, on first use (build_work uploads the pointers).
+int ensure_buffers(lbman_ensemble* e) {
+    const bool fused = e->kernels == LBMAN_KERNELS_FUSED;
+    const size_t words = e->prec == LBMAN_FP64 ? point_stress_words<double>() : point_stress_words<float>();
+    for (EnsBox& B : e->host) {
+        const int64_t V = B.P.V;
+        struct { void** p; size_t n; bool want; } want[] = {
+            {&B.f[1], 15 * V * e->sbytes, fused}, {&B.stress, words * V * e->rbytes, !fused}};
+        for (auto& w : want) {
+            if (!w.want || *w.p) continue;
+            if (cudaMalloc(w.p, w.n) != cudaSuccess) {
+                cudaGetLastError();
+                *w.p = nullptr;
+                return efail(LBMAN_ERR_NOMEM, "cudaMalloc of an ensemble buffer failed");
+            }
+            e->allocs.push_back(*w.p);
+        }
+    }
+    return LBMAN_OK;
+}
+
+template <class T>
+int upload_list(lbman_ensemble* e, const std::vector<T>& v, T** d) {
+    cudaFree(*d);
+    *d = nullptr;
+    if (v.empty()) return LBMAN_OK;
+    E_CUDA(cudaMalloc(d, v.size() * sizeof(T)));
+    // On the ensemble's (non-blocking) stream and waited for by the caller: a
+    // plain cudaMemcpy from pageable memory may return before its DMA lands, and
+    // the legacy stream does not order the kernels queued on this one.
+    E_CUDA(cudaMemcpyAsync(*d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, e->stream));
+    return LBMAN_OK;
+}
+
+// Work lists of the current organisation: one item per z-marching block of
+// each box (fused), or one per 128 columns x kWalk planes and one per
+// kEnsLbmCells cells (split).
 int build_work(lbman_ensemble* e) {
+    constexpr int kWalk = 4;  // planes per thread, as in a large single box
+    if (int st = ensure_buffers(e)) return st;
     std::vector<EnsQWork> q;
+    std::vector<EnsPointWork> p;
     std::vector<EnsLbmWork> l;
+    const bool fused = e->kernels == LBMAN_KERNELS_FUSED;
     for (int b = 0; b < e->n; ++b) {
         EnsBox& B = e->host[b];
+        if (!fused) {
+            const int cb = (int)((B.P.nxy + kPointThreads - 1) / kPointThreads);
+            for (int z = 0; z < B.P.nz; z += kWalk)
+                for (int k = 0; k < cb; ++k) p.push_back({b, k, z, std::min(z + kWalk, B.P.nz)});
+            const int lb = (int)((B.P.V + kEnsLbmCells - 1) / kEnsLbmCells);
+            for (int k = 0; k < lb; ++k) l.push_back({b, k});
+            continue;
+        }
         const int gx = (B.P.nx + e->tcx - 1) / e->tcx, gy = (B.P.ny + e->tcy - 1) / e->tcy;
         int zc = e->zc_target > 0 ? std::min(e->zc_target, B.P.nz) : B.P.nz;
         if (e->zc_target <= 0) {  // enough z chunks that big boxes split across SMs
@@ -117,57 +176,74 @@ int build_work(lbman_ensemble* e) {
         for (int z = 0; z < gz; ++z)
             for (int y = 0; y < gy; ++y)
                 for (int x = 0; x < gx; ++x) q.push_back({b, x, y, z});
-        const int lb = (int)((B.P.V + 255) / 256);
-        for (int k = 0; k < lb; ++k) l.push_back({b, k});
     }
     // largest boxes first: long items start early, short ones fill the tail
     std::stable_sort(q.begin(), q.end(), [&](const EnsQWork& a, const EnsQWork& c) {
         return e->host[a.box].P.V > e->host[c.box].P.V;
     });
-    cudaFree(e->qwork);
-    cudaFree(e->lwork);
-    e->qwork = nullptr;
-    e->lwork = nullptr;
-    E_CUDA(cudaMalloc(&e->qwork, q.size() * sizeof(EnsQWork)));
-    E_CUDA(cudaMalloc(&e->lwork, l.size() * sizeof(EnsLbmWork)));
-    // On the ensemble's (non-blocking) stream and waited for: a plain
-    // cudaMemcpy from pageable memory may return before its DMA lands, and
-    // the legacy stream does not order the kernels queued on this one.
-    E_CUDA(cudaMemcpyAsync(e->qwork, q.data(), q.size() * sizeof(EnsQWork), cudaMemcpyHostToDevice, e->stream));
-    E_CUDA(cudaMemcpyAsync(e->lwork, l.data(), l.size() * sizeof(EnsLbmWork), cudaMemcpyHostToDevice, e->stream));
+    if (int st = upload_list(e, q, &e->qwork)) return st;
+    if (int st = upload_list(e, p, &e->pwork)) return st;
+    if (int st = upload_list(e, l, &e->lwork)) return st;
     E_CUDA(cudaMemcpyAsync(e->dboxes, e->host.data(), e->n * sizeof(EnsBox), cudaMemcpyHostToDevice, e->stream));
     E_CUDA(cudaStreamSynchronize(e->stream));
     e->nq = (int)q.size();
+    e->np = (int)p.size();
     e->nl = (int)l.size();
-    const int bps = std::max(1, e->ops().blocks_per_sm(e->tcx, e->tcy, e->kernels == LBMAN_KERNELS_FUSED));
-    e->qgrid = std::max(1, std::min(e->nq, bps * e->num_sms));
-    e->lgrid = std::max(1, std::min(e->nl, 8 * e->num_sms));
+    if (fused) {
+        const int bps = std::max(1, e->ops().blocks_per_sm(e->tcx, e->tcy));
+        e->qgrid = std::max(1, std::min(e->nq, bps * e->num_sms));
+    }
     drop_graph(e);
+    return LBMAN_OK;
+}
+
+// Post-collision populations of every box between the two-buffer and the
+// in-place layout.
+int ens_layout(lbman_ensemble* e, int phase) {
+    for (EnsBox& B : e->host)
+        if (e->ops().swap_pairs(B.P, B.f[e->fcur], e->stream) != cudaSuccess)
+            return efail(LBMAN_ERR_CUDA, "layout conversion failed");
+    e->launches += e->n;
+    e->fphase = phase;
     return LBMAN_OK;
 }
 
 // One time step of every box (no graph).
 int ens_step_once(lbman_ensemble* e, bool last) {
-    const int first = e->f_post ? 0 : 1;
-    EnsQLaunch L{e->dboxes, e->qwork, e->nq, e->tcx, e->tcy, e->kernels == LBMAN_KERNELS_FUSED, e->upwind,
-                 e->par, first, last ? 1 : 0, e->qgrid};
-    cudaError_t err = e->ops().qstep(L, e->stream);
-    ++e->launches;
-    if (err == cudaSuccess && e->kernels == LBMAN_KERNELS_SPLIT) {
-        err = e->ops().lbm(e->dboxes, e->lwork, e->nl, e->par, first, last ? 1 : 0, e->lgrid, e->stream);
+    cudaError_t err;
+    if (e->kernels == LBMAN_KERNELS_FUSED) {
+        if (e->fphase == F_SWAP)
+            if (int st = ens_layout(e, F_POST)) return st;
+        const EnsFusedLaunch L{e->dboxes, e->qwork, e->nq, e->tcx, e->tcy, e->upwind, e->par, e->fcur,
+                               e->fphase == F_PRE ? 1 : 0, last ? 1 : 0, e->qgrid};
+        err = e->ops().fused(L, e->stream);
         ++e->launches;
+        e->fcur ^= 1;
+        e->fphase = F_POST;
+    } else {
+        if (e->fphase == F_POST)
+            if (int st = ens_layout(e, F_SWAP)) return st;
+        const bool odd = e->fphase == F_SWAP;
+        err = e->ops().qpoint(e->dboxes, e->pwork, e->np, e->upwind, e->par, e->stream);
+        ++e->launches;
+        if (err == cudaSuccess) {
+            err = e->ops().lbm_point(e->dboxes, e->lwork, e->nl, 1 - e->par, e->fcur, odd, last, e->stream);
+            ++e->launches;
+        }
+        e->fphase = odd ? F_PRE : F_SWAP;
     }
     if (err != cudaSuccess) return efail(LBMAN_ERR_CUDA, cudaGetErrorString(err));
     e->par ^= 1;
-    e->f_post = true;
+    e->stepped = true;
     ++e->steps;
     return LBMAN_OK;
 }
 
-// Graph of k steps starting at parity e->par (after the first step).
+// Graph of k steps (k even, so a replay keeps the buffers and the layout it
+// started from) from the current parity and layout.
 int ens_build_graph(lbman_ensemble* e, int k) {
     drop_graph(e);
-    const int par0 = e->par;
+    const int par0 = e->par, fcur0 = e->fcur, fphase0 = e->fphase;
     const int64_t steps0 = e->steps, launches0 = e->launches;
     cudaGraph_t g = nullptr;
     E_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
@@ -175,6 +251,8 @@ int ens_build_graph(lbman_ensemble* e, int k) {
     for (int i = 0; i < k && st == LBMAN_OK; ++i) st = ens_step_once(e, false);
     cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
     e->par = par0;
+    e->fcur = fcur0;
+    e->fphase = fphase0;
     e->steps = steps0;
     e->launches = launches0;
     if (st != LBMAN_OK) {
@@ -187,6 +265,7 @@ int ens_build_graph(lbman_ensemble* e, int k) {
     if (ie != cudaSuccess) return efail(LBMAN_ERR_CUDA, cudaGetErrorString(ie));
     e->graph_steps = k;
     e->graph_par = par0;
+    e->graph_fphase = fphase0;
     return LBMAN_OK;
 }
 
@@ -259,18 +338,23 @@ int lbman_ensemble_create(const lbman_config* cfgs, int nboxes, lbman_ensemble**
         build_sim_params(cfgs[b], B.P);
         B.dnx = make_fastdiv((uint32_t)B.P.nx);
         B.dnxy = make_fastdiv((uint32_t)B.P.nxy);
+        B.mask = impl::point_mask(B.P);
         const int64_t V = B.P.V;
         e->maxV = std::max(e->maxV, V);
         e->cells += V;
-        void** slots[8] = {&B.q[0], &B.q[1], &B.u[0], &B.u[1], &B.f[0], &B.f[1], &B.rho, &B.F};
-        const size_t sizes[8] = {5 * V * e->rbytes, 5 * V * e->rbytes, 3 * V * e->rbytes, 3 * V * e->rbytes,
-                                 15 * V * e->sbytes, 15 * V * e->sbytes, V * e->rbytes, 3 * V * e->rbytes};
-        for (int k = 0; k < 8; ++k) {
+        // the split kernels index 15 V in 32 bits; with a larger box among
+        // them the ensemble steps with the fused kernels (the same results)
+        e->small = e->small && 15 * V < ((int64_t)1 << 31);
+        void** slots[7] = {&B.q[0], &B.q[1], &B.u[0], &B.u[1], &B.f[0], &B.rho, &B.F};
+        const size_t sizes[7] = {5 * V * e->rbytes, 5 * V * e->rbytes, 3 * V * e->rbytes, 3 * V * e->rbytes,
+                                 15 * V * e->sbytes, V * e->rbytes, 3 * V * e->rbytes};
+        for (int k = 0; k < 7; ++k) {
             if (cudaMalloc(slots[k], sizes[k]) != cudaSuccess)
                 return bail(efail(LBMAN_ERR_NOMEM, "cudaMalloc of an ensemble box failed"));
             e->allocs.push_back(*slots[k]);
         }
     }
+    if (!e->small) e->kernels = LBMAN_KERNELS_FUSED;
     if (cudaMalloc(&e->staging, e->maxV * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&e->dboxes, nboxes * sizeof(EnsBox)) != cudaSuccess)
         return bail(efail(LBMAN_ERR_NOMEM, "cudaMalloc failed"));
@@ -291,6 +375,7 @@ int lbman_ensemble_destroy(lbman_ensemble* e) {
     cudaFree(e->staging);
     cudaFree(e->dboxes);
     cudaFree(e->qwork);
+    cudaFree(e->pwork);
     cudaFree(e->lwork);
     if (e->own_stream && e->stream) cudaStreamDestroy(e->stream);
     delete e;
@@ -317,7 +402,7 @@ int lbman_ensemble_init_seeded(lbman_ensemble* e, uint64_t seed, double sigma) {
 int lbman_ensemble_init_seeded_each(lbman_ensemble* e, const uint64_t* seeds, double sigma) {
     if (!e || !seeds) return efail(LBMAN_ERR_ARG, "null argument");
     E_CUDA(cudaSetDevice(e->device));
-    e->par = 0;
+    e->par = e->fcur = 0;
     for (int b = 0; b < e->n; ++b) {
         EnsBox& B = e->host[b];
         const SimParams& P = B.P;
@@ -331,7 +416,8 @@ int lbman_ensemble_init_seeded_each(lbman_ensemble* e, const uint64_t* seeds, do
     }
     E_CUDA(cudaStreamSynchronize(e->stream));
     e->uploaded = true;
-    e->f_post = false;
+    e->fphase = F_PRE;
+    e->stepped = false;
     e->steps = 0;
     drop_graph(e);
     return LBMAN_OK;
@@ -339,7 +425,7 @@ int lbman_ensemble_init_seeded_each(lbman_ensemble* e, const uint64_t* seeds, do
 
 int lbman_ensemble_upload(lbman_ensemble* e, int box, const double* rho, const double* u3, const double* q5) {
     if (!e || box < 0 || box >= e->n || !rho || !u3 || !q5) return efail(LBMAN_ERR_ARG, "bad arguments");
-    if (e->uploaded && e->f_post) return efail(LBMAN_ERR_STATE, "boxes are uploaded before the first step");
+    if (e->uploaded && e->stepped) return efail(LBMAN_ERR_STATE, "boxes are uploaded before the first step");
     E_CUDA(cudaSetDevice(e->device));
     EnsBox& B = e->host[box];
     const SimParams& P = B.P;
@@ -357,7 +443,7 @@ int lbman_ensemble_upload(lbman_ensemble* e, int box, const double* rho, const d
         }
         return LBMAN_OK;
     };
-    e->par = 0;
+    e->par = e->fcur = 0;
     if (int st = in(rho, B.rho, V)) return st;
     if (int st = in(u3, B.u[0], 3 * V)) return st;
     if (int st = in(q5, B.q[0], 5 * V)) return st;
@@ -367,7 +453,8 @@ int lbman_ensemble_upload(lbman_ensemble* e, int box, const double* rho, const d
         return efail(LBMAN_ERR_CUDA, "f_eq initialisation failed");
     E_CUDA(cudaStreamSynchronize(e->stream));
     e->uploaded = true;
-    e->f_post = false;
+    e->fphase = F_PRE;
+    e->stepped = false;
     e->steps = 0;
     drop_graph(e);
     return LBMAN_OK;
@@ -401,18 +488,19 @@ int lbman_ensemble_download(lbman_ensemble* e, int box, double* rho, double* u3,
     if (u3) if (int st = out(u, u3, 3 * V)) return st;
     if (q5) if (int st = out(B.q[p], q5, 5 * V)) return st;
     if (f15) {
-        const void* src = B.f[p];
-        if (e->f_post) {
-            if (e->ops().stream_only(P, B.f[p], B.f[1 - p], B.rho, e->stream) != cudaSuccess)
+        const void* src = B.f[e->fcur];
+        if (e->fphase == F_POST) {
+            if (e->ops().stream_only(P, src, B.f[1 - e->fcur], B.rho, e->stream) != cudaSuccess)
                 return efail(LBMAN_ERR_CUDA, "stream failed");
-            src = B.f[1 - p];
+            src = B.f[1 - e->fcur];
         }
         for (int j = 0; j < 15; ++j) {
-            if (e->prec == LBMAN_FP64) {
+            if (e->fphase != F_SWAP && e->prec == LBMAN_FP64) {
                 E_CUDA(cudaMemcpyAsync(f15 + j * V, (const char*)src + j * V * 8, V * 8, cudaMemcpyDeviceToHost, e->stream));
             } else {
-                if (e->ops().pop_out(P, src, e->staging, j, e->stream) != cudaSuccess)
-                    return efail(LBMAN_ERR_CUDA, "conversion failed");
+                const cudaError_t err = e->fphase == F_SWAP ? e->ops().aa_pop_out(P, src, B.rho, e->staging, j, e->stream)
+                                                            : e->ops().pop_out(P, src, e->staging, j, e->stream);
+                if (err != cudaSuccess) return efail(LBMAN_ERR_CUDA, "conversion failed");
                 E_CUDA(cudaMemcpyAsync(f15 + j * V, e->staging, V * 8, cudaMemcpyDeviceToHost, e->stream));
             }
             E_CUDA(cudaStreamSynchronize(e->stream));
@@ -427,14 +515,16 @@ int lbman_ensemble_step(lbman_ensemble* e, int nsteps) {
     if (!e->uploaded) return efail(LBMAN_ERR_STATE, "step before initialisation");
     E_CUDA(cudaSetDevice(e->device));
     int done = 0;
-    // rho everywhere is refreshed by the final step of each call
-    if (!e->f_post && nsteps > 0) {
+    // rho everywhere is refreshed by the final step of each call; the first
+    // step after an upload or a change of organisation is not captured (its
+    // layout does not come back)
+    if (nsteps > 0 && (e->kernels == LBMAN_KERNELS_FUSED) != (e->fphase == F_POST)) {
         if (int st = ens_step_once(e, nsteps == 1)) return st;
         ++done;
     }
     constexpr int kGraphSteps = 20;  // even, so a replay keeps the buffer parity
     while (nsteps - done > kGraphSteps) {
-        if (!e->graph || e->graph_par != e->par) {
+        if (!e->graph || e->graph_par != e->par || e->graph_fphase != e->fphase) {
             if (int st = ens_build_graph(e, kGraphSteps)) return st;
         }
         E_CUDA(cudaGraphLaunch(e->graph, e->stream));
@@ -461,7 +551,13 @@ int lbman_ensemble_set_shape(lbman_ensemble* e, int kernels, int tile_x, int til
         return efail(LBMAN_ERR_ARG, "kernels must be SPLIT or FUSED");
     if (e->ops().qforce_smem(QTile{tile_x, tile_y, 1}) == 0)
         return efail(LBMAN_ERR_ARG, "tile is not compiled for this precision");
-    if (e->f_post && kernels != e->kernels) {
+    if (!e->small) kernels = LBMAN_KERNELS_FUSED;
+    const int before = e->kernels;
+    e->kernels = kernels;
+    const int have = ensure_buffers(e);
+    e->kernels = before;
+    if (have != LBMAN_OK) return have;
+    if (e->stepped && kernels != e->kernels) {
         // the split organisation keeps u in u[0]; the fused one ping-pongs
         const int p = e->par;
         for (auto& B : e->host) {
@@ -495,21 +591,24 @@ int lbman_ensemble_autotune(lbman_ensemble* e, int steps_per_trial, lbman_shape*
     if (!e->uploaded) return efail(LBMAN_ERR_STATE, "autotune needs an initialised ensemble");
     E_CUDA(cudaSetDevice(e->device));
     // Snapshot every box so the trials leave no trace.
+    constexpr int kFields = 7;
     std::vector<void*> snap;
     auto bytes_of = [&](const EnsBox& B, int k) -> size_t {
         const int64_t V = B.P.V;
-        const size_t s[8] = {5 * V * e->rbytes, 5 * V * e->rbytes, 3 * V * e->rbytes, 3 * V * e->rbytes,
-                             15 * V * e->sbytes, 15 * V * e->sbytes, V * e->rbytes, 3 * V * e->rbytes};
+        const size_t s[kFields] = {5 * V * e->rbytes,  5 * V * e->rbytes, 3 * V * e->rbytes, 3 * V * e->rbytes,
+                                   15 * V * e->sbytes, V * e->rbytes,     3 * V * e->rbytes};
         return s[k];
     };
+    const int fcur0 = e->fcur, fphase0 = e->fphase;
     auto ptr_of = [&](EnsBox& B, int k) -> void* {
-        void* p[8] = {B.q[0], B.q[1], B.u[0], B.u[1], B.f[0], B.f[1], B.rho, B.F};
+        void* p[kFields] = {B.q[0], B.q[1], B.u[0], B.u[1], B.f[fcur0], B.rho, B.F};
         return p[k];
     };
     for (auto& B : e->host)
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < kFields; ++k) {
             void* p = nullptr;
             if (cudaMalloc(&p, bytes_of(B, k)) != cudaSuccess) {
+                cudaGetLastError();
                 for (void* q : snap) cudaFree(q);
                 return efail(LBMAN_ERR_NOMEM, "autotune snapshot allocation failed");
             }
@@ -517,47 +616,57 @@ int lbman_ensemble_autotune(lbman_ensemble* e, int steps_per_trial, lbman_shape*
             E_CUDA(cudaMemcpyAsync(p, ptr_of(B, k), bytes_of(B, k), cudaMemcpyDeviceToDevice, e->stream));
         }
     const int par0 = e->par, kern0 = e->kernels, tx0 = e->tcx, ty0 = e->tcy, zc0 = e->zc_target;
-    const bool fpost0 = e->f_post;
+    const bool stepped0 = e->stepped;
     const int64_t steps0 = e->steps;
     cudaEvent_t a = nullptr, b = nullptr;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     lbman_shape win{kern0, tx0, ty0, zc0, 0, 1e30};
     int count = 0, status = LBMAN_OK;
-    for (int k : {LBMAN_KERNELS_SPLIT, LBMAN_KERNELS_FUSED}) {
-        for (const auto& t : kTileList) {
-            if (e->ops().qforce_smem(QTile{t[0], t[1], 1}) == 0) continue;
-            for (int zc : {0, 16, 48}) {
-                if ((status = lbman_ensemble_set_shape(e, k, t[0], t[1], zc)) != LBMAN_OK) break;
-                if ((status = ens_step_once(e, false)) != LBMAN_OK) break;
-                cudaEventRecord(a, e->stream);
-                for (int n = 0; n < steps_per_trial && status == LBMAN_OK; ++n) status = ens_step_once(e, false);
-                cudaEventRecord(b, e->stream);
-                if (status != LBMAN_OK || cudaEventSynchronize(b) != cudaSuccess) {
-                    if (status == LBMAN_OK) status = efail(LBMAN_ERR_CUDA, "autotune trial failed");
-                    break;
-                }
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, a, b);
-                ++count;
-                if (ms / steps_per_trial < win.ms_per_step) win = {k, t[0], t[1], zc, 0, ms / steps_per_trial};
-            }
-            if (status != LBMAN_OK) break;
+    // the split organisation has no shape; fused tiles x z chunks, where the
+    // second population buffers fit
+    std::vector<lbman_shape> trials;
+    if (e->small) trials.push_back({LBMAN_KERNELS_SPLIT, tx0, ty0, zc0, 0, 0.0, 0});
+    for (const auto& t : kTileList) {
+        if (e->ops().qforce_smem(QTile{t[0], t[1], 1}) == 0) continue;
+        for (int zc : {0, 16, 48}) trials.push_back({LBMAN_KERNELS_FUSED, t[0], t[1], zc, 0, 0.0, 0});
+    }
+    for (const lbman_shape& t : trials) {
+        status = lbman_ensemble_set_shape(e, t.kernels, t.tile_x, t.tile_y, t.zchunk);
+        if (status == LBMAN_ERR_NOMEM && e->small) {
+            status = LBMAN_OK;
+            break;
         }
-        if (status != LBMAN_OK) break;
+        if (status != LBMAN_OK || (status = ens_step_once(e, false)) != LBMAN_OK) break;
+        cudaEventRecord(a, e->stream);
+        for (int n = 0; n < steps_per_trial && status == LBMAN_OK; ++n) status = ens_step_once(e, false);
+        cudaEventRecord(b, e->stream);
+        if (status != LBMAN_OK || cudaEventSynchronize(b) != cudaSuccess) {
+            if (status == LBMAN_OK) status = efail(LBMAN_ERR_CUDA, "autotune trial failed");
+            break;
+        }
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, a, b);
+        ++count;
+        if (ms / steps_per_trial < win.ms_per_step) {
+            win = t;
+            win.ms_per_step = ms / steps_per_trial;
+        }
     }
     // restore: fields, parity and the velocity organisation of the original shape
     e->kernels = kern0;
     int i = 0;
     for (auto& B : e->host)
-        for (int k = 0; k < 8; ++k, ++i)
+        for (int k = 0; k < kFields; ++k, ++i)
             cudaMemcpyAsync(ptr_of(B, k), snap[i], bytes_of(B, k), cudaMemcpyDeviceToDevice, e->stream);
     cudaStreamSynchronize(e->stream);
     for (void* p : snap) cudaFree(p);
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     e->par = par0;
-    e->f_post = fpost0;
+    e->fcur = fcur0;
+    e->fphase = fphase0;
+    e->stepped = stepped0;
     e->steps = steps0;
     if (status != LBMAN_OK) {
         lbman_ensemble_set_shape(e, kern0, tx0, ty0, zc0);

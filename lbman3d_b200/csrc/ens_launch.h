@@ -1,4 +1,5 @@
-// ens_launch.h -- host-side launchers of the ensemble kernels (kernels_ens.cu).
+// ens_launch.h -- host-side launchers of the ensemble kernels (kernels_ens*.cu:
+// the fused organisation; kernels_ens_point*.cu: the split one).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -7,23 +8,25 @@
 
 namespace lbman {
 
-// One Q+force (or fused) launch over every box of an ensemble.
-struct EnsQLaunch {
+// One fused launch over every box of an ensemble.
+struct EnsFusedLaunch {
     const EnsBox* boxes;
     const EnsQWork* work;
     int nwork;
     int tcx, tcy;
-    bool fused, upwind;
-    int par, first, write_rho_all;
+    bool upwind;
+    int par, fcur, first, write_rho_all;
     int grid;
 };
 
-#define LBMAN_ENS_DECLARE(SUF)                                                                           \
-    cudaError_t ens_qstep_##SUF(const EnsQLaunch& L, cudaStream_t st);                                   \
-    cudaError_t ens_lbm_##SUF(const EnsBox* b, const EnsLbmWork* w, int n, int par, int first, int wr, int grid, \
-                              cudaStream_t st);                                                          \
-    cudaError_t ens_prepare_##SUF(size_t max_smem);                                                      \
-    int ens_blocks_per_sm_##SUF(int tcx, int tcy, bool fused);
+#define LBMAN_ENS_DECLARE(SUF)                                                                                \
+    cudaError_t ens_fused_##SUF(const EnsFusedLaunch& L, cudaStream_t st);                                    \
+    cudaError_t ens_prepare_##SUF(size_t max_smem);                                                           \
+    int ens_blocks_per_sm_##SUF(int tcx, int tcy);                                                            \
+    cudaError_t ens_qpoint_##SUF(const EnsBox* boxes, const EnsPointWork* work, int nwork, bool upwind, int par, \
+                                 cudaStream_t st);                                                            \
+    cudaError_t ens_lbm_point_##SUF(const EnsBox* boxes, const EnsLbmWork* work, int nwork, int par, int fcur, \
+                                    bool odd, bool last, cudaStream_t st);
 
 LBMAN_ENS_DECLARE(f64)
 LBMAN_ENS_DECLARE(f32)
