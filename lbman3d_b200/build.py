@@ -40,6 +40,8 @@ UNITS = {
     "kernels_point.cu": [],
     "kernels_point_f16.cu": [],
     "kernels_point_f64.cu": ["--fmad=false"],
+    "kernels_diag.cu": [],
+    "kernels_diag_f64.cu": ["--fmad=false"],
     "kernels_ens.cu": [],
     "kernels_ens_f64.cu": ["--fmad=false"],
     "kernels_ens_point.cu": [],

@@ -62,9 +62,7 @@ struct Ops {
     decltype(&launch_real_out_f64) real_out;
     decltype(&launch_flow_reduce_f64) flow_reduce;
     decltype(&launch_energy_reduce_f64) energy_reduce;
-    decltype(&launch_director_f64) director;
-    decltype(&launch_defect_count_f64) defect_count;
-    decltype(&launch_defect_flags_f64) defect_flags;
+    decltype(&launch_defects_f64) defects;
     decltype(&launch_seeded_init_f64) seeded_init;
     decltype(&launch_qsetup_f64) qsetup;
     decltype(&launch_active_force_f64) active_force;
@@ -77,15 +75,16 @@ struct Ops {
     decltype(&prepare_f64) prepare;
 };
 
-// QSUF: the suffix of the Q stage's point kernels (FP16 storage computes in FP32)
+// QSUF: the suffix of the kernels that do not touch populations (FP16 storage
+// computes in FP32)
 #define LBMAN_OPS(SUF, QSUF)                                                                               \
     Ops {                                                                                              \
         launch_qforce_##SUF, launch_fused_##SUF, launch_lbm_##SUF, launch_stream_only_##SUF,           \
             launch_lbm_aa_##SUF, launch_aa_pop_out_##SUF, launch_swap_pairs_##SUF,                     \
             launch_halo_merge_##SUF,                                                                   \
             launch_feq_init_##SUF, launch_pop_in_##SUF, launch_pop_out_##SUF, launch_real_in_##SUF,    \
-            launch_real_out_##SUF, launch_flow_reduce_##SUF, launch_energy_reduce_##SUF,               \
-            launch_director_##SUF, launch_defect_count_##SUF, launch_defect_flags_##SUF,              \
+            launch_real_out_##SUF, launch_flow_reduce_##QSUF, launch_energy_reduce_##QSUF,             \
+            launch_defects_##QSUF,                                                                     \
             launch_seeded_init_##SUF, launch_qsetup_##SUF, launch_active_force_##SUF,                  \
             launch_qpoint_##QSUF, launch_point_force_##QSUF, launch_lbm_aa_point_##SUF,                \
             qforce_smem_##SUF, qforce_threads_##SUF, march_blocks_##SUF, prepare_##SUF                 \
@@ -176,7 +175,6 @@ struct lbman_solver {
     double* red_dev = nullptr;
     double* red_host = nullptr;
     void* upast = nullptr;
-    void* dirbuf = nullptr;
     int fcur = 0, qcur = 0, ucur = 0;
     // Layout of the populations in f[fcur]: F_PRE pre-collision (after an
     // upload or an odd in-place step), F_POST post-collision of the
@@ -504,7 +502,7 @@ int lbman_destroy(lbman_solver* s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     for (int b = 0; b < 2; ++b) { cudaFree(s->f[b]); cudaFree(s->q[b]); cudaFree(s->u[b]); }
     cudaFree(s->rho); cudaFree(s->F); cudaFree(s->staging); cudaFree(s->partials); cudaFree(s->red_dev);
-    cudaFree(s->upast); cudaFree(s->dirbuf); cudaFree(s->stress); cudaFree(s->pstress); cudaFree(s->fstage);
+    cudaFree(s->upast); cudaFree(s->stress); cudaFree(s->pstress); cudaFree(s->fstage);
     if (s->ev_ready) cudaEventDestroy(s->ev_ready);
     if (s->ev_done) cudaEventDestroy(s->ev_done);
     lbman::stats::destroy(s->stats);
@@ -871,10 +869,8 @@ int lbman_reduce(lbman_solver* s, int flags, lbman_diag* out) {
     // not counted
     const bool defects = (flags & LBMAN_DIAG_DEFECTS) && !s->slab && s->P.nx >= 2 && s->P.ny >= 2 && s->P.nz >= 2;
     if (defects) {
-        if (!s->dirbuf) LB_CUDA(cudaMalloc(&s->dirbuf, 3 * V * s->rbytes));
-        LB_TRY(check_launch(s, o.director(s->P, s->q[s->qcur], nullptr, s->dirbuf, G, s->stream), "director"));
-        LB_TRY(check_launch(s, o.defect_count(s->P, s->dirbuf, s->partials, G, s->stream), "defect_count"));
-        LB_TRY(check_launch(s, launch_fold(s->partials, G, 1, 0, s->red_dev + 9, s->stream), "fold"));
+        LB_TRY(check_launch(s, o.defects(s->P, s->q[s->qcur], nullptr, (unsigned long long*)(s->red_dev + 9), s->stream),
+                            "defects"));
     }
     LB_CUDA(cudaMemcpyAsync(s->red_host, s->red_dev, 10 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     LB_CUDA(cudaStreamSynchronize(s->stream));
@@ -885,7 +881,7 @@ int lbman_reduce(lbman_solver* s, int flags, lbman_diag* out) {
         out->nan_detected = std::isnan(r[0]) || std::isnan(r[1]) || std::isnan(r[2]) || std::isnan(r[3]);
     }
     if (flags & LBMAN_DIAG_ENERGY) out->free_energy = r[8];
-    if (defects) out->defect_faces = (int64_t)std::llround(r[9]);
+    if (defects) std::memcpy(&out->defect_faces, r + 9, sizeof(int64_t));  // an integer count
     if (out->nan_detected) return fail(LBMAN_ERR_DIVERGED, "NaN in the global mass or momentum");
     return LBMAN_OK;
 }
@@ -921,7 +917,7 @@ int lbman_velocity_spectrum(lbman_solver* s, int nbins, double* E, double* count
 int lbman_q_correlation(lbman_solver* s, int nbins, double* C, double* counts, double* xi) {
     if (!s || !C) return fail(LBMAN_ERR_ARG, "null argument");
     LB_TRY(stats_ready(s, nbins));
-    s->launches += 7;  // power x4, to-complex, shell binning, fold (plus cuFFT's own kernels)
+    s->launches += 6;  // power x4, shell binning, fold (plus cuFFT's own kernels)
     LB_TRY(stats_status(lbman::stats::q_correlation(s->stats, s->q[s->qcur], nbins, C, counts, s->stream),
                         "Q correlation"));
     if (xi) {
@@ -964,12 +960,11 @@ int lbman_defect_lines(lbman_solver* s, lbman_defects* info, double* points, int
     const int64_t V = s->P.V;
     const int64_t nf = (int64_t)nx * (ny - 1) * (nz - 1) + (int64_t)(nx - 1) * ny * (nz - 1) +
                        (int64_t)(nx - 1) * (ny - 1) * nz;
-    if (!s->dirbuf) LB_CUDA(cudaMalloc(&s->dirbuf, 3 * V * s->rbytes));
     uint8_t* dflags = nullptr;
     LB_CUDA(cudaMalloc(&dflags, (size_t)nf));
     std::vector<uint8_t> flags((size_t)nf);
-    int st = check_launch(s, s->ops().director(s->P, s->q[s->qcur], nullptr, s->dirbuf, s->red_G, s->stream), "director");
-    if (st == LBMAN_OK) st = check_launch(s, s->ops().defect_flags(s->P, s->dirbuf, dflags, s->red_G, s->stream), "defect_flags");
+    int st = check_launch(s, s->ops().defects(s->P, s->q[s->qcur], dflags, (unsigned long long*)(s->red_dev + 9), s->stream),
+                          "defects");
     if (st == LBMAN_OK && (cudaMemcpyAsync(flags.data(), dflags, (size_t)nf, cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
                            cudaStreamSynchronize(s->stream) != cudaSuccess))
         st = fail(LBMAN_ERR_CUDA, "defect flags copy failed");

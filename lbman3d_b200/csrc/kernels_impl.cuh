@@ -7,7 +7,6 @@
 #include "qsplit.cuh"
 #include "qpair.cuh"
 #include "launch.h"
-#include "reduce.cuh"
 #include "tiles.h"
 
 #include <algorithm>
@@ -393,34 +392,6 @@ cudaError_t real_out(const void* src, double* dst, int64_t n, cudaStream_t st) {
 }
 
 template <class R>
-cudaError_t flow_reduce(const SimParams& P, const void* rho, const void* u, void* upast, double* partials, int G,
-                        cudaStream_t st) {
-    flow_reduce_kernel<R><<<G, kRedThreads, 0, st>>>(P, (const R*)rho, (const R*)u, (R*)upast, partials);
-    return cudaGetLastError();
-}
-template <class R>
-cudaError_t energy_reduce(const SimParams& P, const void* q, double* partials, int G, cudaStream_t st) {
-    energy_reduce_kernel<R><<<G, kRedThreads, 0, st>>>(P, (const R*)q, partials);
-    return cudaGetLastError();
-}
-template <class R>
-cudaError_t director(const SimParams& P, const void* q, void* order, void* dir, int G, cudaStream_t st) {
-    director_kernel<R><<<G, kRedThreads, 0, st>>>(P, (const R*)q, (R*)order, (R*)dir);
-    return cudaGetLastError();
-}
-template <class R>
-cudaError_t defect_flags(const SimParams& P, const void* dir, uint8_t* flags, int G, cudaStream_t st) {
-    defect_flags_kernel<R><<<G, kRedThreads, 0, st>>>(P, (const R*)dir, flags);
-    return cudaGetLastError();
-}
-
-template <class R>
-cudaError_t defect_count(const SimParams& P, const void* dir, double* partials, int G, cudaStream_t st) {
-    defect_count_kernel<R><<<G, kRedThreads, 0, st>>>(P, (const R*)dir, partials);
-    return cudaGetLastError();
-}
-
-template <class R>
 cudaError_t seeded_init(const SimParams& P, uint64_t seed, double S0, double sigma, void* rho, void* u, void* q,
                         void* F, cudaStream_t st) {
     const uint64_t key = splitmix64(seed ^ 0x5851f42d4c957f2dULL);
@@ -537,26 +508,6 @@ cudaError_t prepare(size_t max_smem) {
     }                                                                                                   \
     cudaError_t launch_real_out_##SUF(const void* src, double* dst, int64_t n, cudaStream_t st) {      \
         return impl::real_out<R>(src, dst, n, st);                                                      \
-    }                                                                                                   \
-    cudaError_t launch_flow_reduce_##SUF(const SimParams& P, const void* rho, const void* u,           \
-                                         void* upast, double* partials, int G, cudaStream_t st) {      \
-        return impl::flow_reduce<R>(P, rho, u, upast, partials, G, st);                                 \
-    }                                                                                                   \
-    cudaError_t launch_energy_reduce_##SUF(const SimParams& P, const void* q, double* partials, int G,  \
-                                           cudaStream_t st) {                                          \
-        return impl::energy_reduce<R>(P, q, partials, G, st);                                           \
-    }                                                                                                   \
-    cudaError_t launch_director_##SUF(const SimParams& P, const void* q, void* order, void* dir, int G, \
-                                      cudaStream_t st) {                                               \
-        return impl::director<R>(P, q, order, dir, G, st);                                              \
-    }                                                                                                   \
-    cudaError_t launch_defect_flags_##SUF(const SimParams& P, const void* dir, uint8_t* flags, int G,  \
-                                          cudaStream_t st) {                                           \
-        return impl::defect_flags<R>(P, dir, flags, G, st);                                             \
-    }                                                                                                   \
-    cudaError_t launch_defect_count_##SUF(const SimParams& P, const void* dir, double* partials, int G, \
-                                          cudaStream_t st) {                                           \
-        return impl::defect_count<R>(P, dir, partials, G, st);                                          \
     }                                                                                                   \
     cudaError_t launch_seeded_init_##SUF(const SimParams& P, uint64_t seed, double S0, double sigma,    \
                                          void* rho, void* u, void* q, void* F, cudaStream_t st) {      \

@@ -49,12 +49,8 @@ struct LaunchShape {
                                          void* upast, double* partials, int G, cudaStream_t st);       \
     cudaError_t launch_energy_reduce_##SUF(const SimParams& P, const void* q, double* partials, int G,  \
                                            cudaStream_t st);                                           \
-    cudaError_t launch_director_##SUF(const SimParams& P, const void* q, void* order, void* dir, int G, \
-                                      cudaStream_t st);                                                \
-    cudaError_t launch_defect_flags_##SUF(const SimParams& P, const void* dir, uint8_t* flags, int G,  \
-                                          cudaStream_t st);                                            \
-    cudaError_t launch_defect_count_##SUF(const SimParams& P, const void* dir, double* partials, int G, \
-                                          cudaStream_t st);                                            \
+    cudaError_t launch_defects_##SUF(const SimParams& P, const void* q, uint8_t* flags,                 \
+                                     unsigned long long* count, cudaStream_t st);                      \
     cudaError_t launch_seeded_init_##SUF(const SimParams& P, uint64_t seed, double S0, double sigma,    \
                                          void* rho, void* u, void* q, void* F, cudaStream_t st);       \
     cudaError_t launch_qsetup_##SUF(const SimParams& P, const void* qin, const void* uin, void* qout,   \

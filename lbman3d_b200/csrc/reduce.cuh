@@ -50,6 +50,43 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NQ], double* part
     }
 }
 
+// Four consecutive values as one load / store (float: 16 bytes, double: 32).
+template <class R>
+struct Quad {
+    R v[4];
+};
+__device__ __forceinline__ Quad<float> ld4(const float* p) {
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    return {{a.x, a.y, a.z, a.w}};
+}
+__device__ __forceinline__ Quad<double> ld4(const double* p) {
+    const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+    return {{a.x, a.y, b.x, b.y}};
+}
+__device__ __forceinline__ void st4(float* p, const Quad<float>& q) {
+    *reinterpret_cast<float4*>(p) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]);
+}
+__device__ __forceinline__ void st4(double* p, const Quad<double>& q) {
+    *reinterpret_cast<double2*>(p) = make_double2(q.v[0], q.v[1]);
+    *reinterpret_cast<double2*>(p + 2) = make_double2(q.v[2], q.v[3]);
+}
+__device__ __forceinline__ bool quad_ok(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+__device__ __forceinline__ void flow_cell(double (&v)[kFlowQ], double r, double ux, double uy, double uz, double px,
+                                          double py, double pz) {
+    v[0] += r;
+    v[1] += r * ux;
+    v[2] += r * uy;
+    v[3] += r * uz;
+    const double u2 = ux * ux + uy * uy + uz * uz;
+    v[4] += 0.5 * r * u2;
+    v[5] += (ux - px) * (ux - px) + (uy - py) * (uy - py) + (uz - pz) * (uz - pz);
+    v[6] += u2;
+    v[7] = fmax(v[7], u2);
+}
+
+// Memory bound (10 words per cell): four cells per thread where every array
+// allows 16-byte accesses (256^3 FP32: 161 us one cell at a time).
 template <class R>
 __global__ void __launch_bounds__(kRedThreads) flow_reduce_kernel(SimParams P, const R* __restrict__ rho,
                                                                   const R* __restrict__ u,
@@ -57,160 +94,261 @@ __global__ void __launch_bounds__(kRedThreads) flow_reduce_kernel(SimParams P, c
                                                                   double* __restrict__ partials) {
     const int64_t V = P.V;
     double v[kFlowQ] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int64_t c = P.c0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < P.c1;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        const double r = (double)rho[c];
-        const double ux = (double)u[c], uy = (double)u[V + c], uz = (double)u[2 * V + c];
-        const double px = (double)upast[c], py = (double)upast[V + c], pz = (double)upast[2 * V + c];
-        v[0] += r;
-        v[1] += r * ux;
-        v[2] += r * uy;
-        v[3] += r * uz;
-        const double u2 = ux * ux + uy * uy + uz * uz;
-        v[4] += 0.5 * r * u2;
-        v[5] += (ux - px) * (ux - px) + (uy - py) * (uy - py) + (uz - pz) * (uz - pz);
-        v[6] += u2;
-        v[7] = fmax(v[7], u2);
-        upast[c] = u[c];
-        upast[V + c] = u[V + c];
-        upast[2 * V + c] = u[2 * V + c];
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    if (V % 4 == 0 && P.c0 % 4 == 0 && P.c1 % 4 == 0 && quad_ok(rho) && quad_ok(u) && quad_ok(upast)) {
+        for (int64_t c = P.c0 + 4 * t; c < P.c1; c += 4 * nt) {
+            const Quad<R> r = ld4(rho + c);
+            Quad<R> a[3], b[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                a[k] = ld4(u + k * V + c);
+                b[k] = ld4(upast + k * V + c);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                flow_cell(v, (double)r.v[i], (double)a[0].v[i], (double)a[1].v[i], (double)a[2].v[i], (double)b[0].v[i],
+                          (double)b[1].v[i], (double)b[2].v[i]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) st4(upast + k * V + c, a[k]);
+        }
+    } else {
+        for (int64_t c = P.c0 + t; c < P.c1; c += nt) {
+            const R ux = u[c], uy = u[V + c], uz = u[2 * V + c];
+            flow_cell(v, (double)rho[c], (double)ux, (double)uy, (double)uz, (double)upast[c], (double)upast[V + c],
+                      (double)upast[2 * V + c]);
+            upast[c] = ux;
+            upast[V + c] = uy;
+            upast[2 * V + c] = uz;
+        }
     }
     block_reduce_store<kFlowQ, 1>(v, partials);
 }
 
-// NematicFreeEnergyDensity with the QXoff-clamped 7-point Laplacian.
+// Tiles of the z-marching diagnostics: one thread per (x, y) column of a tile,
+// kDiagZ planes per work item.
+constexpr int kDiagZ = 32;
+
+// Index of the neighbour a + s under the QXoff clamp / wrap of one axis.
+__device__ __forceinline__ int qx_off(int a, int n, int per_lo, int per_hi) {
+    if (a < 0) return per_lo ? a + n : 0;
+    if (a >= n) return per_hi ? a - n : n - 1;
+    return a;
+}
+
+// NematicFreeEnergyDensity with the QXoff-clamped 7-point Laplacian, in FP64.
+// FP32 fields: a value is converted once -- each thread converts its own
+// column, keeps three planes of it in registers and shares the current plane
+// through shared memory -- because the conversions, at a quarter of the FP64
+// rate or less, were what bounded the one-thread-per-cell form (35 per cell;
+// 256^3: 331 us).
+constexpr int kEnX = 32, kEnY = 8;
+static_assert(kEnX * kEnY == kRedThreads, "one thread per column of a tile");
 template <class R>
-__global__ void __launch_bounds__(kRedThreads) energy_reduce_kernel(SimParams P, const R* __restrict__ q,
+__global__ void __launch_bounds__(kRedThreads) energy_reduce_kernel(const __grid_constant__ SimParams P,
+                                                                    const R* __restrict__ q,
                                                                     double* __restrict__ partials) {
+    constexpr int SX = kEnX + 2, SY = kEnY + 2;
+    __shared__ double sh[5][SY][SX];
     const int64_t V = P.V;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     double v[1] = {0.0};
-    for (int64_t c = P.c0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < P.c1;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        const int z = (int)(c / P.nxy);
-        const int rr = (int)(c - (int64_t)z * P.nxy);
-        const int y = rr / nx, x = rr - y * nx;
-        auto off = [&](int a, int s, int n, int lo, int hi) {
-            const int t = a + s;
-            if (t < 0) return P.qper[lo] ? t + n : 0;
-            if (t >= n) return P.qper[hi] ? t - n : n - 1;
-            return t;
-        };
-        const int xm = off(x, -1, nx, 0, 1), xp = off(x, 1, nx, 0, 1);
-        const int ym = off(y, -1, ny, 2, 3), yp = off(y, 1, ny, 2, 3);
-        const int zm = off(z, -1, nz, 4, 5), zp = off(z, 1, nz, 4, 5);
-        double Q[5], l[5];
+    const int gx = (nx + kEnX - 1) / kEnX, gy = (ny + kEnY - 1) / kEnY, gz = (P.zhi - P.zlo + kDiagZ - 1) / kDiagZ;
+    const int lx = threadIdx.x % kEnX, ly = threadIdx.x / kEnX;
+    // this thread's halo point of a plane (threads 0 .. 2 (kEnX + kEnY) - 1)
+    const int h = threadIdx.x;
+    const bool halo = h < 2 * (kEnX + kEnY);
+    const int hx = h < 2 * kEnX ? h % kEnX + 1 : (h - 2 * kEnX < kEnY ? 0 : SX - 1);
+    const int hy = h < 2 * kEnX ? (h < kEnX ? 0 : SY - 1) : (h - 2 * kEnX) % kEnY + 1;
+    for (int item = blockIdx.x; item < gx * gy * gz; item += gridDim.x) {
+        const int x0 = item % gx * kEnX, y0 = item / gx % gy * kEnY, z0 = P.zlo + item / (gx * gy) * kDiagZ;
+        const int z1 = min(z0 + kDiagZ, P.zhi);
+        const int x = x0 + lx, y = y0 + ly;
+        const bool live = x < nx && y < ny;
+        const int64_t col = (int64_t)min(y, ny - 1) * nx + min(x, nx - 1);
+        const int64_t hcol = (int64_t)qx_off(min(y0 + hy - 1, ny), ny, P.qper[2], P.qper[3]) * nx +
+                             qx_off(min(x0 + hx - 1, nx), nx, P.qper[0], P.qper[1]);
+        double qm[5], qc[5], qp[5];
+        const int64_t zm0 = (int64_t)qx_off(z0 - 1, nz, P.qper[4], P.qper[5]) * P.nxy;
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            const R* a = q + k * V;
-            auto at = [&](int xx, int yy, int zz) { return (double)a[(int64_t)zz * P.nxy + (int64_t)yy * nx + xx]; };
-            Q[k] = (double)a[c];
-            l[k] = at(xp, y, z) + at(xm, y, z) + at(x, yp, z) + at(x, ym, z) + at(x, y, zp) + at(x, y, zm) -
-                   6.0 * Q[k];
+            qm[k] = (double)q[k * V + zm0 + col];
+            qc[k] = (double)q[k * V + (int64_t)z0 * P.nxy + col];
         }
-        const double Qxx = Q[0], Qxy = Q[1], Qxz = Q[2], Qyy = Q[3], Qyz = Q[4];
-        const double half = (Qxx * Qxx + Qxx * Qyy + Qyy * Qyy + Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
-        const double TrQ2 = 2.0 * half;
-        const double k13 = 1.0 / 3.0;
-        const double Q2_xx = Qxx * Qxx + Qxy * Qxy + Qxz * Qxz - k13 * TrQ2;
-        const double Q2_xy = Qxx * Qxy + Qxy * Qyy + Qxz * Qyz;
-        const double Q2_xz = Qxy * Qyz - Qxz * Qyy;
-        const double Q2_yy = Qxy * Qxy + Qyy * Qyy + Qyz * Qyz - k13 * TrQ2;
-        const double Q2_yz = Qxy * Qxz - Qyz * Qxx;
-        const double TrQ3 = 2.0 * Qxx * Q2_xx + 2.0 * Qyy * Q2_yy + Qxx * Q2_yy + Qyy * Q2_xx +
-                            2.0 * (Qxy * Q2_xy + Qxz * Q2_xz + Qyz * Q2_yz);
-        const double QlQ = 2.0 * Qxx * l[0] + 2.0 * Qyy * l[3] + Qxx * l[3] + Qyy * l[0] +
-                           2.0 * (Qxy * l[1] + Qxz * l[2] + Qyz * l[4]);
-        v[0] += 0.5 * P.A * TrQ2 + (P.B / 3.0) * TrQ3 + 0.25 * P.C * TrQ2 * TrQ2 - 0.5 * P.L * QlQ;
+        for (int z = z0; z < z1; ++z) {
+            const int64_t zp = (int64_t)qx_off(z + 1, nz, P.qper[4], P.qper[5]) * P.nxy;
+            __syncthreads();  // the previous plane has been read
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                qp[k] = (double)q[k * V + zp + col];
+                sh[k][ly + 1][lx + 1] = qc[k];
+                if (halo) sh[k][hy][hx] = (double)q[k * V + (int64_t)z * P.nxy + hcol];
+            }
+            __syncthreads();
+            if (live) {
+                // the neighbour beyond a partial tile's last cell comes from
+                // global memory (its shared slot holds a column outside the box)
+                double l[5];
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    const R* a = q + k * V + (int64_t)z * P.nxy;
+                    const double xp = (x == nx - 1 && lx != kEnX - 1)
+                                          ? (double)a[(int64_t)y * nx + qx_off(nx, nx, P.qper[0], P.qper[1])]
+                                          : sh[k][ly + 1][lx + 2];
+                    const double yp = (y == ny - 1 && ly != kEnY - 1)
+                                          ? (double)a[(int64_t)qx_off(ny, ny, P.qper[2], P.qper[3]) * nx + x]
+                                          : sh[k][ly + 2][lx + 1];
+                    l[k] = xp + sh[k][ly + 1][lx] + yp + sh[k][ly][lx + 1] + qp[k] + qm[k] - 6.0 * qc[k];
+                }
+                const double Qxx = qc[0], Qxy = qc[1], Qxz = qc[2], Qyy = qc[3], Qyz = qc[4];
+                const double half = (Qxx * Qxx + Qxx * Qyy + Qyy * Qyy + Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
+                const double TrQ2 = 2.0 * half;
+                const double k13 = 1.0 / 3.0;
+                const double Q2_xx = Qxx * Qxx + Qxy * Qxy + Qxz * Qxz - k13 * TrQ2;
+                const double Q2_xy = Qxx * Qxy + Qxy * Qyy + Qxz * Qyz;
+                const double Q2_xz = Qxy * Qyz - Qxz * Qyy;
+                const double Q2_yy = Qxy * Qxy + Qyy * Qyy + Qyz * Qyz - k13 * TrQ2;
+                const double Q2_yz = Qxy * Qxz - Qyz * Qxx;
+                const double TrQ3 = 2.0 * Qxx * Q2_xx + 2.0 * Qyy * Q2_yy + Qxx * Q2_yy + Qyy * Q2_xx +
+                                    2.0 * (Qxy * Q2_xy + Qxz * Q2_xz + Qyz * Q2_yz);
+                const double QlQ = 2.0 * Qxx * l[0] + 2.0 * Qyy * l[3] + Qxx * l[3] + Qyy * l[0] +
+                                   2.0 * (Qxy * l[1] + Qxz * l[2] + Qyz * l[4]);
+                v[0] += 0.5 * P.A * TrQ2 + (P.B / 3.0) * TrQ3 + 0.25 * P.C * TrQ2 * TrQ2 - 0.5 * P.L * QlQ;
+            }
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                qm[k] = qc[k];
+                qc[k] = qp[k];
+            }
+        }
     }
     block_reduce_store<1, 0>(v, partials);
 }
 
-// Scalar order S and director n per cell (closed form, no diagonalisation).
+// Director n of a cell (closed form, no diagonalisation), in FP64, rounded to
+// the field's precision.
 template <class R>
-__global__ void __launch_bounds__(kRedThreads) director_kernel(SimParams P, const R* __restrict__ q,
-                                                               R* __restrict__ order,
-                                                               R* __restrict__ director) {
-    const int64_t V = P.V;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < V; c += (int64_t)gridDim.x * blockDim.x) {
-        const double Qxx = q[c], Qxy = q[V + c], Qxz = q[2 * V + c], Qyy = q[3 * V + c], Qyz = q[4 * V + c];
-        const double pp = (Qxx * Qxx + Qxx * Qyy + Qyy * Qyy + Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
-        const double qq = (-(Qxx + Qyy) * (Qxx * Qyy - Qxy * Qxy) - Qyy * Qxz * Qxz - Qxx * Qyz * Qyz +
-                           2 * Qxy * Qxz * Qyz);
-        const double r = 2.0 * sqrt(pp / 3.0);
-        double arg = 4 * qq / (r * r * r);
-        arg = arg < -1.0 ? -1.0 : (1.0 < arg ? 1.0 : arg);
-        const double S = r * cos(1.0 / 3.0 * acos(arg));
-        double nx_ = Qxz * (Qyy - S) - Qxy * Qyz;
-        double ny_ = Qyz * (Qxx - S) - Qxy * Qxz;
-        double nz_ = Qxy * Qxy - (Qxx - S) * (Qyy - S);
-        const double ninv = 1.0 / sqrt(nx_ * nx_ + ny_ * ny_ + nz_ * nz_);
-        if (order) order[c] = (R)S;
-        director[3 * c + 0] = (R)(nx_ * ninv);
-        director[3 * c + 1] = (R)(ny_ * ninv);
-        director[3 * c + 2] = (R)(nz_ * ninv);
-    }
+__device__ __forceinline__ void director(double Qxx, double Qxy, double Qxz, double Qyy, double Qyz, R n[3]) {
+    const double pp = (Qxx * Qxx + Qxx * Qyy + Qyy * Qyy + Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
+    const double qq = (-(Qxx + Qyy) * (Qxx * Qyy - Qxy * Qxy) - Qyy * Qxz * Qxz - Qxx * Qyz * Qyz +
+                       2 * Qxy * Qxz * Qyz);
+    const double r = 2.0 * sqrt(pp / 3.0);
+    double arg = 4 * qq / (r * r * r);
+    arg = arg < -1.0 ? -1.0 : (1.0 < arg ? 1.0 : arg);
+    const double S = r * cos(1.0 / 3.0 * acos(arg));
+    double nx_ = Qxz * (Qyy - S) - Qxy * Qyz;
+    double ny_ = Qyz * (Qxx - S) - Qxy * Qxz;
+    double nz_ = Qxy * Qxy - (Qxx - S) * (Qyy - S);
+    const double ninv = 1.0 / sqrt(nx_ * nx_ + ny_ * ny_ + nz_ * nz_);
+    n[0] = (R)(nx_ * ninv);
+    n[1] = (R)(ny_ * ninv);
+    n[2] = (R)(nz_ * ninv);
 }
 
+// Is a.b <= 0, with b negated if flip: decided in FP64.  For FP32 directors an
+// FP32 evaluation decides first: three products of components of at most 1 in
+// magnitude sum with an error below 3e-7, so beyond 1e-6 its sign is the FP64
+// one (NaN takes the FP64 branch).
+__device__ __forceinline__ bool dot_nonpositive(const double a[3], const double b[3], bool flip) {
+    const double d = a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+    return (flip ? -d : d) <= 0.0;
+}
+__device__ __forceinline__ bool dot_nonpositive(const float a[3], const float b[3], bool flip) {
+    const float d = fmaf(a[2], b[2], fmaf(a[1], b[1], a[0] * b[0]));
+    if (fabsf(d) > 1e-6f) return flip ? d > 0.0f : d < 0.0f;
+    const double e = (double)a[0] * b[0] + (double)a[1] * b[1] + (double)a[2] * b[2];
+    return (flip ? -e : e) <= 0.0;
+}
+// Do the directors of a plaquette, each made to point along the one before,
+// end up against the first (src/analysis/defect_finder.tpp)?  The signs of the
+// second to fourth are kept as flips.
 template <class R>
-__device__ __forceinline__ int plaquette_flip(const R* d1, const R* d2, const R* d3, const R* d4) {
-    auto dot = [](const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; };
-    const double n1[3] = {(double)d1[0], (double)d1[1], (double)d1[2]};
-    double n2[3] = {(double)d2[0], (double)d2[1], (double)d2[2]};
-    double n3[3] = {(double)d3[0], (double)d3[1], (double)d3[2]};
-    double n4[3] = {(double)d4[0], (double)d4[1], (double)d4[2]};
-    if (dot(n1, n2) <= 0.0) { n2[0] = -n2[0]; n2[1] = -n2[1]; n2[2] = -n2[2]; }
-    if (dot(n2, n3) <= 0.0) { n3[0] = -n3[0]; n3[1] = -n3[1]; n3[2] = -n3[2]; }
-    if (dot(n3, n4) <= 0.0) { n4[0] = -n4[0]; n4[1] = -n4[1]; n4[2] = -n4[2]; }
-    return dot(n4, n1) <= 0.0;
+__device__ __forceinline__ bool plaquette_flip(const R d1[3], const R d2[3], const R d3[3], const R d4[3]) {
+    const bool f2 = dot_nonpositive(d1, d2, false);
+    const bool f3 = dot_nonpositive(d2, d3, f2);
+    const bool f4 = dot_nonpositive(d3, d4, f3);
+    return dot_nonpositive(d4, d1, f4);
 }
 
-// Count of flagged plaquettes over the three face families (the periodic
-// seam faces are not visited, as in the reference).
+// Plaquette sign-flip flags of the three face families in one z march: a
+// thread evaluates the director of one column, planes z and z - 1 meet in shared
+// memory, and the threads of the tile's first kDefX x kDefY columns test the
+// three plaquettes of their cell.  Bound by the director's FP64 arithmetic
+// (each is formed 1.1 times), where a director pass and a pass over its 24-byte
+// records took 567 us for 256^3 FP32.  The periodic seam faces are not visited,
+// as in the reference.
+//   count: receives the number of flagged plaquettes (added atomically);
+//   flags: if not null, the flags in the reference's DefectFields layout
+//   (src/analysis/defect_fields.h:16-29): def_x nx*(ny-1)*(nz-1), then def_y
+//   (nx-1)*ny*(nz-1), then def_z (nx-1)*(ny-1)*nz, each x fastest.
+constexpr int kDefTX = 32, kDefTY = 16, kDefX = kDefTX - 1, kDefY = kDefTY - 1, kDefThreads = kDefTX * kDefTY;
 template <class R>
-__global__ void __launch_bounds__(kRedThreads) defect_count_kernel(SimParams P, const R* __restrict__ dir,
-                                                                   double* __restrict__ partials) {
-    const int64_t V = P.V;
-    const int nx = P.nx, ny = P.ny, nz = P.nz;
-    double v[1] = {0.0};
-    auto D = [&](int x, int y, int z) { return dir + 3 * ((int64_t)z * P.nxy + (int64_t)y * nx + x); };
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < V; c += (int64_t)gridDim.x * blockDim.x) {
-        const int z = (int)(c / P.nxy);
-        const int rr = (int)(c - (int64_t)z * P.nxy);
-        const int y = rr / nx, x = rr - y * nx;
-        int n = 0;
-        if (y < ny - 1 && z < nz - 1) n += plaquette_flip<R>(D(x, y, z), D(x, y + 1, z), D(x, y + 1, z + 1), D(x, y, z + 1));
-        if (x < nx - 1 && z < nz - 1) n += plaquette_flip<R>(D(x, y, z), D(x + 1, y, z), D(x + 1, y, z + 1), D(x, y, z + 1));
-        if (x < nx - 1 && y < ny - 1) n += plaquette_flip<R>(D(x, y, z), D(x + 1, y, z), D(x + 1, y + 1, z), D(x, y + 1, z));
-        v[0] += n;
-    }
-    block_reduce_store<1, 0>(v, partials);
-}
-
-// Plaquette flags of the three face families in the reference's DefectFields
-// layout (src/analysis/defect_fields.h:16-29): def_x nx*(ny-1)*(nz-1), then
-// def_y (nx-1)*ny*(nz-1), then def_z (nx-1)*(ny-1)*nz, each x fastest.
-template <class R>
-__global__ void __launch_bounds__(kRedThreads) defect_flags_kernel(SimParams P, const R* __restrict__ dir,
-                                                                   uint8_t* __restrict__ flags) {
+__global__ void __launch_bounds__(kDefThreads) defect_kernel(const __grid_constant__ SimParams P,
+                                                             const R* __restrict__ q, uint8_t* __restrict__ flags,
+                                                             unsigned long long* __restrict__ count) {
+    __shared__ R sh[2][3][kDefTY][kDefTX];
+    __shared__ int total;
     const int64_t V = P.V;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const int64_t nfx = (int64_t)nx * (ny - 1) * (nz - 1), nfy = (int64_t)(nx - 1) * ny * (nz - 1);
-    auto D = [&](int x, int y, int z) { return dir + 3 * ((int64_t)z * P.nxy + (int64_t)y * nx + x); };
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < V; c += (int64_t)gridDim.x * blockDim.x) {
-        const int z = (int)(c / P.nxy);
-        const int rr = (int)(c - (int64_t)z * P.nxy);
-        const int y = rr / nx, x = rr - y * nx;
-        if (y < ny - 1 && z < nz - 1)
-            flags[((int64_t)z * (ny - 1) + y) * nx + x] =
-                (uint8_t)plaquette_flip<R>(D(x, y, z), D(x, y + 1, z), D(x, y + 1, z + 1), D(x, y, z + 1));
-        if (x < nx - 1 && z < nz - 1)
-            flags[nfx + ((int64_t)z * ny + y) * (nx - 1) + x] =
-                (uint8_t)plaquette_flip<R>(D(x, y, z), D(x + 1, y, z), D(x + 1, y, z + 1), D(x, y, z + 1));
-        if (x < nx - 1 && y < ny - 1)
-            flags[nfx + nfy + ((int64_t)z * (ny - 1) + y) * (nx - 1) + x] =
-                (uint8_t)plaquette_flip<R>(D(x, y, z), D(x + 1, y, z), D(x + 1, y + 1, z), D(x, y + 1, z));
+    const int lx = threadIdx.x % kDefTX, ly = threadIdx.x / kDefTX;
+    const int x = blockIdx.x * kDefX + lx, y = blockIdx.y * kDefY + ly;
+    const int z0 = blockIdx.z * kDiagZ, z1 = min(z0 + kDiagZ, nz);  // def_z planes of this block
+    const bool in = x < nx && y < ny;
+    const bool own = in && lx < kDefX && ly < kDefY;
+    const int64_t col = (int64_t)y * nx + x;
+    if (threadIdx.x == 0) total = 0;
+    auto at = [&](int b, int dx, int dy, R d[3]) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) d[k] = sh[b][k][ly + dy][lx + dx];
+    };
+    int n = 0;
+    for (int z = z0; z <= min(z1, nz - 1); ++z) {
+        const int b = z & 1;
+        if (in) {
+            const R* a = q + (int64_t)z * P.nxy + col;
+            R d[3];
+            director<R>((double)a[0], (double)a[V], (double)a[2 * V], (double)a[3 * V], (double)a[4 * V], d);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) sh[b][k][ly][lx] = d[k];
+        }
+        __syncthreads();
+        if (own) {
+            R d00[3], d10[3], d01[3];
+            at(b, 0, 0, d00);
+            if (x < nx - 1) at(b, 1, 0, d10);
+            if (y < ny - 1) at(b, 0, 1, d01);
+            if (z < z1 && x < nx - 1 && y < ny - 1) {  // def_z of plane z
+                R d11[3];
+                at(b, 1, 1, d11);
+                const bool f = plaquette_flip<R>(d00, d10, d11, d01);
+                n += f;
+                if (flags) flags[nfx + nfy + ((int64_t)z * (ny - 1) + y) * (nx - 1) + x] = f;
+            }
+            if (z > z0) {  // def_x, def_y between the planes z - 1 and z
+                R p00[3];
+                at(b ^ 1, 0, 0, p00);
+                if (y < ny - 1) {
+                    R p01[3];
+                    at(b ^ 1, 0, 1, p01);
+                    const bool f = plaquette_flip<R>(p00, p01, d01, d00);
+                    n += f;
+                    if (flags) flags[((int64_t)(z - 1) * (ny - 1) + y) * nx + x] = f;
+                }
+                if (x < nx - 1) {
+                    R p10[3];
+                    at(b ^ 1, 1, 0, p10);
+                    const bool f = plaquette_flip<R>(p00, p10, d10, d00);
+                    n += f;
+                    if (flags) flags[nfx + ((int64_t)(z - 1) * ny + y) * (nx - 1) + x] = f;
+                }
+            }
+        }
+        __syncthreads();  // plane z - 1's slot takes plane z + 1
     }
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_down_sync(0xffffffffu, n, o);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&total, n);
+    __syncthreads();
+    if (threadIdx.x == 0 && total) atomicAdd(count, (unsigned long long)total);
 }
 
 // Pass 2: fold G partials of NQ quantities (the last nmax by max) in order.
