@@ -29,6 +29,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "pdl.cuh"
 #include "tc.cuh"
 
 namespace lbman {
@@ -369,13 +370,10 @@ __global__ void __launch_bounds__(conv_threads(COUT)) conv_dhalo_kernel(Grid3 g,
     const int za = (int)(blockIdx.x / (unsigned)cols) * zc, len = min(zc, g.nz - za);
     const int last = len + 1;  // steps 0 .. last: input planes za - 1 .. za + len
     const bool worker = t < WORKERS;
-    if (worker) {
-        dhalo_load_plane<CIN, WORKERS>(g, in, x0, y0, za - 1, Hs);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        dhalo_load_plane<CIN, WORKERS>(g, in, x0, y0, za, Hs + SLOT);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    for (int i = t; i < BBYTES / 16; i += THREADS) reinterpret_cast<uint4*>(Bs)[i] = bimg[i];
+    // What no kernel still running writes (weights, biases) comes before
+    // pdl_begin(), the input planes after it.
+    for (int i = t; i < BBYTES / 16; i += THREADS)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(tc::smem_addr(Bs + i * 16)), "l"(bimg + i));
     if (t == 0) {
         tc::mbar_init(&bar[0], 1);
         tc::mbar_init(&bar[1], 1);
@@ -386,7 +384,16 @@ __global__ void __launch_bounds__(conv_threads(COUT)) conv_dhalo_kernel(Grid3 g,
 #pragma unroll
     for (int j = 0; j < kEpiCols; ++j)
         bias_h[j] = (MODE != kBwdData && worker) ? bias[(t >> 7) * kEpiCols + j] : 0.0f;
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // plane za - 1 in; za may be in flight
+    pdl_begin();
+    if (worker) {
+        dhalo_load_plane<CIN, WORKERS>(g, in, x0, y0, za - 1, Hs);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        dhalo_load_plane<CIN, WORKERS>(g, in, x0, y0, za, Hs + SLOT);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // weights and plane za - 1 in; za may be in flight
+    } else {
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+    }
     tc::fence_smem_async();
     tc::fence_before_sync();
     __syncthreads();
@@ -682,6 +689,7 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    pdl_begin();
     const uint32_t tmem = tslot;
     const uint32_t idesc = tc::idesc_bf16(kTileM, COUT, 1, 1);
     const uint32_t s0 = tc::smem_addr(sm), g0 = tc::smem_addr(Gs);
@@ -834,6 +842,7 @@ __global__ void __launch_bounds__(kFoldThreads) sum_partials_kernel(const float*
     __shared__ float slice[kFoldThreads / 32][32];
     const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
     const int j = blockIdx.x * 32 + lane;
+    pdl_begin();
     float acc = 0.0f;
     if (j < n)
         for (int p = s; p < P; p += kFoldThreads / 32) acc += partials[(int64_t)p * n + j];
@@ -927,6 +936,7 @@ __global__ void features_kernel(const float* __restrict__ rho, const float* __re
                                 const float* __restrict__ q5, int64_t V, const float* __restrict__ shift,
                                 const float* __restrict__ inv_scale, __nv_bfloat16* __restrict__ act0,
                                 float noise_std, uint64_t noise_key) {
+    pdl_begin();
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < V; c += (int64_t)gridDim.x * blockDim.x) {
         __align__(16) __nv_bfloat16 v[16];
         float x[9];
@@ -959,6 +969,7 @@ __global__ void __launch_bounds__(kThreads) loss_kernel(const float* __restrict_
     __shared__ double sh[kThreads / 32];
     double acc = 0.0;
     const float gscale = 2.0f / (8.0f * (float)V);
+    pdl_begin();
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < V; c += (int64_t)gridDim.x * blockDim.x) {
         __align__(16) __nv_bfloat16 gv[16];
 #pragma unroll
@@ -988,6 +999,7 @@ __global__ void __launch_bounds__(kThreads) loss_kernel(const float* __restrict_
 // (k < 5), u_d += gain out[5+d][c] s_{5+d}.
 __global__ void apply_kernel(const float* __restrict__ out, const float* __restrict__ out_scale, int64_t V,
                              float gain, float* __restrict__ u3, float* __restrict__ q5) {
+    pdl_begin();
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < V; c += (int64_t)gridDim.x * blockDim.x) {
 #pragma unroll
         for (int k = 0; k < 5; ++k) q5[k * V + c] += gain * out[k * V + c] * out_scale[k];

@@ -21,6 +21,7 @@
 #include "../../include/lbman3d.h"
 #include "closure.cuh"
 #include "closure_selftest.cuh"
+#include "pdl.cuh"
 #include "solver_view.h"
 
 using namespace lbman;
@@ -160,9 +161,9 @@ int run_conv(lbman_closure* c, cudaStream_t st, const __nv_bfloat16* in, const _
         const int zc = (c->nz + nch - 1) / nch;
         const int grid = cols * ((c->nz + zc - 1) / zc);
         const cl::Grid3 gr{c->nx, c->ny, c->nz, c->V};
-        K<<<grid, cl::conv_threads(COUT), smem, st>>>(gr, zc, in, reinterpret_cast<const uint4*>(img), bias, pre_below,
-                                             out_pre, out_bf, out_f, c->err, c->wait_limit);
-        CL_CUDA(cudaGetLastError());
+        CL_CUDA(launch_dependent(K, dim3(grid), cl::conv_threads(COUT), smem, st, gr, zc, in,
+                                 reinterpret_cast<const uint4*>(img), bias, pre_below, out_pre, out_bf, out_f, c->err,
+                                 c->wait_limit));
         return LBMAN_OK;
     }
     const int halo = cl::halo_ok(c->nx, c->ny) && cl::halo_bytes(c->nx, CIN) <= 96 * 1024 ? 1 : 0;
@@ -190,11 +191,9 @@ int run_wgrad(lbman_closure* c, cudaStream_t st, const __nv_bfloat16* a, const _
         constexpr auto K = cl::wgrad_march_kernel<CIN, COUT>;
         const int grid = (int)std::min<int64_t>(c->num_sms, c->V / cl::kTileM);
         CL_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, WM::SMEM));
-        K<<<grid, cl::kZThreads, WM::SMEM, st>>>(g3, a, gr, c->wpart, c->err, c->wait_limit);
-        CL_CUDA(cudaGetLastError());
-        cl::sum_partials_kernel<<<(WM::NOUT + 31) / 32, cl::kFoldThreads, 0, st>>>(c->wpart, grid, WM::NOUT,
-                                                                                    c->g + w_off(layer));
-        CL_CUDA(cudaGetLastError());
+        CL_CUDA(launch_dependent(K, dim3(grid), cl::kZThreads, WM::SMEM, st, g3, a, gr, c->wpart, c->err, c->wait_limit));
+        CL_CUDA(launch_dependent(cl::sum_partials_kernel, dim3((WM::NOUT + 31) / 32), cl::kFoldThreads, 0, st,
+                                 (const float*)c->wpart, grid, (int)WM::NOUT, c->g + w_off(layer)));
         return LBMAN_OK;
     }
     using WS = cl::WGradShape<CIN, COUT>;
@@ -237,9 +236,8 @@ int upload_scales(lbman_closure* c) {
 
 int features(lbman_closure* c, cudaStream_t st, const float* rho, const float* u3, const float* q5,
              float noise_std = 0.0f, uint64_t noise_key = 0) {
-    cl::features_kernel<<<c->Gb, 256, 0, st>>>(rho, u3, q5, c->V, c->scales, c->scales + 9, c->act0, noise_std,
-                                                noise_key);
-    CL_CUDA(cudaGetLastError());
+    CL_CUDA(launch_dependent(cl::features_kernel, dim3(c->Gb), 256, 0, st, rho, u3, q5, c->V, (const float*)c->scales,
+                             (const float*)(c->scales + 9), c->act0, noise_std, noise_key));
     return LBMAN_OK;
 }
 
@@ -271,8 +269,8 @@ int backward(lbman_closure* c, cudaStream_t st) {
 }
 
 int loss_grad(lbman_closure* c, cudaStream_t st, const float* tgt) {
-    cl::loss_kernel<<<c->Gb, cl::kThreads, 0, st>>>(c->out, tgt, c->scales + 26, c->V, c->gout, c->lpart);
-    CL_CUDA(cudaGetLastError());
+    CL_CUDA(launch_dependent(cl::loss_kernel, dim3(c->Gb), cl::kThreads, 0, st, (const float*)c->out, tgt,
+                             (const float*)(c->scales + 26), c->V, c->gout, c->lpart));
     return LBMAN_OK;
 }
 
@@ -599,9 +597,9 @@ static int corrected_step(lbman_closure* c, lbman_solver* coarse) {
     CL_TRY(solver_reset_populations(coarse));
     CL_TRY(lbman_step(coarse, 1));
     CL_TRY(solver_view(coarse, &w));
-    cl::apply_kernel<<<c->Gb, 256, 0, w.stream>>>(c->out, c->scales + 18, c->V, c->gain, static_cast<float*>(w.u),
-                                                  static_cast<float*>(w.q));
-    CL_CUDA(cudaGetLastError());
+    CL_CUDA(launch_dependent(cl::apply_kernel, dim3(c->Gb), 256, 0, w.stream, (const float*)c->out,
+                             (const float*)(c->scales + 18), c->V, c->gain, static_cast<float*>(w.u),
+                             static_cast<float*>(w.q)));
     return LBMAN_OK;
 }
 

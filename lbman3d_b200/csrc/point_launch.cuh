@@ -4,6 +4,7 @@
 #pragma once
 
 #include "launch.h"
+#include "pdl.cuh"
 #include "qpoint.cuh"
 
 #include <algorithm>
@@ -46,8 +47,10 @@ cudaError_t qpoint(const SimParams& P, bool pair, int num_sms, const void* qin, 
     const int per_block = kPointThreads * (pair ? 2 : 1);
     const int zc = point_walk(P.nxy, P.nz, per_block, num_sms);
     const dim3 g((unsigned)((P.nxy + per_block - 1) / per_block), (unsigned)((P.nz + zc - 1) / zc));
+    cudaError_t err = cudaErrorInvalidValue;
     auto launch = [&](auto k) {
-        k<<<g, kPointThreads, 0, st>>>(P, dnx, zc, (const R*)qin, (const R*)uin, (R*)qout, (R*)stress, (R*)F);
+        err = launch_dependent(k, g, kPointThreads, 0, st, P, dnx, zc, (const R*)qin, (const R*)uin, (R*)qout, (R*)stress,
+                               (R*)F);
     };
     with_mask(point_mask(P), [&](auto m) {
         constexpr int QW = decltype(m)::value;
@@ -61,7 +64,7 @@ cudaError_t qpoint(const SimParams& P, bool pair, int num_sms, const void* qin, 
         if (P.upwind) launch(qpoint_kernel<R, true, QW>);
         else launch(qpoint_kernel<R, false, QW>);
     });
-    return cudaGetLastError();
+    return err;
 }
 
 template <class R>
@@ -69,18 +72,21 @@ cudaError_t point_force(const SimParams& P, bool pair, const void* qn, const voi
                         cudaStream_t st) {
     const FastDiv dnx = make_fastdiv((uint32_t)P.nx), dnxy = make_fastdiv((uint32_t)P.nxy);
     const unsigned nb = (unsigned)((P.V + 255) / 256);
+    cudaError_t err = cudaErrorInvalidValue;
+    auto launch = [&](auto k) {
+        err = launch_dependent(k, dim3(nb), 256, 0, st, P, dnx, dnxy, (const R*)qn, (const R*)stress, (const R*)u, (R*)F);
+    };
     with_mask(point_mask(P), [&](auto m) {
         constexpr int QW = decltype(m)::value;
         if constexpr (sizeof(R) == 4) {
             if (pair) {
-                point_force_kernel<R, QW, true><<<nb, 256, 0, st>>>(P, dnx, dnxy, (const R*)qn, (const R*)stress,
-                                                                    (const R*)u, (R*)F);
+                launch(point_force_kernel<R, QW, true>);
                 return;
             }
         }
-        point_force_kernel<R, QW><<<nb, 256, 0, st>>>(P, dnx, dnxy, (const R*)qn, (const R*)stress, (const R*)u, (R*)F);
+        launch(point_force_kernel<R, QW, false>);
     });
-    return cudaGetLastError();
+    return err;
 }
 
 template <class R, class S, bool DEV>
@@ -88,9 +94,10 @@ cudaError_t lbm_aa_point(const SimParams& P, bool pair, bool odd, bool last, voi
                          const void* stress, void* F, void* rho, void* u, cudaStream_t st) {
     const FastDiv dnx = make_fastdiv((uint32_t)P.nx), dnxy = make_fastdiv((uint32_t)P.nxy);
     const unsigned nb = (unsigned)((P.V + kPointThreads - 1) / kPointThreads);
+    cudaError_t err = cudaErrorInvalidValue;
     auto launch = [&](auto k) {
-        k<<<nb, kPointThreads, 0, st>>>(P, dnx, dnxy, (S*)f, (const R*)qn, (const R*)stress, (R*)F, (R*)rho, (R*)u,
-                                        last ? 1 : 0);
+        err = launch_dependent(k, dim3(nb), kPointThreads, 0, st, P, dnx, dnxy, (S*)f, (const R*)qn, (const R*)stress,
+                               (R*)F, (R*)rho, (R*)u, last ? 1 : 0);
     };
     with_mask(point_mask(P), [&](auto m) {
         constexpr int QW = decltype(m)::value, WM = QW & 7;
@@ -101,10 +108,10 @@ cudaError_t lbm_aa_point(const SimParams& P, bool pair, bool odd, bool last, voi
                 return;
             }
         }
-        if (odd) launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, true>);
-        else launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, false>);
+        if (odd) launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, true, false>);
+        else launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, false, false>);
     });
-    return cudaGetLastError();
+    return err;
 }
 
 }  // namespace impl

@@ -34,6 +34,7 @@
 #pragma once
 
 #include "lbm.cuh"
+#include "pdl.cuh"
 #include "qforce.cuh"
 #include "qpair.cuh"
 
@@ -287,6 +288,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<R>())
     if (!live) col = n - 1;
     const int y = (int)fdiv((uint32_t)col, dnx), x = col - y * P.nx;
     const int z0 = (int)blockIdx.y * zc;
+    pdl_begin();
     qpoint_column<R, UPWIND, QW>(P, x, y, col, z0, min(z0 + zc, P.nz), live, qin, uin, qout, stress, F);
 }
 
@@ -450,6 +452,7 @@ __global__ void __launch_bounds__(kPointThreads, kPairPointMinBlocks)
     if (!live) col = n - 2;
     const int y = (int)fdiv((uint32_t)col, dnx), x = col - y * P.nx;
     const int z0 = (int)blockIdx.y * zc;
+    pdl_begin();
     qpoint2_column<UPWIND, QW>(P, x, y, col, z0, min(z0 + zc, P.nz), live, qin, uin, qout, stress, F);
 }
 
@@ -584,6 +587,7 @@ __global__ void __launch_bounds__(256)
     point_force_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, const R* __restrict__ qn,
                        const R* __restrict__ stress, const R* u, R* F) {
     const int c = (int)(blockIdx.x * 256 + threadIdx.x);
+    pdl_begin();
     if (c >= (int)P.V) return;
     const int V = (int)P.V;
     R out[3];
@@ -616,6 +620,7 @@ __global__ void __launch_bounds__(kPointThreads)
     lbm_aa_point_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, S* f, const R* __restrict__ qn,
                         const R* __restrict__ stress, R* F, R* __restrict__ rho_buf, R* u, int last) {
     const int c = (int)(blockIdx.x * kPointThreads + threadIdx.x);
+    pdl_begin();
     if (c >= (int)P.V) return;
     const KeptPointForce<R, QW, PAIR> force{{P, qn, stress, u, F}, F, last};
     if constexpr (ODD) aa_odd_cell<R, S, DEV, WM, int>(P, dnx, dnxy, c, f, force, rho_buf, u, last);
