@@ -15,15 +15,18 @@
     }                                                                                                          \
     cudaError_t launch_energy_reduce_##SUF(const SimParams& P, const void* q, double* partials, int G,         \
                                            cudaStream_t st) {                                                  \
-        energy_reduce_kernel<R><<<G, kRedThreads, 0, st>>>(P, (const R*)q, partials);                          \
+        const int64_t tiles = (int64_t)((P.nx + kEnX - 1) / kEnX) * ((P.ny + kEnY - 1) / kEnY);                \
+        energy_reduce_kernel<R><<<G, kRedThreads, 0, st>>>(P, diag_planes(tiles, P.zhi - P.zlo), (const R*)q,  \
+                                                           partials);                                          \
         return cudaGetLastError();                                                                             \
     }                                                                                                          \
     cudaError_t launch_defects_##SUF(const SimParams& P, const void* q, uint8_t* flags,                        \
                                      unsigned long long* count, cudaStream_t st) {                             \
         if (cudaError_t e = cudaMemsetAsync(count, 0, sizeof(*count), st)) return e;                           \
-        const dim3 g((unsigned)((P.nx + kDefX - 1) / kDefX), (unsigned)((P.ny + kDefY - 1) / kDefY),           \
-                     (unsigned)((P.nz + kDiagZ - 1) / kDiagZ));                                                \
-        defect_kernel<R><<<g, kDefThreads, 0, st>>>(P, (const R*)q, flags, count);                             \
+        const int gx = (P.nx + kDefX - 1) / kDefX, gy = (P.ny + kDefY - 1) / kDefY;                            \
+        const int zc = diag_planes((int64_t)gx * gy, P.nz);                                                    \
+        defect_kernel<R><<<dim3(gx, gy, (P.nz + zc - 1) / zc), kDefThreads, 0, st>>>(P, zc, (const R*)q,       \
+                                                                                     flags, count);            \
         return cudaGetLastError();                                                                             \
     }                                                                                                          \
     }

@@ -89,7 +89,7 @@ constexpr int kEnsLbmCells = 4 * kPointThreads;
 
 // par: the buffer holding Q_new.
 template <class R, class S, bool DEV, bool ODD>
-__global__ void __launch_bounds__(kPointThreads)
+__global__ void __launch_bounds__(kPointThreads, sizeof(R) == 4 ? 8 : 4)
     ens_lbm_point_kernel(const EnsBox* __restrict__ boxes, const EnsLbmWork* __restrict__ work, int par, int fcur,
                          int last) {
     __shared__ __align__(16) uint32_t buf[sizeof(EnsBox) / 4];

@@ -12,6 +12,8 @@
 
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace lbman {
 
 constexpr int kRedThreads = 256;
@@ -50,28 +52,6 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NQ], double* part
     }
 }
 
-// Four consecutive values as one load / store (float: 16 bytes, double: 32).
-template <class R>
-struct Quad {
-    R v[4];
-};
-__device__ __forceinline__ Quad<float> ld4(const float* p) {
-    const float4 a = *reinterpret_cast<const float4*>(p);
-    return {{a.x, a.y, a.z, a.w}};
-}
-__device__ __forceinline__ Quad<double> ld4(const double* p) {
-    const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
-    return {{a.x, a.y, b.x, b.y}};
-}
-__device__ __forceinline__ void st4(float* p, const Quad<float>& q) {
-    *reinterpret_cast<float4*>(p) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]);
-}
-__device__ __forceinline__ void st4(double* p, const Quad<double>& q) {
-    *reinterpret_cast<double2*>(p) = make_double2(q.v[0], q.v[1]);
-    *reinterpret_cast<double2*>(p + 2) = make_double2(q.v[2], q.v[3]);
-}
-__device__ __forceinline__ bool quad_ok(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
 __device__ __forceinline__ void flow_cell(double (&v)[kFlowQ], double r, double ux, double uy, double uz, double px,
                                           double py, double pz) {
     v[0] += r;
@@ -85,48 +65,54 @@ __device__ __forceinline__ void flow_cell(double (&v)[kFlowQ], double r, double 
     v[7] = fmax(v[7], u2);
 }
 
-// Memory bound (10 words per cell): four cells per thread where every array
-// allows 16-byte accesses (256^3 FP32: 161 us one cell at a time).
+// Memory bound (10 words per cell): two cells per thread and turn, all their
+// loads issued before the first use.  256^3 FP32: 111 us; one cell at a time
+// 161-191 us, four neighbouring cells as 16-byte accesses 424 us (the lanes'
+// accesses to seven arrays at that stride collide in the cache).
 template <class R>
 __global__ void __launch_bounds__(kRedThreads) flow_reduce_kernel(SimParams P, const R* __restrict__ rho,
                                                                   const R* __restrict__ u,
                                                                   R* __restrict__ upast,
                                                                   double* __restrict__ partials) {
-    const int64_t V = P.V;
+    const int64_t V = P.V, nt = (int64_t)gridDim.x * blockDim.x;
     double v[kFlowQ] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
-    if (V % 4 == 0 && P.c0 % 4 == 0 && P.c1 % 4 == 0 && quad_ok(rho) && quad_ok(u) && quad_ok(upast)) {
-        for (int64_t c = P.c0 + 4 * t; c < P.c1; c += 4 * nt) {
-            const Quad<R> r = ld4(rho + c);
-            Quad<R> a[3], b[3];
+    for (int64_t c = P.c0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < P.c1; c += 2 * nt) {
+        R r[2], a[2][3], b[2][3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                a[k] = ld4(u + k * V + c);
-                b[k] = ld4(upast + k * V + c);
+        for (int i = 0; i < 2; ++i) {
+            const int64_t d = c + i * nt;
+            if (d < P.c1) {
+                r[i] = rho[d];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    a[i][k] = u[k * V + d];
+                    b[i][k] = upast[k * V + d];
+                }
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                flow_cell(v, (double)r.v[i], (double)a[0].v[i], (double)a[1].v[i], (double)a[2].v[i], (double)b[0].v[i],
-                          (double)b[1].v[i], (double)b[2].v[i]);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) st4(upast + k * V + c, a[k]);
         }
-    } else {
-        for (int64_t c = P.c0 + t; c < P.c1; c += nt) {
-            const R ux = u[c], uy = u[V + c], uz = u[2 * V + c];
-            flow_cell(v, (double)rho[c], (double)ux, (double)uy, (double)uz, (double)upast[c], (double)upast[V + c],
-                      (double)upast[2 * V + c]);
-            upast[c] = ux;
-            upast[V + c] = uy;
-            upast[2 * V + c] = uz;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int64_t d = c + i * nt;
+            if (d < P.c1) {
+                flow_cell(v, (double)r[i], (double)a[i][0], (double)a[i][1], (double)a[i][2], (double)b[i][0],
+                          (double)b[i][1], (double)b[i][2]);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) upast[k * V + d] = a[i][k];
+            }
         }
     }
     block_reduce_store<kFlowQ, 1>(v, partials);
 }
 
-// Tiles of the z-marching diagnostics: one thread per (x, y) column of a tile,
-// kDiagZ planes per work item.
-constexpr int kDiagZ = 32;
+// Planes per work item of the z-marching diagnostics (one thread per column of
+// an x-y tile): as many as leave 8 items for each of the part's 148 SMs, between
+// 2 and 32 -- a longer march re-reads less, a shorter one fills the chip.
+// Defects, 20x100x100 FP64: 18 us at 2 planes, 70 us at 32; 256^3 FP32: 610 us
+// at 2, 472 us at 32.  Energy: 13 / 31 us and 337 / 252 us.
+inline int diag_planes(int64_t tiles, int nz) {
+    const int64_t chunks = (8 * 148 + tiles - 1) / tiles;
+    return (int)std::max<int64_t>(2, std::min<int64_t>(32, (nz + chunks - 1) / chunks));
+}
 
 // Index of the neighbour a + s under the QXoff clamp / wrap of one axis.
 __device__ __forceinline__ int qx_off(int a, int n, int per_lo, int per_hi) {
@@ -138,21 +124,24 @@ __device__ __forceinline__ int qx_off(int a, int n, int per_lo, int per_hi) {
 // NematicFreeEnergyDensity with the QXoff-clamped 7-point Laplacian, in FP64.
 // FP32 fields: a value is converted once -- each thread converts its own
 // column, keeps three planes of it in registers and shares the current plane
-// through shared memory -- because the conversions, at a quarter of the FP64
-// rate or less, were what bounded the one-thread-per-cell form (35 per cell;
-// 256^3: 331 us).
+// through shared memory -- because the conversions (a fraction of the FP64
+// rate) were what bounded the one-thread-per-cell form, with 35 per cell.  The
+// next plane's values are loaded while this one is worked on.  256^3 FP32:
+// 331 us one thread per cell, 252 us now at 3 blocks per SM (293 at 2, 294 at
+// 4, which spills); FP64, which converts nothing: 343-352 us at 2 blocks, 369 at 3.
 constexpr int kEnX = 32, kEnY = 8;
 static_assert(kEnX * kEnY == kRedThreads, "one thread per column of a tile");
 template <class R>
-__global__ void __launch_bounds__(kRedThreads) energy_reduce_kernel(const __grid_constant__ SimParams P,
-                                                                    const R* __restrict__ q,
+__global__ void __launch_bounds__(kRedThreads, sizeof(R) == 4 ? 3 : 2) energy_reduce_kernel(const __grid_constant__ SimParams P,
+                                                                    int zc, const R* __restrict__ q,
                                                                     double* __restrict__ partials) {
     constexpr int SX = kEnX + 2, SY = kEnY + 2;
-    __shared__ double sh[5][SY][SX];
+    __shared__ double sh[2][5][SY][SX];
     const int64_t V = P.V;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     double v[1] = {0.0};
-    const int gx = (nx + kEnX - 1) / kEnX, gy = (ny + kEnY - 1) / kEnY, gz = (P.zhi - P.zlo + kDiagZ - 1) / kDiagZ;
+    int b = 0;
+    const int gx = (nx + kEnX - 1) / kEnX, gy = (ny + kEnY - 1) / kEnY, gz = (P.zhi - P.zlo + zc - 1) / zc;
     const int lx = threadIdx.x % kEnX, ly = threadIdx.x / kEnX;
     // this thread's halo point of a plane (threads 0 .. 2 (kEnX + kEnY) - 1)
     const int h = threadIdx.x;
@@ -160,30 +149,44 @@ __global__ void __launch_bounds__(kRedThreads) energy_reduce_kernel(const __grid
     const int hx = h < 2 * kEnX ? h % kEnX + 1 : (h - 2 * kEnX < kEnY ? 0 : SX - 1);
     const int hy = h < 2 * kEnX ? (h < kEnX ? 0 : SY - 1) : (h - 2 * kEnX) % kEnY + 1;
     for (int item = blockIdx.x; item < gx * gy * gz; item += gridDim.x) {
-        const int x0 = item % gx * kEnX, y0 = item / gx % gy * kEnY, z0 = P.zlo + item / (gx * gy) * kDiagZ;
-        const int z1 = min(z0 + kDiagZ, P.zhi);
+        const int x0 = item % gx * kEnX, y0 = item / gx % gy * kEnY, z0 = P.zlo + item / (gx * gy) * zc;
+        const int z1 = min(z0 + zc, P.zhi);
         const int x = x0 + lx, y = y0 + ly;
         const bool live = x < nx && y < ny;
         const int64_t col = (int64_t)min(y, ny - 1) * nx + min(x, nx - 1);
         const int64_t hcol = (int64_t)qx_off(min(y0 + hy - 1, ny), ny, P.qper[2], P.qper[3]) * nx +
                              qx_off(min(x0 + hx - 1, nx), nx, P.qper[0], P.qper[1]);
-        double qm[5], qc[5], qp[5];
+        const R* const qx = q + col;
+        const R* const qh = q + hcol;
+        double qm[5], qc[5];
+        R rp[5], rh[5];  // plane z + 1 of the column, plane z of the halo point
         const int64_t zm0 = (int64_t)qx_off(z0 - 1, nz, P.qper[4], P.qper[5]) * P.nxy;
+        const int64_t zp0 = (int64_t)qx_off(z0 + 1, nz, P.qper[4], P.qper[5]) * P.nxy;
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            qm[k] = (double)q[k * V + zm0 + col];
-            qc[k] = (double)q[k * V + (int64_t)z0 * P.nxy + col];
+            qm[k] = (double)qx[k * V + zm0];
+            qc[k] = (double)qx[k * V + (int64_t)z0 * P.nxy];
+            rp[k] = qx[k * V + zp0];
+            rh[k] = qh[k * V + (int64_t)z0 * P.nxy];
         }
         for (int z = z0; z < z1; ++z) {
-            const int64_t zp = (int64_t)qx_off(z + 1, nz, P.qper[4], P.qper[5]) * P.nxy;
-            __syncthreads();  // the previous plane has been read
+            b ^= 1;
+            double qp[5];
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
-                qp[k] = (double)q[k * V + zp + col];
-                sh[k][ly + 1][lx + 1] = qc[k];
-                if (halo) sh[k][hy][hx] = (double)q[k * V + (int64_t)z * P.nxy + hcol];
+                sh[b][k][ly + 1][lx + 1] = qc[k];
+                if (halo) sh[b][k][hy][hx] = (double)rh[k];
+                qp[k] = (double)rp[k];
             }
-            __syncthreads();
+            __syncthreads();  // the other buffer's readers are at most one plane behind
+            if (z + 1 < z1) {
+                const int64_t zn = (int64_t)qx_off(z + 2, nz, P.qper[4], P.qper[5]) * P.nxy;
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    rp[k] = qx[k * V + zn];
+                    rh[k] = qh[k * V + (int64_t)(z + 1) * P.nxy];
+                }
+            }
             if (live) {
                 // the neighbour beyond a partial tile's last cell comes from
                 // global memory (its shared slot holds a column outside the box)
@@ -193,11 +196,11 @@ __global__ void __launch_bounds__(kRedThreads) energy_reduce_kernel(const __grid
                     const R* a = q + k * V + (int64_t)z * P.nxy;
                     const double xp = (x == nx - 1 && lx != kEnX - 1)
                                           ? (double)a[(int64_t)y * nx + qx_off(nx, nx, P.qper[0], P.qper[1])]
-                                          : sh[k][ly + 1][lx + 2];
+                                          : sh[b][k][ly + 1][lx + 2];
                     const double yp = (y == ny - 1 && ly != kEnY - 1)
                                           ? (double)a[(int64_t)qx_off(ny, ny, P.qper[2], P.qper[3]) * nx + x]
-                                          : sh[k][ly + 2][lx + 1];
-                    l[k] = xp + sh[k][ly + 1][lx] + yp + sh[k][ly][lx + 1] + qp[k] + qm[k] - 6.0 * qc[k];
+                                          : sh[b][k][ly + 2][lx + 1];
+                    l[k] = xp + sh[b][k][ly + 1][lx] + yp + sh[b][k][ly][lx + 1] + qp[k] + qm[k] - 6.0 * qc[k];
                 }
                 const double Qxx = qc[0], Qxy = qc[1], Qxz = qc[2], Qyy = qc[3], Qyz = qc[4];
                 const double half = (Qxx * Qxx + Qxx * Qyy + Qyy * Qyy + Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
@@ -282,7 +285,7 @@ __device__ __forceinline__ bool plaquette_flip(const R d1[3], const R d2[3], con
 //   (nx-1)*ny*(nz-1), then def_z (nx-1)*(ny-1)*nz, each x fastest.
 constexpr int kDefTX = 32, kDefTY = 16, kDefX = kDefTX - 1, kDefY = kDefTY - 1, kDefThreads = kDefTX * kDefTY;
 template <class R>
-__global__ void __launch_bounds__(kDefThreads) defect_kernel(const __grid_constant__ SimParams P,
+__global__ void __launch_bounds__(kDefThreads) defect_kernel(const __grid_constant__ SimParams P, int zc,
                                                              const R* __restrict__ q, uint8_t* __restrict__ flags,
                                                              unsigned long long* __restrict__ count) {
     __shared__ R sh[2][3][kDefTY][kDefTX];
@@ -292,7 +295,7 @@ __global__ void __launch_bounds__(kDefThreads) defect_kernel(const __grid_consta
     const int64_t nfx = (int64_t)nx * (ny - 1) * (nz - 1), nfy = (int64_t)(nx - 1) * ny * (nz - 1);
     const int lx = threadIdx.x % kDefTX, ly = threadIdx.x / kDefTX;
     const int x = blockIdx.x * kDefX + lx, y = blockIdx.y * kDefY + ly;
-    const int z0 = blockIdx.z * kDiagZ, z1 = min(z0 + kDiagZ, nz);  // def_z planes of this block
+    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);  // def_z planes of this block
     const bool in = x < nx && y < ny;
     const bool own = in && lx < kDefX && ly < kDefY;
     const int64_t col = (int64_t)y * nx + x;
