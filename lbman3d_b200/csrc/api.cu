@@ -228,22 +228,26 @@ int default_zchunk(int nx, int ny, int nz, int tcx, int tcy, int num_sms) {
 }
 
 // Largest box (cells) an untuned AUTO handle steps with the point kernels
-// (qpoint.cuh), whole steps timed on B200 against the z-marching kernels:
-//   FP64             faster at every size tried (32^3 67 -> 12 us, 256^3 2865 ->
-//                    2100 us); the kernels index 15 V in 32 bits
-//   FP32, one point  64x256x256 slit 280 -> 248 us, 256^3 939 -> 969 us
-//   FP32, packed     120x128x128 Q stage 102 -> 80 us; 256^3 541 -> 512 us alone,
-//                    but the FP16 step there 1.00 -> 1.02 ms (the stress is 72 B
-//                    of HBM traffic per cell)
-int64_t point_limit(int prec) {
-    if (prec == LBMAN_FP64) return (((int64_t)1 << 31) - 1) / 15;
-    return (int64_t)8 << 20;
-}
+// (qpoint.cuh): they index 15 V in 32 bits.  Below that they were the faster
+// ones at every size tried.  Whole steps on B200, z-marching kernels -> these:
+//   FP64             32^3 67 -> 8 us, 256^3 2865 -> 2100 us
+//   FP32, one point  64x256x256 slit 282 -> 243 us, 256^3 slit 981 -> 834 us,
+//                    301x300x300 channel 2914 -> 1766 us
+//   FP32, packed     128^3 139 -> 126 us, 256^3 944 -> 803 us, 512x512x256
+//                    3547 -> 3216 us
+//   FP16, packed     256^3 844 -> 664 us, 512x512x256 3136 -> 2745 us
+constexpr int64_t kPointCells = (((int64_t)1 << 31) - 1) / 15;
 
-// Up to this size the LBM kernel forms the body force itself (one launch and
-// the force's round trip less); above it a force kernel runs before the LBM
-// step (FP32 64x256x256: 248 us fused, 264 us apart; 256^3: 995 and 969 us).
+// FP64: up to this size the LBM kernel forms the body force itself (one launch
+// and the force's round trip less); above it a force kernel runs before the LBM
+// step.  FP32 forms it there at every size
+// (256^3 slit, a force kernel / formed there: 858 / 834 us, FP16 801 / 746 us).
 constexpr int64_t kPointFusedCells = (int64_t)6 << 20;
+
+// Memory (words per cell) a handle must leave free when it takes the point
+// kernels' scratch: the buffers it may ask for later (second population buffer,
+// two-phase stress, snapshots, statistics), so that none of them fails for it.
+constexpr int64_t kPointSpareWords = 48;
 
 // Default z-marching tile before any autotuning: the widest compiled tile
 // up to 32 cells whose last partial tile pads x by at most 10% (wide rows
@@ -470,10 +474,14 @@ int lbman_create(const lbman_config* cfg, lbman_solver** out) {
         if (int st = alloc(&s->u[b], 3 * V * s->rbytes)) return bail(st);
     }
     if (cfg->kernels == LBMAN_KERNELS_AUTO && cfg->tile_x == 0 && cfg->tile_y == 0 && cfg->zchunk == 0 &&
-        V <= point_limit(s->prec)) {
+        V <= kPointCells) {
         // 9 row-stress words (FP32) or Sigma and tau (FP64) per cell; a box that
         // has no room for them keeps the z-marching kernels
-        s->point = cudaMalloc(&s->pstress, (s->prec == LBMAN_FP64 ? 8 : 9) * V * s->rbytes) == cudaSuccess;
+        const size_t words = s->prec == LBMAN_FP64 ? 8 : 9;
+        size_t free_bytes = 0, total = 0;
+        if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess &&
+            (words + kPointSpareWords) * V * s->rbytes <= free_bytes)
+            s->point = cudaMalloc(&s->pstress, words * V * s->rbytes) == cudaSuccess;
         if (!s->point) {
             cudaGetLastError();
             s->pstress = nullptr;
@@ -706,7 +714,8 @@ static int q_stage(lbman_solver* s, bool force) {
                                         s->pstress, s->F, s->stream),
                             "qpoint"));
         if (force)
-            LB_TRY(check_launch(s, o.point_force(s->P, pair, s->q[1 - s->qcur], s->pstress, s->u[s->ucur], s->F, s->stream),
+            LB_TRY(check_launch(s, o.point_force(s->P, pair, s->num_sms, s->q[1 - s->qcur], s->pstress, s->u[s->ucur], s->F,
+                                              s->stream),
                                 "point_force"));
     } else {
         LB_TRY(check_launch(s, o.qforce(s->P, s->shape, s->q[s->qcur], s->u[s->ucur], s->q[1 - s->qcur], s->F, s->stream),
@@ -734,12 +743,13 @@ static int one_step(lbman_solver* s, bool last) {
         s->ucur ^= 1;
         s->fcur ^= 1;
         s->fphase = F_POST;
-    } else if (s->point && s->P.V <= kPointFusedCells) {
+    } else if (s->point && (s->prec != LBMAN_FP64 || s->P.V <= kPointFusedCells)) {
         LB_TRY(q_stage(s, false));
         LB_TRY(aa_layout(s));
         const bool odd = s->fphase == F_SWAP;
-        LB_TRY(check_launch(s, o.lbm_aa_point(s->P, s->kernels == LBMAN_KERNELS_SPLIT_PAIR, odd, last, s->f[s->fcur],
-                                              s->q[s->qcur], s->pstress, s->F, s->rho, s->u[s->ucur], s->stream),
+        LB_TRY(check_launch(s, o.lbm_aa_point(s->P, s->kernels == LBMAN_KERNELS_SPLIT_PAIR, s->num_sms, odd, last,
+                                              s->f[s->fcur], s->q[s->qcur], s->pstress, s->F, s->rho, s->u[s->ucur],
+                                              s->stream),
                             "lbm_aa_point"));
         s->fphase = odd ? F_PRE : F_SWAP;
     } else {
@@ -957,7 +967,6 @@ int lbman_defect_lines(lbman_solver* s, lbman_defects* info, double* points, int
     const int nx = s->P.nx, ny = s->P.ny, nz = s->P.nz;
     if (nx < 2 || ny < 2 || nz < 2) return fail(LBMAN_ERR_ARG, "defect lines need at least 2 cells per side");
     LB_TRY(set_device(s));
-    const int64_t V = s->P.V;
     const int64_t nf = (int64_t)nx * (ny - 1) * (nz - 1) + (int64_t)(nx - 1) * ny * (nz - 1) +
                        (int64_t)(nx - 1) * (ny - 1) * nz;
     uint8_t* dflags = nullptr;

@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(kPointThreads, sizeof(R) == 4 ? 8 : 4)
     const R* qn = (const R*)(par ? B.q[1] : B.q[0]);
     ens_with_mask(B.mask, [&](auto m) {
         constexpr int QW = decltype(m)::value, WM = QW & 7;
-        const KeptPointForce<R, QW, false> force{{P, qn, (const R*)B.stress, (const R*)B.u[0], (const R*)B.F}, (R*)B.F, last};
+        const KeptPointForce<R, QW, false> force{
+            {P, 0, qn, (const R*)B.stress, (const R*)B.u[0], (const R*)B.F}, (R*)B.F, last};
 #pragma unroll 1
         for (int c = c0; c < c1; c += kPointThreads) {
             if constexpr (ODD)

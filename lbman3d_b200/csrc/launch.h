@@ -60,9 +60,9 @@ struct LaunchShape {
     cudaError_t launch_qpoint_##SUF(const SimParams& P, bool pair, int num_sms, const void* qin,        \
                                     const void* uin, void* qout, void* stress, void* F,                \
                                     cudaStream_t st);                                                  \
-    cudaError_t launch_point_force_##SUF(const SimParams& P, bool pair, const void* qn,                 \
+    cudaError_t launch_point_force_##SUF(const SimParams& P, bool pair, int num_sms, const void* qn,    \
                                          const void* stress, const void* u, void* F, cudaStream_t st); \
-    cudaError_t launch_lbm_aa_point_##SUF(const SimParams& P, bool pair, bool odd, bool last, void* f,  \
+    cudaError_t launch_lbm_aa_point_##SUF(const SimParams& P, bool pair, int num_sms, bool odd, bool last, void* f, \
                                           const void* qn, const void* stress, void* F, void* rho,      \
                                           void* u, cudaStream_t st);                                   \
     size_t qforce_smem_##SUF(const QTile& T);                                                          \

@@ -571,23 +571,41 @@ __global__ void __launch_bounds__(256, lbm_min_blocks<R, S, WM != 0>())
 // stays race-free.  Plain loads on F: this kernel writes it.  (Device code
 // only: host C++ checks of this header skip it.)
 #if defined(__CUDACC__)
-template <bool DEV, class I>
-__global__ void __launch_bounds__(256, 4)
-    lbm_aa_even_h2_kernel(const __grid_constant__ SimParams P, __half* F, const float* __restrict__ Fb,
-                          float* __restrict__ rho_buf, float* __restrict__ uout, int write_rho_all) {
-    const I c = (I)P.c0 + 2 * ((I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x);
-    if (c >= (I)P.c1) return;
+// Force source of the two cells: begin(c, position of c) once, then get<i>.
+// This one reads the force's array, each cell's values when they are used.
+template <class I>
+struct LoadForce2 {
+    const float* __restrict__ Fb;
+    I V;
+    struct Values {
+        const float* p;
+        I V;
+        template <int K>
+        __device__ __forceinline__ void get(float f[3]) const {
+            f[0] = __ldg(p + K);
+            f[1] = __ldg(p + V + K);
+            f[2] = __ldg(p + 2 * V + K);
+        }
+    };
+    __device__ __forceinline__ Values begin(I c, const CellPos&) const { return {Fb + c, V}; }
+};
+
+template <bool DEV, class I, class Force>
+__device__ __forceinline__ void aa_even_h2(const SimParams& P, I c, const CellPos& q, __half* F, const Force& force,
+                                           float* __restrict__ rho_buf, float* __restrict__ uout, int write_rho_all) {
     const I V = (I)P.V;
     const Phys<float>& K = phys_ref<float>(P);
     __half2 w[15];
 #pragma unroll
     for (int j = 0; j < 15; ++j) w[j] = *reinterpret_cast<const __half2*>(F + j * V + c);
-    float f[15];
+    const auto fs = force.begin(c, q);
+    float f[15], Fc[3];
     float rho, ux, uy, uz;
     // cell c; its post-collision values replace the low halves
 #pragma unroll
     for (int j = 0; j < 15; ++j) f[j] = __low2float(w[j]);
-    collide<float, DEV>(K, f, __ldg(Fb + c), __ldg(Fb + V + c), __ldg(Fb + 2 * V + c), rho, ux, uy, uz);
+    fs.template get<0>(Fc);
+    collide<float, DEV>(K, f, Fc[0], Fc[1], Fc[2], rho, ux, uy, uz);
 #pragma unroll
     for (int j = 0; j < 15; ++j) w[j] = __halves2half2(__float2half_rn(f[j]), __high2half(w[j]));
     uout[c] = ux;
@@ -598,7 +616,8 @@ __global__ void __launch_bounds__(256, 4)
     const I c1 = c + 1;
 #pragma unroll
     for (int j = 0; j < 15; ++j) f[j] = __high2float(w[j]);
-    collide<float, DEV>(K, f, __ldg(Fb + c1), __ldg(Fb + V + c1), __ldg(Fb + 2 * V + c1), rho, ux, uy, uz);
+    fs.template get<1>(Fc);
+    collide<float, DEV>(K, f, Fc[0], Fc[1], Fc[2], rho, ux, uy, uz);
     // V through an empty asm: the 15 store addresses are formed here rather
     // than kept live from the loads across both collisions (64 registers and
     // 4 blocks per SM instead of 80 and 3)
@@ -616,24 +635,16 @@ __global__ void __launch_bounds__(256, 4)
     if (write_rho_all) rho_buf[c1] = rho;
 }
 
-template <bool DEV, class I>
-__global__ void __launch_bounds__(256, 3)
-    lbm_aa_odd_h2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, __half* F,
-                         const float* __restrict__ Fb, float* __restrict__ rho_buf, float* __restrict__ uout,
-                         int write_rho_all) {
-    const I c = (I)P.c0 + 2 * ((I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x);
-    if (c >= (I)P.c1) return;
+template <bool DEV, class I, class Force>
+__device__ __forceinline__ void aa_odd_h2(const SimParams& P, I c, const CellPos& q, __half* F, const Force& force,
+                                          float* __restrict__ rho_buf, float* __restrict__ uout, int write_rho_all) {
     const I V = (I)P.V;
     const Phys<float>& K = phys_ref<float>(P);
-    CellPos q;
-    q.z = (int)fdiv((uint32_t)c, dnxy);
-    const uint32_t r = (uint32_t)((int64_t)c - (int64_t)q.z * P.nxy);
-    q.y = (int)fdiv(r, dnx);
-    q.x = (int)(r - (uint32_t)q.y * (uint32_t)P.nx);
     const AxisOff<I> o0 = axis_off<I>(P, q);  // cell c (x even)
     CellPos q1 = q;
     q1.x += 1;
     const AxisOff<I> o1 = axis_off<I>(P, q1);  // cell c + 1: only the x offsets differ
+    const auto fs = force.begin(c, q);
     // gather: every load of both cells issued before the first widening;
     // directions without an x component load both cells as one word, the
     // others load two halves, packed into one word once all are in flight
@@ -651,13 +662,14 @@ __global__ void __launch_bounds__(256, 3)
 #pragma unroll
     for (int j = 0; j < 15; ++j)
         if (ex_(j) != 0) w[j] = __halves2half2(a[j], b[j]);
-    float f[15];
+    float f[15], Fc[3];
     float rho, ux, uy, uz;
     // cell c; the directions without an x component keep its value in the
     // low half until cell c + 1's joins it
 #pragma unroll
     for (int j = 0; j < 15; ++j) f[j] = __low2float(w[j]);
-    collide<float, DEV>(K, f, __ldg(Fb + c), __ldg(Fb + V + c), __ldg(Fb + 2 * V + c), rho, ux, uy, uz);
+    fs.template get<0>(Fc);
+    collide<float, DEV>(K, f, Fc[0], Fc[1], Fc[2], rho, ux, uy, uz);
     // scatter: f*_k to slot k of c + e_k (= c - e_opp(k))
 #pragma unroll
     for (int k = 0; k < 15; ++k) {
@@ -672,7 +684,8 @@ __global__ void __launch_bounds__(256, 3)
     const I c1 = c + 1;
 #pragma unroll
     for (int j = 0; j < 15; ++j) f[j] = __high2float(w[j]);
-    collide<float, DEV>(K, f, __ldg(Fb + c1), __ldg(Fb + V + c1), __ldg(Fb + 2 * V + c1), rho, ux, uy, uz);
+    fs.template get<1>(Fc);
+    collide<float, DEV>(K, f, Fc[0], Fc[1], Fc[2], rho, ux, uy, uz);
 #pragma unroll
     for (int k = 0; k < 15; ++k) {
         if (ex_(k) == 0) {
@@ -686,6 +699,25 @@ __global__ void __launch_bounds__(256, 3)
     uout[V + c1] = uy;
     uout[2 * V + c1] = uz;
     if (write_rho_all) rho_buf[c1] = rho;
+}
+
+template <bool DEV, class I>
+__global__ void __launch_bounds__(256, 4)
+    lbm_aa_even_h2_kernel(const __grid_constant__ SimParams P, __half* F, const float* __restrict__ Fb,
+                          float* __restrict__ rho_buf, float* __restrict__ uout, int write_rho_all) {
+    const I c = (I)P.c0 + 2 * ((I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x);
+    if (c >= (I)P.c1) return;
+    aa_even_h2<DEV, I>(P, c, CellPos{0, 0, 0}, F, LoadForce2<I>{Fb, (I)P.V}, rho_buf, uout, write_rho_all);
+}
+
+template <bool DEV, class I>
+__global__ void __launch_bounds__(256, 3)
+    lbm_aa_odd_h2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, __half* F,
+                         const float* __restrict__ Fb, float* __restrict__ rho_buf, float* __restrict__ uout,
+                         int write_rho_all) {
+    const I c = (I)P.c0 + 2 * ((I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x);
+    if (c >= (I)P.c1) return;
+    aa_odd_h2<DEV, I>(P, c, cell_pos<I>(P, c, dnx, dnxy), F, LoadForce2<I>{Fb, (I)P.V}, rho_buf, uout, write_rho_all);
 }
 #endif  // __CUDACC__
 

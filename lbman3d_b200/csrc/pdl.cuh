@@ -7,7 +7,7 @@
 // memory that another kernel writes.  pdl_begin() waits first and only then
 // lets the next kernel start, so whatever runs early can rely on every kernel
 // before its predecessor being complete.  Small boxes are bound by launches: a
-// 32^3 FP64 step of two kernels takes 11.4 us without and 8 us with the overlap.
+// 32^3 FP64 step of two kernels takes 11.4 us without and 7.8 us with the overlap.
 #pragma once
 
 #include <cuda_runtime.h>

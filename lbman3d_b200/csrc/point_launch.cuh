@@ -31,13 +31,20 @@ void with_mask(int m, F&& f) {
     else f(std::integral_constant<int, 15>{});
 }
 
-// Planes per thread: the longest walk (at most 4, where the gain ends) that
-// still gives 16 blocks per SM.
-inline int point_walk(int64_t nxy, int nz, int cells_per_block, int num_sms) {
-    const int64_t cols = (nxy + cells_per_block - 1) / cells_per_block;
-    int zc = 4;
-    while (zc > 1 && cols * ((nz + zc - 1) / zc) < (int64_t)16 * num_sms) zc /= 2;
-    return std::min(zc, nz);
+// Planes per thread (a power of two): the longest walk that still gives every
+// SM a few blocks.  At most 4 planes, where the gain of reusing the centre
+// values ends, and 16 blocks per SM; packed kernels on planes with long walks
+// (long_walks), where a walk also saves the z terms' trip through memory, at
+// most 16 planes and 6 blocks per SM.  Steps with 1 / 2 / 4 / 8 / 16 planes there:
+// 128^3 138 / 135 / 131 / 127 / 131 us (the rule: 8), 160^3 274 / 261 / 254 / 249 /
+// 247 us (16).
+inline int point_walk(const SimParams& P, bool pair, int num_sms) {
+    const bool longer = pair && long_walks(P);
+    const int per_block = kPointThreads * (pair ? 2 : 1);
+    const int64_t cols = (P.nxy + per_block - 1) / per_block, blocks = (int64_t)(longer ? 6 : 16) * num_sms;
+    int zc = longer ? 16 : 4;
+    while (zc > 1 && cols * ((P.nz + zc - 1) / zc) < blocks) zc /= 2;
+    return zc;
 }
 
 template <class R>
@@ -45,7 +52,7 @@ cudaError_t qpoint(const SimParams& P, bool pair, int num_sms, const void* qin, 
                    void* stress, void* F, cudaStream_t st) {
     const FastDiv dnx = make_fastdiv((uint32_t)P.nx);
     const int per_block = kPointThreads * (pair ? 2 : 1);
-    const int zc = point_walk(P.nxy, P.nz, per_block, num_sms);
+    const int zc = point_walk(P, pair, num_sms);
     const dim3 g((unsigned)((P.nxy + per_block - 1) / per_block), (unsigned)((P.nz + zc - 1) / zc));
     cudaError_t err = cudaErrorInvalidValue;
     auto launch = [&](auto k) {
@@ -56,8 +63,9 @@ cudaError_t qpoint(const SimParams& P, bool pair, int num_sms, const void* qin, 
         constexpr int QW = decltype(m)::value;
         if constexpr (sizeof(R) == 4) {
             if (pair) {
-                if (P.upwind) launch(qpoint2_kernel<true, QW>);
-                else launch(qpoint2_kernel<false, QW>);
+                const bool walks = long_walks(P);
+                if (P.upwind) launch(walks ? qpoint2_kernel<true, QW, true> : qpoint2_kernel<true, QW, false>);
+                else launch(walks ? qpoint2_kernel<false, QW, true> : qpoint2_kernel<false, QW, false>);
                 return;
             }
         }
@@ -68,19 +76,20 @@ cudaError_t qpoint(const SimParams& P, bool pair, int num_sms, const void* qin, 
 }
 
 template <class R>
-cudaError_t point_force(const SimParams& P, bool pair, const void* qn, const void* stress, const void* u, void* F,
-                        cudaStream_t st) {
+cudaError_t point_force(const SimParams& P, bool pair, int num_sms, const void* qn, const void* stress, const void* u,
+                        void* F, cudaStream_t st) {
     const FastDiv dnx = make_fastdiv((uint32_t)P.nx), dnxy = make_fastdiv((uint32_t)P.nxy);
     const unsigned nb = (unsigned)((P.V + 255) / 256);
+    const int zm = point_walk(P, pair, num_sms) - 1;
     cudaError_t err = cudaErrorInvalidValue;
     auto launch = [&](auto k) {
-        err = launch_dependent(k, dim3(nb), 256, 0, st, P, dnx, dnxy, (const R*)qn, (const R*)stress, (const R*)u, (R*)F);
+        err = launch_dependent(k, dim3(nb), 256, 0, st, P, dnx, dnxy, zm, (const R*)qn, (const R*)stress, (const R*)u, (R*)F);
     };
     with_mask(point_mask(P), [&](auto m) {
         constexpr int QW = decltype(m)::value;
         if constexpr (sizeof(R) == 4) {
             if (pair) {
-                launch(point_force_kernel<R, QW, true>);
+                launch(long_walks(P) ? point_force_kernel<R, QW, true, true> : point_force_kernel<R, QW, true, false>);
                 return;
             }
         }
@@ -90,19 +99,32 @@ cudaError_t point_force(const SimParams& P, bool pair, const void* qn, const voi
 }
 
 template <class R, class S, bool DEV>
-cudaError_t lbm_aa_point(const SimParams& P, bool pair, bool odd, bool last, void* f, const void* qn,
+cudaError_t lbm_aa_point(const SimParams& P, bool pair, int num_sms, bool odd, bool last, void* f, const void* qn,
                          const void* stress, void* F, void* rho, void* u, cudaStream_t st) {
     const FastDiv dnx = make_fastdiv((uint32_t)P.nx), dnxy = make_fastdiv((uint32_t)P.nxy);
     const unsigned nb = (unsigned)((P.V + kPointThreads - 1) / kPointThreads);
+    const int zm = point_walk(P, pair, num_sms) - 1;
     cudaError_t err = cudaErrorInvalidValue;
     auto launch = [&](auto k) {
-        err = launch_dependent(k, dim3(nb), kPointThreads, 0, st, P, dnx, dnxy, (S*)f, (const R*)qn, (const R*)stress,
-                               (R*)F, (R*)rho, (R*)u, last ? 1 : 0);
+        err = launch_dependent(k, dim3(nb), kPointThreads, 0, st, P, dnx, dnxy, zm, (S*)f, (const R*)qn,
+                               (const R*)stress, (R*)F, (R*)rho, (R*)u, last ? 1 : 0);
     };
     with_mask(point_mask(P), [&](auto m) {
         constexpr int QW = decltype(m)::value, WM = QW & 7;
         if constexpr (sizeof(R) == 4) {
             if (pair) {
+                if (long_walks(P)) {
+                    if constexpr (std::is_same<S, __half>::value && QW == 0) {
+                        // two cells per thread (the packed kernels' boxes have an even nx)
+                        err = launch_dependent(odd ? lbm_aa_point_h2_kernel<DEV, true> : lbm_aa_point_h2_kernel<DEV, false>,
+                                               dim3((unsigned)((P.V / 2 + 255) / 256)), 256, 0, st, P, dnx, dnxy, zm,
+                                               (S*)f, (const R*)stress, (R*)F, (R*)rho, (R*)u, last ? 1 : 0);
+                    } else {
+                        if (odd) launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, true, true, true>);
+                        else launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, false, true, true>);
+                    }
+                    return;
+                }
                 if (odd) launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, true, true>);
                 else launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, false, true>);
                 return;
@@ -123,16 +145,16 @@ cudaError_t lbm_aa_point(const SimParams& P, bool pair, bool odd, bool last, voi
                                     void* qout, void* stress, void* F, cudaStream_t st) {                         \
         return impl::qpoint<R>(P, pair, num_sms, qin, uin, qout, stress, F, st);                                  \
     }                                                                                                             \
-    cudaError_t launch_point_force_##SUF(const SimParams& P, bool pair, const void* qn, const void* stress,       \
-                                         const void* u, void* F, cudaStream_t st) {                               \
-        return impl::point_force<R>(P, pair, qn, stress, u, F, st);                                               \
+    cudaError_t launch_point_force_##SUF(const SimParams& P, bool pair, int num_sms, const void* qn,              \
+                                         const void* stress, const void* u, void* F, cudaStream_t st) {           \
+        return impl::point_force<R>(P, pair, num_sms, qn, stress, u, F, st);                                      \
     }                                                                                                             \
     }
 #define LBMAN_DEFINE_POINT_LBM(SUF, R, S, DEV)                                                                    \
     namespace lbman {                                                                                             \
-    cudaError_t launch_lbm_aa_point_##SUF(const SimParams& P, bool pair, bool odd, bool last, void* f,            \
-                                          const void* qn, const void* stress, void* F, void* rho, void* u,        \
-                                          cudaStream_t st) {                                                      \
-        return impl::lbm_aa_point<R, S, DEV>(P, pair, odd, last, f, qn, stress, F, rho, u, st);                   \
+    cudaError_t launch_lbm_aa_point_##SUF(const SimParams& P, bool pair, int num_sms, bool odd, bool last,        \
+                                          void* f, const void* qn, const void* stress, void* F, void* rho,        \
+                                          void* u, cudaStream_t st) {                                             \
+        return impl::lbm_aa_point<R, S, DEV>(P, pair, num_sms, odd, last, f, qn, stress, F, rho, u, st);          \
     }                                                                                                             \
     }

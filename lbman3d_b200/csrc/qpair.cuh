@@ -19,9 +19,10 @@
 //     the 16-byte boundary at or below x0 - 2 and is 36 columns wide;
 //   * the z derivative of the row stress reads only the thread's own column,
 //     so its three planes live in registers, not shared memory, and the
-//     force of plane zc is accumulated before plane zc + 1 is updated (all
-//     but the +z term), which ends the life of that plane's Q_new, u and
-//     Ericksen force before the next update starts;
+//     force of plane zc is accumulated before plane zc + 1 is updated (all but
+//     the +z term; on planes with long walks also without x and y), which ends
+//     the life of that plane's Q_new, u and Ericksen force before the next
+//     update starts;
 //   * where shared memory allows it without losing a block per SM, the
 //     staging ring holds five planes and each copy gets two planes of lead.
 // Wall rules are applied to each half separately (they are per-point
@@ -355,6 +356,137 @@ __device__ __forceinline__ void qp_partial_force(const SimParams& P, const Phys<
     for (int a = 0; a < 3; ++a) part[a] = fma2(nMU, cur.u[a], f[a]) - cur.ern[a];
 }
 
+// ---- the order of the packed force --------------------------------------------
+// Both orders sum the same terms.  Planes of 2^15 cells and more are stepped with
+// long z walks (qpoint.cuh), which can finish the z terms; there
+//   W = Ericksen - MU u, plus the corrections of anchoring walls (the Q_new ghost
+//       differs from the clamp)                        -- the cell's own values
+//   g = W - Pi_z(z-1) / 2 + Pi_z(z+1) / 2              -- its z column
+//   F = g + ((Pi_x(x+1) - Pi_x(x-1)) + (Pi_y(y+1) - Pi_y(y-1))) / 2
+// A step in this order and in that of qp_partial_force: 256^3 FP32 841 / 870 us,
+// FP16 703 / 775 us; 512x512x256 3378 / 3630 and 2866 / 3248 us; but 128^3 131 /
+// 126 us, where a walk has few planes.  The rule is on the plane, not on the
+// box, so that the z slabs of a box sum as the whole box does.
+__host__ __device__ __forceinline__ bool long_walks(const SimParams& P) { return P.nxy >= 1 << 15; }
+
+// Anchoring corrections of W (sign: -1 where W is kept negated).
+template <class R>
+__device__ __forceinline__ void anchor_force_x(const Phys<R>& K, const AxisRule& r, const R q[5], R sign, R w[3]) {
+    if (!(r.m_ghost || r.p_ghost)) return;
+    const R A = -sign * K.ALPHA;
+    w[0] = __fmaf_rn(A, anchor_delta<R>(r, K, 0, q[0]), w[0]);
+    w[1] = __fmaf_rn(A, anchor_delta<R>(r, K, 1, q[1]), w[1]);
+    w[2] = __fmaf_rn(A, anchor_delta<R>(r, K, 2, q[2]), w[2]);
+}
+template <class R>
+__device__ __forceinline__ void anchor_force_y(const Phys<R>& K, const AxisRule& r, const R q[5], R sign, R w[3]) {
+    if (!(r.m_ghost || r.p_ghost)) return;
+    const R A = -sign * K.ALPHA;
+    w[0] = __fmaf_rn(A, anchor_delta<R>(r, K, 1, q[1]), w[0]);
+    w[1] = __fmaf_rn(A, anchor_delta<R>(r, K, 3, q[3]), w[1]);
+    w[2] = __fmaf_rn(A, anchor_delta<R>(r, K, 4, q[4]), w[2]);
+}
+template <class R>
+__device__ __forceinline__ void anchor_force_z(const Phys<R>& K, const AxisRule& r, const R q[5], R sign, R w[3]) {
+    if (!(r.m_ghost || r.p_ghost)) return;
+    const R A = -sign * K.ALPHA;
+    w[0] = __fmaf_rn(A, anchor_delta<R>(r, K, 2, q[2]), w[0]);
+    w[1] = __fmaf_rn(A, anchor_delta<R>(r, K, 4, q[4]), w[1]);
+    w[2] = __fmaf_rn(-A, anchor_delta<R>(r, K, 0, q[0]) + anchor_delta<R>(r, K, 3, q[3]), w[2]);
+}
+template <class R>
+__device__ __forceinline__ R force_z(R w, R zm, R zp) {
+    return __fmaf_rn(R(0.5), zp, __fmaf_rn(R(-0.5), zm, w));
+}
+template <class R>
+__device__ __forceinline__ R force_xy(R g, R xm, R xp, R ym, R yp) {
+    return __fmaf_rn(R(0.5), __fadd_rn(__fsub_rn(xp, xm), __fsub_rn(yp, ym)), g);
+}
+
+// Corrections of anchoring walls to the negated W of both points.
+__device__ __forceinline__ void qp_anchor_force(const Phys<float>& K, bool rx, bool ry, bool rz, const AxisRule& qx0,
+                                                const AxisRule& qx1, const AxisRule& qy, const AxisRule& qz,
+                                                const F2 qn[5], F2 wn[3]) {
+    const float q0[5] = {qn[0].v.x, qn[1].v.x, qn[2].v.x, qn[3].v.x, qn[4].v.x};
+    const float q1[5] = {qn[0].v.y, qn[1].v.y, qn[2].v.y, qn[3].v.y, qn[4].v.y};
+    float w0[3] = {wn[0].v.x, wn[1].v.x, wn[2].v.x}, w1[3] = {wn[0].v.y, wn[1].v.y, wn[2].v.y};
+    if (rx) {
+        anchor_force_x<float>(K, qx0, q0, -1.0f, w0);
+        anchor_force_x<float>(K, qx1, q1, -1.0f, w1);
+    }
+    if (ry) {
+        anchor_force_y<float>(K, qy, q0, -1.0f, w0);
+        anchor_force_y<float>(K, qy, q1, -1.0f, w1);
+    }
+    if (rz) {
+        anchor_force_z<float>(K, qz, q0, -1.0f, w0);
+        anchor_force_z<float>(K, qz, q1, -1.0f, w1);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) wn[a] = f2(w0[a], w1[a]);
+}
+
+// Force of the pair's tile cells in plane zc in the order above, with the sign of
+// W and g turned (ern holds the Ericksen force negated).  First W and the -z neighbour, from registers alone: cur is
+// plane zc at the points, zm_pz the z-differenced row stress of plane zc - 1.
+template <int RM>
+__device__ __forceinline__ void qp_force_own(const SimParams& P, const Phys<float>& K, const PairGeo& G,
+                                             const PairRules& R, int zc, const PairPlane& cur, const F2 zm_pz[3],
+                                             F2 wn[3]) {
+    const bool rx = RM == 1 || (RM == 2 && G.wx), ry = RM == 2 && G.wy, rz = RM == 2 && G.wz;
+    const F2 MU = f2(K.MU);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) wn[a] = fma2(MU, cur.u[a], cur.ern[a]);
+    AxisRule qz;
+    if (rz) qz = q_rule(P, 2, zc, P.nz);
+    if (rx || ry || rz) qp_anchor_force(K, rx, ry, rz, R.qx0, R.qx1, R.qy, qz, cur.qn, wn);
+    const bool zmc = rz && zc == 0 && !P.qper[4];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) wn[a] = fma2(f2(0.5f), zmc ? cur.pz[a] : zm_pz[a], wn[a]);
+}
+
+// Then, once plane zc + 1 is known, the +z neighbour zp and the x and y
+// differences from plane zc's result slot (not written again before the next
+// barrier but one).
+template <class TL, int RM>
+__device__ __forceinline__ void qp_force_rest(const SimParams& P, const PairGeo& G, int x0, int y0, int z0, int zc,
+                                              const float* Bs, const F2 own_pz[3], const F2 next_pz[3],
+                                              F2 w[3]) {
+    const bool rx = RM == 1 || (RM == 2 && G.wx), ry = RM == 2 && G.wy, rz = RM == 2 && G.wz;
+    constexpr int NB = TL::NB, BXP = TL::BXP;
+    const int p0 = G.p0, p1 = G.p1;
+    const float* Bxy = Bs + ((zc - z0) & 1) * 6 * NB;
+    const int gy = y0 + G.lby - 1;
+    // Sigma / tau differences with the Neumann/periodic index clamp QXoff
+    // (src/offsets.h:59-83, used by PassiveStressDivergence)
+    const bool zpc = rz && zc == P.nz - 1 && !P.qper[5];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float* px = Bxy + a * NB;
+        const float* py = Bxy + (3 + a) * NB;
+        F2 xm = ld2(px, p0 - 1, p1 - 1), xp = ld2(px, p0 + 1, p1 + 1);
+        F2 ym = ld2(py, p0 - BXP, p1 - BXP), yp = ld2(py, p0 + BXP, p1 + BXP);
+        if (rx) {
+            const int gx0 = x0 + G.lbx0 - 1, gx1 = x0 + G.lbx1 - 1;
+            const float c0 = px[p0], c1 = px[p1];
+            float xm0 = xm.v.x, xm1 = xm.v.y, xp0 = xp.v.x, xp1 = xp.v.y;
+            if (gx0 == 0 && !P.qper[0]) xm0 = c0;
+            if (gx1 == 0 && !P.qper[0]) xm1 = c1;
+            if (gx0 == P.nx - 1 && !P.qper[1]) xp0 = c0;
+            if (gx1 == P.nx - 1 && !P.qper[1]) xp1 = c1;
+            xm = f2(xm0, xm1);
+            xp = f2(xp0, xp1);
+        }
+        if (ry) {
+            const F2 c = ld2(py, p0, p1);
+            if (gy == 0 && !P.qper[2]) ym = c;
+            if (gy == P.ny - 1 && !P.qper[3]) yp = c;
+        }
+        const F2 gn = fma2(f2(-0.5f), zpc ? own_pz[a] : next_pz[a], w[a]);
+        w[a] = ((xp - xm) + (yp - ym)) * f2(0.5f) - gn;  // the product is exact: the fma of force_xy
+    }
+}
+
 // Marches a block through planes [z0, z1) of the column at (x0, y0).
 template <class TL, bool UPWIND, class OutQ, class OutF>
 __device__ __forceinline__ void qp_march(const SimParams& P, int x0, int y0, int z0, int z1,
@@ -377,6 +509,7 @@ __device__ __forceinline__ void qp_march(const SimParams& P, int x0, int y0, int
     PairSrc<TL> ps;
     pair_src_init<TL>(P, s0, y0, qin, uin, ps);
     const int rm = (G.wx || G.wy || G.wz) ? ((G.wy || G.wz) ? 2 : 1) : 0;
+    const bool walks = long_walks(P);
     // (a macro, not a lambda: a lambda taking the plane structs by reference
     // put them in local memory)
 #define LBMAN_QP_COMPUTE(zb, pl)                                                              \
@@ -417,15 +550,20 @@ __device__ __forceinline__ void qp_march(const SimParams& P, int x0, int y0, int
     for (int zc = z0; zc < z1; ++zc) {
         if (zc + LEAD + 2 <= z1 + 1) pair_load_plane<TL>(P, z0, zc + LEAD + 2, QU, ps);
         cp_async_commit();
-        // Force of plane zc without its +z term: reads the x/y row stress of
-        // plane zc (complete since the last barrier) and registers.  Only
-        // pairs holding a tile cell: their neighbours' result indices lie
-        // inside the result planes (a pair of a halo row has none).
+        // Force of plane zc as far as known (without its +z term, or from
+        // registers alone), which ends the life of that plane's u and
+        // Ericksen force.  Only pairs holding a tile
+        // cell: their neighbours' result indices lie inside the result planes
+        // (a pair of a halo row has none).
         const bool cell = G.isC0 || G.isC1;
         F2 part[3];
         bool zp_clamped = false;
         if (cell) {
-            if (rm == 0) qp_partial_force<TL, 0>(P, K, G, R, x0, y0, z0, zc, Bs, cur, zm_pz, part, zp_clamped);
+            if (walks) {
+                if (rm == 0) qp_force_own<0>(P, K, G, R, zc, cur, zm_pz, part);
+                else if (rm == 1) qp_force_own<1>(P, K, G, R, zc, cur, zm_pz, part);
+                else qp_force_own<2>(P, K, G, R, zc, cur, zm_pz, part);
+            } else if (rm == 0) qp_partial_force<TL, 0>(P, K, G, R, x0, y0, z0, zc, Bs, cur, zm_pz, part, zp_clamped);
             else if (rm == 1) qp_partial_force<TL, 1>(P, K, G, R, x0, y0, z0, zc, Bs, cur, zm_pz, part, zp_clamped);
             else qp_partial_force<TL, 2>(P, K, G, R, x0, y0, z0, zc, Bs, cur, zm_pz, part, zp_clamped);
         }
@@ -438,7 +576,11 @@ __device__ __forceinline__ void qp_march(const SimParams& P, int x0, int y0, int
         // needed, nobody reads that slot before the next one.
         LBMAN_QP_COMPUTE(zc + 1, cur);
         if (cell) {
-            if (!zp_clamped) {
+            if (walks) {
+                if (rm == 0) qp_force_rest<TL, 0>(P, G, x0, y0, z0, zc, Bs, zm_pz, cur.pz, part);
+                else if (rm == 1) qp_force_rest<TL, 1>(P, G, x0, y0, z0, zc, Bs, zm_pz, cur.pz, part);
+                else qp_force_rest<TL, 2>(P, G, x0, y0, z0, zc, Bs, zm_pz, cur.pz, part);
+            } else if (!zp_clamped) {
 #pragma unroll
                 for (int a = 0; a < 3; ++a) part[a] = fma2(f2(0.5f), cur.pz[a], part[a]);
             }

@@ -7,30 +7,38 @@
 //   qpoint_kernel        the Beris-Edwards update of a cell: Q_new, the stress
 //                        (FP64: Sigma and tau; FP32: the row stress Pi of
 //                        qforce.cuh, grouped by the axis it is differentiated
-//                        along) and the Ericksen force, to global memory;
-//   point_force_kernel   the stress divergence, the active term and -MU u added
-//                        to the Ericksen force (the Q stage alone);
+//                        along) and the Ericksen force (in F), to global memory;
+//   point_force_kernel   the rest of the force added to F (the Q stage alone);
 //   lbm_aa_point_kernel  the same force formed in registers by the in-place
 //                        collide-and-stream, so it never goes to memory.
 //
-// The arithmetic is that of qf_compute_plane / qf_force_cell, value for value
-// (what those keep in shared memory is what qpoint_kernel stores), so both
-// organisations give the same bits.
+// The arithmetic is that of the z-marching kernels, value for value (what those
+// keep in shared memory is what qpoint_kernel stores), so both organisations
+// give the same bits.
 //
-// A thread of qpoint_kernel walks zc planes of one (x, y) column and keeps the
-// centre values of three planes in registers, so a plane costs its x and y
-// neighbours (first-level cache) and one new centre value per field.  No point
-// is updated twice and no warp waits for another; the price is the stress's
-// trip through the second-level cache, or HBM for large boxes.
+// A thread of qpoint_kernel walks a chunk of planes of one (x, y) column and
+// keeps the centre values of three planes in registers, so a plane costs its x
+// and y neighbours (first-level cache) and one new centre value per field,
+// asked into the second-level cache two planes ahead (FP32).  No point is
+// updated twice and no warp waits for another; the price is the stress's trip
+// through the second-level cache, or HBM for large boxes.  The packed kernels
+// (qpoint2_kernel) on planes with long walks (long_walks, qpair.cuh) finish the z
+// terms of the force in the walk, for all but a chunk's first and last plane:
+// per cell 6 stress words and 3 of force go to the LBM kernel instead of 9
+// stress words, 3 of Ericksen force and the 3 of the old velocity.
 //
 // What bounds it: launches below about 10^5 cells, registers and latency up to
-// a few 10^6 (12-20 warps per SM), then HBM (FP32 100 B per cell in the update,
-// 315 us for 256^3 packed against a 260 us floor) and, in FP64, the FP64 pipe.
-// Whole steps before (z-marching Q kernel, then LBM) and with these kernels:
-//   32^3 FP64             67 ->  12 us     20x100x100 FP64    150 -> 29 us
-//   67x101x131 FP32      161 ->  66 us     same, FP64         325 -> 127 us
-//   64x256x256 slit FP32 280 -> 248 us     same, FP64         898 -> 515 us
-//   256^3 FP64          2865 -> 2100 us
+// a few 10^6 (12-20 warps per SM), then HBM: packed on long walks 94 B per cell in
+// the update (256^3: 298 us against a 244 us floor; 330 us without the prefetch,
+// 318 us with 4-plane walks) and 174 B in the LBM step (449 / 490 us even / odd
+// against 440 us; FP16 storage 114 B, 323 / 379 us against 290 us), and, in
+// FP64, the FP64 pipe.  Whole steps before (z-marching Q kernel, then LBM) and
+// with these kernels:
+//   32^3 FP64             67 ->  8 us      20x100x100 FP64    150 -> 26 us
+//   67x101x131 FP32      161 ->  64 us     64^3 FP32           39 -> 17 us
+//   64x256x256 slit FP32 282 -> 243 us     same, FP64         898 -> 515 us
+//   256^3 slit FP32      981 -> 834 us     256^3 FP64        2865 -> 2100 us
+//   256^3 FP32 / FP16    944 -> 803, 844 -> 664 us
 #pragma once
 
 #include "lbm.cuh"
@@ -183,6 +191,14 @@ __device__ __forceinline__ void point_update(const SimParams& P, const Phys<R>& 
         pointwise_q<R, UPWIND>(K, qc, uc[0], uc[1], uc[2], d, g, qn, sg, ta, er);
 }
 
+// Is plane z the first or last of a chunk (zm = planes per chunk - 1, a power of
+// two minus 1)?  A long walk has both z neighbours of its inner planes and
+// finishes g there; for these planes the force's reader adds them from the
+// stored stress.
+__device__ __forceinline__ bool chunk_edge(int z, int zm, int nz) {
+    return (z & zm) == 0 || (z & zm) == zm || z == nz - 1;
+}
+
 // Stores of one updated cell.
 template <class R>
 __device__ __forceinline__ void point_store(const Phys<R>& K, int V, int c, const R qn[5], const R sg[5], const R ta[3],
@@ -212,6 +228,21 @@ __device__ __forceinline__ void point_store(const Phys<R>& K, int V, int c, cons
     for (int k = 0; k < 3; ++k) F[k * V + c] = er[k];
 }
 
+// The warp's cells of plane z + 2 -- WC consecutive cells of Q (5) and u (3) --
+// are asked into the second-level cache two planes ahead, one 128-byte line
+// per lane: the walk's only loads that miss it.
+template <int WC, class R>
+__device__ __forceinline__ const R* walk_prefetch_base(const R* q, const R* u, int V, int col, int n) {
+    constexpr int LPF = WC / 32;  // lines per field
+    const int lane = threadIdx.x & 31, k = lane / LPF;
+    const int at = min(__shfl_sync(0xffffffffu, col, 0) + 32 * (lane % LPF), n - 1);
+    return k < 5 ? q + ((int64_t)k * V + at) : k < 8 ? u + ((int64_t)(k - 5) * V + at) : nullptr;
+}
+template <class R>
+__device__ __forceinline__ void walk_prefetch(const R* base, int64_t off) {
+    if (base) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + off));
+}
+
 // Column `col` (index within the plane) of planes [z0, z1).
 template <class R, bool UPWIND, int QW>
 __device__ __forceinline__ void qpoint_column(const SimParams& P, int x, int y, int col, int z0, int z1, bool live,
@@ -229,6 +260,7 @@ __device__ __forceinline__ void qpoint_column(const SimParams& P, int x, int y, 
         r.qx = q_rule(P, 0, x, P.nx);
         r.qy = q_rule(P, 1, y, P.ny);
     }
+    [[maybe_unused]] const R* const pf = walk_prefetch_base<32>(qin, uin, V, col, nxy);
     R qm[5], qc[5], qp[5], um[2], uc[3], up[3];
     {
         const int m = (z0 == 0 ? nz - 1 : z0 - 1) * nxy + col, c = z0 * nxy + col;
@@ -250,6 +282,8 @@ __device__ __forceinline__ void qpoint_column(const SimParams& P, int x, int y, 
         for (int k = 0; k < 5; ++k) qp[k] = qin[k * V + p];
 #pragma unroll
         for (int k = 0; k < 3; ++k) up[k] = uin[k * V + p];
+        if constexpr (sizeof(R) == 4)
+            if (z + 1 < z1 && z + 2 < nz) walk_prefetch(pf, (int64_t)(z + 2) * nxy);
         R qn[5], sg[5], ta[3], er[3];
         point_update<R, UPWIND, QW>(P, K, r, z, qin, uin, c, qm, qc, qp, um, uc, up, qn, sg, ta, er);
         if (live) point_store<R>(K, V, c, qn, sg, ta, er, qout, stress, F);
@@ -267,10 +301,10 @@ __device__ __forceinline__ void qpoint_column(const SimParams& P, int x, int y, 
 }
 
 // Blocks of 128 threads per SM the registers are held to.  Measured on B200
-// (update kernel alone): FP32, 256^3: 3 / 4 / 5 / 6 blocks 449 / 455 / 404 / 410 us;
-// FP64: 2 / 3 / 4 blocks 1030 / 797 / 787 us at 256^3, 246 / 197 / 351 us on the
-// 64x256x256 slit; packed FP32: 2 / 3 / 4 blocks 324 / 315 / 315 us at 256^3 (four
-// spill).
+// (update kernel alone, with 4-plane walks where not said): FP32, 256^3: 3 / 4 /
+// 5 / 6 blocks 449 / 455 / 404 / 410 us; FP64: 2 / 3 / 4 blocks 1030 / 797 /
+// 787 us at 256^3, 246 / 197 / 351 us on the 64x256x256 slit; packed FP32,
+// 16-plane walks, 256^3: 2 / 3 / 4 blocks 352 / 298 / 319 us (four spill).
 template <class R>
 constexpr int point_min_blocks() {
     return sizeof(R) == 4 ? 5 : 3;
@@ -296,7 +330,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<R>())
 // The point update in the packed arithmetic of qpair.cuh (its values, bit for
 // bit): a thread updates the cells x, x + 1 (x even; nx a multiple of 4), so
 // every field moves as one 8-byte access except the two x neighbours outside
-// the pair.  F holds the negated Ericksen force.
+// the pair.  F holds g (or W) negated.
 __device__ __forceinline__ F2 ldg2(const float* p) { return {__ldg(reinterpret_cast<const float2*>(p))}; }
 __device__ __forceinline__ void stg2(float* p, F2 v) { *reinterpret_cast<float2*>(p) = v.v; }
 
@@ -305,7 +339,7 @@ struct PairRulesX {
     Nbr o;                // y offsets (from x)
 };
 
-template <bool UPWIND, int QW>
+template <bool UPWIND, int QW, bool WALKS>
 __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y, int col, int z0, int z1, bool live,
                                                const float* __restrict__ qin, const float* __restrict__ uin,
                                                float* __restrict__ qout, float* __restrict__ stress,
@@ -330,6 +364,10 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
         qy = q_rule(P, 1, y, P.ny);
     }
     F2 qm[5], qc[5], um[2], uc[3];
+    const float* const pf = walk_prefetch_base<64>(qin, uin, V, col, nxy);
+    F2 wz[3], pzm[3];  // negated W - Pi_z(z-1)/2 of the plane before, its Pi_z
+#pragma unroll
+    for (int k = 0; k < 3; ++k) wz[k] = pzm[k] = f2(0.0f);
     {
         const int m = (z0 == 0 ? nz - 1 : z0 - 1) * nxy + col, c = z0 * nxy + col;
 #pragma unroll
@@ -347,6 +385,7 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
     for (int z = z0; z < z1; ++z) {
         const int c = z * nxy + col, p = (z == nz - 1 ? 0 : z + 1) * nxy + col;
         const bool zw = (QW & QW_Z) && (z == 0 || z == nz - 1);
+        if (z + 1 < z1 && z + 2 < nz) walk_prefetch(pf, (int64_t)(z + 2) * nxy);
         AxisRule qz;
         VWall vz;
         if (zw) {
@@ -415,17 +454,38 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
         g.ux_x = gr[0]; g.ux_y = gr[1]; g.ux_z = gr[2];
         g.uy_x = gr[3]; g.uy_y = gr[4]; g.uy_z = gr[5];
         g.uz_x = gr[6]; g.uz_y = gr[7];
-        F2 qn[5], pxy[6], pz[3], ern[3];
-        pointwise_q_pair<UPWIND>(K, qc, uc[0], uc[1], uc[2], d, g, qn, pxy, pz, ern);
+        F2 qn[5], pxy[6], pz[3], wn[3];
+        pointwise_q_pair<UPWIND>(K, qc, uc[0], uc[1], uc[2], d, g, qn, pxy, pz, wn);
+        if (WALKS) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) wn[k] = fma2(f2(K.MU), uc[k], wn[k]);
+            if constexpr (QW & QW_ANCHOR) {
+                AxisRule qzr = q_rule(P, 2, z, nz);
+                qp_anchor_force(K, true, true, z == 0 || z == nz - 1, qx0, qx1, qy, qzr, qn, wn);
+            }
+        }
         if (live) {
 #pragma unroll
             for (int k = 0; k < 5; ++k) stg2(qout + (k * V + c), qn[k]);
 #pragma unroll
             for (int k = 0; k < 6; ++k) stg2(stress + (k * V + c), pxy[k]);
+            if (!WALKS || z <= z0 + 1 || z >= z1 - 2) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) stg2(stress + ((6 + k) * V + c), pz[k]);
+                for (int k = 0; k < 3; ++k) stg2(stress + ((6 + k) * V + c), pz[k]);
+            }
+            if (WALKS && z > z0 + 1) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) stg2(F + (k * V + c), ern[k]);
+                for (int k = 0; k < 3; ++k) stg2(F + (k * V + c - nxy), fma2(f2(-0.5f), pz[k], wz[k]));
+            }
+            if (!WALKS || z == z0 || z == z1 - 1) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) stg2(F + (k * V + c), wn[k]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            wz[k] = fma2(f2(0.5f), pzm[k], wn[k]);
+            pzm[k] = pz[k];
         }
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
@@ -441,7 +501,7 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
 }
 
 // Block (bx, bz): cells [256 bx, 256 bx + 256) of each plane of z chunk bz.
-template <bool UPWIND, int QW>
+template <bool UPWIND, int QW, bool WALKS>
 __global__ void __launch_bounds__(kPointThreads, kPairPointMinBlocks)
     qpoint2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, int zc, const float* __restrict__ qin,
                    const float* __restrict__ uin, float* __restrict__ qout, float* __restrict__ stress,
@@ -453,18 +513,21 @@ __global__ void __launch_bounds__(kPointThreads, kPairPointMinBlocks)
     const int y = (int)fdiv((uint32_t)col, dnx), x = col - y * P.nx;
     const int z0 = (int)blockIdx.y * zc;
     pdl_begin();
-    qpoint2_column<UPWIND, QW>(P, x, y, col, z0, min(z0 + zc, P.nz), live, qin, uin, qout, stress, F);
+    qpoint2_column<UPWIND, QW, WALKS>(P, x, y, col, z0, min(z0 + zc, P.nz), live, qin, uin, qout, stress, F);
 }
 
 // ---- body force from the stored stress -----------------------------------------
 // Force source of aa_even_cell / aa_odd_cell: the Ericksen force in F plus the
 // stress divergence, the active term and -MU u.  u is read before the LBM
 // step overwrites it (own cell only); stress and Q are not written by it.
-// PAIR: the packed kernels' order of operations (qp_partial_force).
-template <class R, int QW, bool PAIR = false>
+// PAIR: the packed kernels' order of operations (qp_partial_force); WALKS: that of
+// planes with long walks, where F holds g negated, or W in the planes next to a
+// chunk boundary (zm), and only the x and y differences remain.
+template <class R, int QW, bool PAIR = false, bool WALKS = false>
 struct PointForce {
     static constexpr bool kNeedsPos = true;
     const SimParams& P;
+    int zm;
     const R* __restrict__ qn;
     const R* __restrict__ stress;
     const R* u;
@@ -474,6 +537,28 @@ struct PointForce {
         const int V = (int)P.V;
         const Nbr w = wrapped_nbr(P, q.x, q.y, q.z);
         const Nbr s = stress_nbr<QW>(P, q.x, q.y, q.z, w);
+        if constexpr (WALKS) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) out[a] = -F[a * V + c];
+            R xy[3][4];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const R* px = stress + (a * V + c);
+                const R* py = stress + ((3 + a) * V + c);
+                xy[a][0] = px[s.xm]; xy[a][1] = px[s.xp];
+                xy[a][2] = py[s.ym]; xy[a][3] = py[s.yp];
+            }
+            if (chunk_edge(q.z, zm, P.nz)) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const R* pz = stress + ((6 + a) * V + c);
+                    out[a] = force_z<R>(out[a], pz[s.zm], pz[s.zp]);
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < 3; ++a) out[a] = force_xy<R>(out[a], xy[a][0], xy[a][1], xy[a][2], xy[a][3]);
+            return;
+        }
         const R u0[3] = {u[c], u[V + c], u[2 * V + c]};
         const R er[3] = {F[c], F[V + c], F[2 * V + c]};
         AxisRule qx, qy, qz;
@@ -582,25 +667,25 @@ struct PointForce {
     }
 };
 
-template <class R, int QW, bool PAIR = false>
+template <class R, int QW, bool PAIR = false, bool WALKS = false>
 __global__ void __launch_bounds__(256)
-    point_force_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, const R* __restrict__ qn,
+    point_force_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, int zm, const R* __restrict__ qn,
                        const R* __restrict__ stress, const R* u, R* F) {
     const int c = (int)(blockIdx.x * 256 + threadIdx.x);
     pdl_begin();
     if (c >= (int)P.V) return;
     const int V = (int)P.V;
     R out[3];
-    PointForce<R, QW, PAIR>{P, qn, stress, u, F}(c, cell_pos<int>(P, c, dnx, dnxy), out);
+    PointForce<R, QW, PAIR, WALKS>{P, zm, qn, stress, u, F}(c, cell_pos<int>(P, c, dnx, dnxy), out);
 #pragma unroll
     for (int k = 0; k < 3; ++k) F[k * V + c] = out[k];
 }
 
 // PointForce, also stored to F when last (the body force a caller may download).
-template <class R, int QW, bool PAIR>
+template <class R, int QW, bool PAIR, bool WALKS = false>
 struct KeptPointForce {
     static constexpr bool kNeedsPos = true;
-    PointForce<R, QW, PAIR> pf;
+    PointForce<R, QW, PAIR, WALKS> pf;
     R* F;
     int last;
     __device__ __forceinline__ void operator()(int c, const CellPos& q, R out[3]) const {
@@ -613,18 +698,96 @@ struct KeptPointForce {
     }
 };
 
+// The packed force of the cells c, c + 1 (c even) of a box without walls, for
+// aa_even_h2 / aa_odd_h2: the pair's own values and y neighbours as 8-byte
+// accesses, the x differences from four consecutive cells.
+struct PairPointForce {
+    const SimParams& P;
+    int zm;
+    const float* __restrict__ stress;
+    float* F;
+    int last;
+    struct Values {
+        float v[2][3];
+        template <int I>
+        __device__ __forceinline__ void get(float f[3]) const {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) f[a] = v[I][a];
+        }
+    };
+    __device__ __forceinline__ Values begin(int c, const CellPos& q) const {
+        const int V = (int)P.V;
+        const Nbr w = wrapped_nbr(P, q.x, q.y, q.z);
+        const int xr = q.x + 2 == P.nx ? 2 - P.nx : 2;
+        Values o;
+        float2 g[3], px[3], ym[3], yp[3];
+        float l[3], r[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float* sx = stress + (a * V + c);
+            const float* sy = stress + ((3 + a) * V + c);
+            g[a] = *reinterpret_cast<const float2*>(F + (a * V + c));
+            px[a] = __ldg(reinterpret_cast<const float2*>(sx));
+            l[a] = __ldg(sx + w.xm);
+            r[a] = __ldg(sx + xr);
+            ym[a] = __ldg(reinterpret_cast<const float2*>(sy + w.ym));
+            yp[a] = __ldg(reinterpret_cast<const float2*>(sy + w.yp));
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) o.v[0][a] = -g[a].x, o.v[1][a] = -g[a].y;
+        if (chunk_edge(q.z, zm, P.nz)) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float* sz = stress + ((6 + a) * V + c);
+                const float2 m = __ldg(reinterpret_cast<const float2*>(sz + w.zm));
+                const float2 p = __ldg(reinterpret_cast<const float2*>(sz + w.zp));
+                o.v[0][a] = force_z<float>(o.v[0][a], m.x, p.x);
+                o.v[1][a] = force_z<float>(o.v[1][a], m.y, p.y);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            o.v[0][a] = force_xy<float>(o.v[0][a], l[a], px[a].y, ym[a].x, yp[a].x);
+            o.v[1][a] = force_xy<float>(o.v[1][a], px[a].x, r[a], ym[a].y, yp[a].y);
+        }
+        if (last) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                *reinterpret_cast<float2*>(F + (a * V + c)) = make_float2(o.v[0][a], o.v[1][a]);
+        }
+        return o;
+    }
+};
+
 // In-place LBM step with the force formed on the fly.  last: rho and the body
 // force are also written everywhere, as after the last step of a call.
-template <class R, class S, bool DEV, int WM, int QW, bool ODD, bool PAIR = false>
+template <class R, class S, bool DEV, int WM, int QW, bool ODD, bool PAIR = false, bool WALKS = false>
 __global__ void __launch_bounds__(kPointThreads)
-    lbm_aa_point_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, S* f, const R* __restrict__ qn,
-                        const R* __restrict__ stress, R* F, R* __restrict__ rho_buf, R* u, int last) {
+    lbm_aa_point_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, int zm, S* f,
+                        const R* __restrict__ qn, const R* __restrict__ stress, R* F, R* __restrict__ rho_buf, R* u, int last) {
     const int c = (int)(blockIdx.x * kPointThreads + threadIdx.x);
     pdl_begin();
     if (c >= (int)P.V) return;
-    const KeptPointForce<R, QW, PAIR> force{{P, qn, stress, u, F}, F, last};
+    const KeptPointForce<R, QW, PAIR, WALKS> force{{P, zm, qn, stress, u, F}, F, last};
     if constexpr (ODD) aa_odd_cell<R, S, DEV, WM, int>(P, dnx, dnxy, c, f, force, rho_buf, u, last);
     else aa_even_cell<R, S, DEV, WM, int>(P, dnx, dnxy, c, f, force, rho_buf, u, last);
+}
+
+// The same for FP16 storage without walls and an even nx, packed arithmetic:
+// two cells per thread (aa_even_h2, aa_odd_h2), because 2-byte accesses of one
+// cell leave the load-store path, not HBM, as the bound.  256^3, even / odd step:
+// one cell 363 / 401 us, two cells 323 / 379 us.
+template <bool DEV, bool ODD>
+__global__ void __launch_bounds__(256, 3)
+    lbm_aa_point_h2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, int zm, __half* f,
+                           const float* __restrict__ stress, float* F, float* __restrict__ rho_buf, float* u, int last) {
+    const int c = 2 * (int)(blockIdx.x * 256 + threadIdx.x);
+    pdl_begin();
+    if (c >= (int)P.V) return;
+    const PairPointForce force{P, zm, stress, F, last};
+    const CellPos q = cell_pos<int>(P, c, dnx, dnxy);
+    if constexpr (ODD) aa_odd_h2<DEV, int>(P, c, q, f, force, rho_buf, u, last);
+    else aa_even_h2<DEV, int>(P, c, q, f, force, rho_buf, u, last);
 }
 
 }  // namespace lbman

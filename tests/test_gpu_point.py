@@ -2,8 +2,7 @@
 take: value for value the arithmetic of the z-marching kernels, so a box must
 come out bit for bit as with explicitly chosen z-marching kernels, whole steps
 and the Q stage alone, on every wall mask (none, x, x and y, all, anchoring,
-mixed Q tags), on thin and odd boxes, and across the size where the body force
-moves from the LBM kernel to a kernel of its own."""
+mixed Q tags), on thin and odd boxes, and on boxes large enough for long walks."""
 import numpy as np
 import pytest
 
@@ -65,16 +64,27 @@ def test_point_kernels_equal_the_marching_kernels_bitwise(grid, bc, upwind, prec
         s.close()
 
 
-@pytest.mark.parametrize("grid,bc", [((182, 187, 191), "periodic"), ((240, 160, 168), "slit")],
-                         ids=["one_point", "packed"])
-def test_large_box_with_a_separate_force_kernel(grid, bc):
-    """Just above the size up to which the LBM kernel forms the force."""
-    packed = grid[0] == 240
-    a, b = _pair(grid, bc, L.Precision.FP32, False, N.KERNELS_SPLIT_PAIR if packed else N.KERNELS_SPLIT,
-                 (30, 10, 32) if packed else (32, 8, 32))
+# Large boxes, where a thread walks 4 planes (one point per thread) or 16 (packed,
+# planes of 2^15 cells: the z terms of the force are finished in the walk, except
+# at chunk boundaries), with a short last chunk.  FP64 there forms the force in a
+# kernel of its own.
+@pytest.mark.parametrize("grid,bc,precision", [((182, 187, 191), "box_mixed", L.Precision.FP32),
+                                               ((240, 160, 165), "box_mixed", L.Precision.FP32),
+                                               ((256, 240, 167), "periodic", L.Precision.FP32),
+                                               ((256, 240, 167), "periodic", L.Precision.FP16),
+                                               ((240, 160, 5), "slit", L.Precision.FP16),
+                                               ((182, 187, 191), "periodic", L.Precision.FP64)],
+                         ids=["one_point", "packed_mixed", "packed", "packed_fp16", "packed_thin_fp16", "fp64"])
+def test_long_walks(grid, bc, precision):
+    packed = grid[0] % 4 == 0
+    a, b = _pair(grid, bc, precision, False, N.KERNELS_SPLIT_PAIR if packed else N.KERNELS_SPLIT,
+                 (30, 10, 32) if packed else (14, 14, 32) if precision == L.Precision.FP64 else (32, 8, 32))
     for n in (1, 2):
         a.step(n)
         b.step(n)
         _same(a, b, f=False)
+    for s in (a, b):
+        s.qtensor_step()
+    _same(a, b, f=False)
     for s in (a, b):
         s.close()
