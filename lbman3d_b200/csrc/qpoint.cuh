@@ -18,10 +18,10 @@
 //
 // A thread of qpoint_kernel walks a chunk of planes of one (x, y) column and
 // keeps the centre values of three planes in registers, so a plane costs its x
-// and y neighbours (first-level cache) and one new centre value per field,
-// asked into the second-level cache two planes ahead (FP32).  No point is
-// updated twice and no warp waits for another; the price is the stress's trip
-// through the second-level cache, or HBM for large boxes.  The packed kernels
+// and y neighbours (first-level cache) and one new centre value per field.  No
+// point is updated twice and no warp waits for another; the price is the
+// stress's trip through the second-level cache, or HBM for large boxes.  The
+// packed kernels
 // (qpoint2_kernel) on planes with long walks (long_walks, qpair.cuh) finish the z
 // terms of the force in the walk, for all but a chunk's first and last plane:
 // per cell 6 stress words and 3 of force go to the LBM kernel instead of 9
@@ -35,7 +35,7 @@
 // FP64, the FP64 pipe.  Whole steps before (z-marching Q kernel, then LBM) and
 // with these kernels:
 //   32^3 FP64             67 ->  8 us      20x100x100 FP64    150 -> 26 us
-//   67x101x131 FP32      161 ->  64 us     64^3 FP32           39 -> 17 us
+//   67x101x131 FP32      161 ->  61 us     64^3 FP32           39 -> 16 us
 //   64x256x256 slit FP32 282 -> 243 us     same, FP64         898 -> 515 us
 //   256^3 slit FP32      981 -> 834 us     256^3 FP64        2865 -> 2100 us
 //   256^3 FP32 / FP16    944 -> 803, 844 -> 664 us
@@ -228,21 +228,6 @@ __device__ __forceinline__ void point_store(const Phys<R>& K, int V, int c, cons
     for (int k = 0; k < 3; ++k) F[k * V + c] = er[k];
 }
 
-// The warp's cells of plane z + 2 -- WC consecutive cells of Q (5) and u (3) --
-// are asked into the second-level cache two planes ahead, one 128-byte line
-// per lane: the walk's only loads that miss it.
-template <int WC, class R>
-__device__ __forceinline__ const R* walk_prefetch_base(const R* q, const R* u, int V, int col, int n) {
-    constexpr int LPF = WC / 32;  // lines per field
-    const int lane = threadIdx.x & 31, k = lane / LPF;
-    const int at = min(__shfl_sync(0xffffffffu, col, 0) + 32 * (lane % LPF), n - 1);
-    return k < 5 ? q + ((int64_t)k * V + at) : k < 8 ? u + ((int64_t)(k - 5) * V + at) : nullptr;
-}
-template <class R>
-__device__ __forceinline__ void walk_prefetch(const R* base, int64_t off) {
-    if (base) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + off));
-}
-
 // Column `col` (index within the plane) of planes [z0, z1).
 template <class R, bool UPWIND, int QW>
 __device__ __forceinline__ void qpoint_column(const SimParams& P, int x, int y, int col, int z0, int z1, bool live,
@@ -260,7 +245,6 @@ __device__ __forceinline__ void qpoint_column(const SimParams& P, int x, int y, 
         r.qx = q_rule(P, 0, x, P.nx);
         r.qy = q_rule(P, 1, y, P.ny);
     }
-    [[maybe_unused]] const R* const pf = walk_prefetch_base<32>(qin, uin, V, col, nxy);
     R qm[5], qc[5], qp[5], um[2], uc[3], up[3];
     {
         const int m = (z0 == 0 ? nz - 1 : z0 - 1) * nxy + col, c = z0 * nxy + col;
@@ -282,8 +266,6 @@ __device__ __forceinline__ void qpoint_column(const SimParams& P, int x, int y, 
         for (int k = 0; k < 5; ++k) qp[k] = qin[k * V + p];
 #pragma unroll
         for (int k = 0; k < 3; ++k) up[k] = uin[k * V + p];
-        if constexpr (sizeof(R) == 4)
-            if (z + 1 < z1 && z + 2 < nz) walk_prefetch(pf, (int64_t)(z + 2) * nxy);
         R qn[5], sg[5], ta[3], er[3];
         point_update<R, UPWIND, QW>(P, K, r, z, qin, uin, c, qm, qc, qp, um, uc, up, qn, sg, ta, er);
         if (live) point_store<R>(K, V, c, qn, sg, ta, er, qout, stress, F);
@@ -334,6 +316,20 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<R>())
 __device__ __forceinline__ F2 ldg2(const float* p) { return {__ldg(reinterpret_cast<const float2*>(p))}; }
 __device__ __forceinline__ void stg2(float* p, F2 v) { *reinterpret_cast<float2*>(p) = v.v; }
 
+// The warp's 64 cells of plane z + 2 are asked into the second-level cache two
+// planes ahead, one 128-byte line of Q (5 fields) or u (3) per lane: the long
+// walk's only loads that miss it (256^3: 330 -> 298 us).  Short walks and the
+// one-point kernel, with more warps in flight, lose by it (64^3 step 15.9 ->
+// 17.2 us, 96 boxes 1130 -> 1145 us).
+__device__ __forceinline__ const float* walk_prefetch_base(const float* q, const float* u, int V, int col, int n) {
+    const int lane = threadIdx.x & 31, k = lane / 2;
+    const int at = min(__shfl_sync(0xffffffffu, col, 0) + 32 * (lane & 1), n - 1);
+    return k < 5 ? q + ((int64_t)k * V + at) : k < 8 ? u + ((int64_t)(k - 5) * V + at) : nullptr;
+}
+__device__ __forceinline__ void walk_prefetch(const float* base, int64_t off) {
+    if (base) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + off));
+}
+
 struct PairRulesX {
     int xl, xr;           // offsets of the left neighbour of x and the right one of x + 1
     Nbr o;                // y offsets (from x)
@@ -364,7 +360,7 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
         qy = q_rule(P, 1, y, P.ny);
     }
     F2 qm[5], qc[5], um[2], uc[3];
-    const float* const pf = walk_prefetch_base<64>(qin, uin, V, col, nxy);
+    const float* const pf = walk_prefetch_base(qin, uin, V, col, nxy);
     F2 wz[3], pzm[3];  // negated W - Pi_z(z-1)/2 of the plane before, its Pi_z
 #pragma unroll
     for (int k = 0; k < 3; ++k) wz[k] = pzm[k] = f2(0.0f);
@@ -385,7 +381,7 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
     for (int z = z0; z < z1; ++z) {
         const int c = z * nxy + col, p = (z == nz - 1 ? 0 : z + 1) * nxy + col;
         const bool zw = (QW & QW_Z) && (z == 0 || z == nz - 1);
-        if (z + 1 < z1 && z + 2 < nz) walk_prefetch(pf, (int64_t)(z + 2) * nxy);
+        if (WALKS && z + 1 < z1 && z + 2 < nz) walk_prefetch(pf, (int64_t)(z + 2) * nxy);
         AxisRule qz;
         VWall vz;
         if (zw) {
