@@ -135,6 +135,7 @@ void build_sim_params(const lbman_config& c, SimParams& P) {
     P.omega_prime = c.DT / c.TAUF;
     P.omega_forcing = 1.0 - c.DT / 2.0 / c.TAUF;
     P.upwind = c.advection == LBMAN_UPWIND;
+    P.half_pop = c.precision == LBMAN_FP16;
     P.moving_any = 0;
     for (int k = 0; k < 6; ++k) {
         P.face[k].qbc = c.face[k].qbc;

@@ -48,6 +48,7 @@ struct SimParams {
     Face face[6];          // XLo, XHi, YLo, YHi, ZLo, ZHi
     int qper[6], uper[6];  // face tag is Periodic (Q / velocity)
     int moving_any;        // some face is a MovingWall
+    int half_pop;          // populations stored in FP16
     Phys<double> pd;       // the constants above, per compute precision; kernels
     Phys<float> pf;        // read them in place from the parameter space
 };

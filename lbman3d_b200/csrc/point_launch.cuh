@@ -63,9 +63,14 @@ cudaError_t qpoint(const SimParams& P, bool pair, int num_sms, const void* qin, 
         constexpr int QW = decltype(m)::value;
         if constexpr (sizeof(R) == 4) {
             if (pair) {
-                const bool walks = long_walks(P);
-                if (P.upwind) launch(walks ? qpoint2_kernel<true, QW, true> : qpoint2_kernel<true, QW, false>);
-                else launch(walks ? qpoint2_kernel<false, QW, true> : qpoint2_kernel<false, QW, false>);
+                auto go = [&](auto walk) {
+                    constexpr int W = decltype(walk)::value;
+                    if (P.upwind) launch(qpoint2_kernel<true, QW, W>);
+                    else launch(qpoint2_kernel<false, QW, W>);
+                };
+                if (force_in_walk(P)) go(std::integral_constant<int, WALK_FORCE>{});
+                else if (long_walks(P)) go(std::integral_constant<int, WALK_LONG>{});
+                else go(std::integral_constant<int, WALK_SHORT>{});
                 return;
             }
         }
@@ -89,7 +94,7 @@ cudaError_t point_force(const SimParams& P, bool pair, int num_sms, const void* 
         constexpr int QW = decltype(m)::value;
         if constexpr (sizeof(R) == 4) {
             if (pair) {
-                launch(long_walks(P) ? point_force_kernel<R, QW, true, true> : point_force_kernel<R, QW, true, false>);
+                launch(force_in_walk(P) ? point_force_kernel<R, QW, true, true> : point_force_kernel<R, QW, true, false>);
                 return;
             }
         }
@@ -113,17 +118,20 @@ cudaError_t lbm_aa_point(const SimParams& P, bool pair, int num_sms, bool odd, b
         constexpr int QW = decltype(m)::value, WM = QW & 7;
         if constexpr (sizeof(R) == 4) {
             if (pair) {
-                if (long_walks(P)) {
-                    if constexpr (std::is_same<S, __half>::value && QW == 0) {
-                        // two cells per thread (the packed kernels' boxes have an even nx)
-                        err = launch_dependent(odd ? lbm_aa_point_h2_kernel<DEV, true> : lbm_aa_point_h2_kernel<DEV, false>,
-                                               dim3((unsigned)((P.V / 2 + 255) / 256)), 256, 0, st, P, dnx, dnxy, zm,
-                                               (S*)f, (const R*)stress, (R*)F, (R*)rho, (R*)u, last ? 1 : 0);
-                    } else {
+                if constexpr (!std::is_same<S, __half>::value) {
+                    if (force_in_walk(P)) {
                         if (odd) launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, true, true, true>);
                         else launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, false, true, true>);
+                        return;
                     }
-                    return;
+                } else if constexpr (QW == 0) {
+                    if (long_walks(P)) {
+                        // two cells per thread (the packed kernels' boxes have an even nx)
+                        err = launch_dependent(odd ? lbm_aa_point_h2_kernel<DEV, true> : lbm_aa_point_h2_kernel<DEV, false>,
+                                               dim3((unsigned)((P.V / 2 + 255) / 256)), 256, 0, st, P, dnx, dnxy, (S*)f,
+                                               (const R*)stress, (R*)F, (R*)rho, (R*)u, last ? 1 : 0);
+                        return;
+                    }
                 }
                 if (odd) launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, true, true>);
                 else launch(lbm_aa_point_kernel<R, S, DEV, WM, QW, false, true>);

@@ -20,7 +20,7 @@
 //   * the z derivative of the row stress reads only the thread's own column,
 //     so its three planes live in registers, not shared memory, and the
 //     force of plane zc is accumulated before plane zc + 1 is updated (all but
-//     the +z term; on planes with long walks also without x and y), which ends
+//     the +z term; on planes with long walks in FP32 also without x and y), which ends
 //     the life of that plane's Q_new, u and Ericksen force before the next
 //     update starts;
 //   * where shared memory allows it without losing a block per SM, the
@@ -358,16 +358,21 @@ __device__ __forceinline__ void qp_partial_force(const SimParams& P, const Phys<
 
 // ---- the order of the packed force --------------------------------------------
 // Both orders sum the same terms.  Planes of 2^15 cells and more are stepped with
-// long z walks (qpoint.cuh), which can finish the z terms; there
+// long z walks (qpoint.cuh), which can finish the z terms; there, in FP32,
 //   W = Ericksen - MU u, plus the corrections of anchoring walls (the Q_new ghost
 //       differs from the clamp)                        -- the cell's own values
 //   g = W - Pi_z(z-1) / 2 + Pi_z(z+1) / 2              -- its z column
 //   F = g + ((Pi_x(x+1) - Pi_x(x-1)) + (Pi_y(y+1) - Pi_y(y-1))) / 2
-// A step in this order and in that of qp_partial_force: 256^3 FP32 841 / 870 us,
-// FP16 703 / 775 us; 512x512x256 3378 / 3630 and 2866 / 3248 us; but 128^3 131 /
-// 126 us, where a walk has few planes.  The rule is on the plane, not on the
-// box, so that the z slabs of a box sum as the whole box does.
+// A step in this order and in that of qp_partial_force: 256^3 FP32 784 / 846 us,
+// 512x512x256 3162 / 3442 us, 512^3 6423 / 7078 us; on smaller planes a walk
+// has few planes and gains nothing.  Boxes with FP16 populations keep the order
+// of qp_partial_force on every plane: the two orders differ in the force's last
+// bit, which turns roundings of the stored populations, and after 200 steps at
+// 256^3 the fields were 4e-4 apart (a step takes 703 us for the 662 us of the
+// other order).  The rules are on the plane, not on the box, so that the z slabs
+// of a box sum as the whole box does.
 __host__ __device__ __forceinline__ bool long_walks(const SimParams& P) { return P.nxy >= 1 << 15; }
+__host__ __device__ __forceinline__ bool force_in_walk(const SimParams& P) { return long_walks(P) && !P.half_pop; }
 
 // Anchoring corrections of W (sign: -1 where W is kept negated).
 template <class R>
@@ -509,7 +514,7 @@ __device__ __forceinline__ void qp_march(const SimParams& P, int x0, int y0, int
     PairSrc<TL> ps;
     pair_src_init<TL>(P, s0, y0, qin, uin, ps);
     const int rm = (G.wx || G.wy || G.wz) ? ((G.wy || G.wz) ? 2 : 1) : 0;
-    const bool walks = long_walks(P);
+    const bool walks = force_in_walk(P);
     // (a macro, not a lambda: a lambda taking the plane structs by reference
     // put them in local memory)
 #define LBMAN_QP_COMPUTE(zb, pl)                                                              \

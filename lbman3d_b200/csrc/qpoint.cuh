@@ -335,11 +335,16 @@ struct PairRulesX {
     Nbr o;                // y offsets (from x)
 };
 
-template <bool UPWIND, int QW, bool WALKS>
+// What a walk of qpoint2_column does besides the update: nothing, the prefetch, or
+// the prefetch and the z terms of the force (force_in_walk).
+enum : int { WALK_SHORT = 0, WALK_LONG = 1, WALK_FORCE = 2 };
+
+template <bool UPWIND, int QW, int WALK>
 __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y, int col, int z0, int z1, bool live,
                                                const float* __restrict__ qin, const float* __restrict__ uin,
                                                float* __restrict__ qout, float* __restrict__ stress,
                                                float* __restrict__ F) {
+    constexpr bool WALKS = WALK == WALK_FORCE;
     const Phys<float>& K = phys_ref<float>(P);
     const int V = (int)P.V, nxy = (int)P.nxy, nz = P.nz, x1 = x + 1;
     const Nbr w0 = wrapped_nbr(P, x, y, 0), w1 = wrapped_nbr(P, x1, y, 0);
@@ -381,7 +386,7 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
     for (int z = z0; z < z1; ++z) {
         const int c = z * nxy + col, p = (z == nz - 1 ? 0 : z + 1) * nxy + col;
         const bool zw = (QW & QW_Z) && (z == 0 || z == nz - 1);
-        if (WALKS && z + 1 < z1 && z + 2 < nz) walk_prefetch(pf, (int64_t)(z + 2) * nxy);
+        if (WALK != WALK_SHORT && z + 1 < z1 && z + 2 < nz) walk_prefetch(pf, (int64_t)(z + 2) * nxy);
         AxisRule qz;
         VWall vz;
         if (zw) {
@@ -497,7 +502,7 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
 }
 
 // Block (bx, bz): cells [256 bx, 256 bx + 256) of each plane of z chunk bz.
-template <bool UPWIND, int QW, bool WALKS>
+template <bool UPWIND, int QW, int WALK>
 __global__ void __launch_bounds__(kPointThreads, kPairPointMinBlocks)
     qpoint2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, int zc, const float* __restrict__ qin,
                    const float* __restrict__ uin, float* __restrict__ qout, float* __restrict__ stress,
@@ -509,7 +514,7 @@ __global__ void __launch_bounds__(kPointThreads, kPairPointMinBlocks)
     const int y = (int)fdiv((uint32_t)col, dnx), x = col - y * P.nx;
     const int z0 = (int)blockIdx.y * zc;
     pdl_begin();
-    qpoint2_column<UPWIND, QW, WALKS>(P, x, y, col, z0, min(z0 + zc, P.nz), live, qin, uin, qout, stress, F);
+    qpoint2_column<UPWIND, QW, WALK>(P, x, y, col, z0, min(z0 + zc, P.nz), live, qin, uin, qout, stress, F);
 }
 
 // ---- body force from the stored stress -----------------------------------------
@@ -695,12 +700,12 @@ struct KeptPointForce {
 };
 
 // The packed force of the cells c, c + 1 (c even) of a box without walls, for
-// aa_even_h2 / aa_odd_h2: the pair's own values and y neighbours as 8-byte
-// accesses, the x differences from four consecutive cells.
+// aa_even_h2 / aa_odd_h2: the pair's own values and its y and z neighbours as
+// 8-byte accesses, the x differences from four consecutive cells.
 struct PairPointForce {
     const SimParams& P;
-    int zm;
-    const float* __restrict__ stress;
+    const float* stress;
+    const float* u;
     float* F;
     int last;
     struct Values {
@@ -711,40 +716,28 @@ struct PairPointForce {
             for (int a = 0; a < 3; ++a) f[a] = v[I][a];
         }
     };
+    __device__ __forceinline__ static float2 ld(const float* p) { return *reinterpret_cast<const float2*>(p); }
+    __device__ __forceinline__ static float sum(float xm, float xp, float ym, float yp, float zm, float zp, float nmu,
+                                                float u, float er) {
+        const float f = __fmul_rn(__fsub_rn(__fadd_rn(__fsub_rn(xp, xm), __fsub_rn(yp, ym)), zm), 0.5f);
+        return __fmaf_rn(0.5f, zp, __fsub_rn(__fmaf_rn(nmu, u, f), er));
+    }
     __device__ __forceinline__ Values begin(int c, const CellPos& q) const {
         const int V = (int)P.V;
+        const float nmu = -phys_ref<float>(P).MU;
         const Nbr w = wrapped_nbr(P, q.x, q.y, q.z);
         const int xr = q.x + 2 == P.nx ? 2 - P.nx : 2;
         Values o;
-        float2 g[3], px[3], ym[3], yp[3];
-        float l[3], r[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const float* sx = stress + (a * V + c);
             const float* sy = stress + ((3 + a) * V + c);
-            g[a] = *reinterpret_cast<const float2*>(F + (a * V + c));
-            px[a] = __ldg(reinterpret_cast<const float2*>(sx));
-            l[a] = __ldg(sx + w.xm);
-            r[a] = __ldg(sx + xr);
-            ym[a] = __ldg(reinterpret_cast<const float2*>(sy + w.ym));
-            yp[a] = __ldg(reinterpret_cast<const float2*>(sy + w.yp));
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) o.v[0][a] = -g[a].x, o.v[1][a] = -g[a].y;
-        if (chunk_edge(q.z, zm, P.nz)) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float* sz = stress + ((6 + a) * V + c);
-                const float2 m = __ldg(reinterpret_cast<const float2*>(sz + w.zm));
-                const float2 p = __ldg(reinterpret_cast<const float2*>(sz + w.zp));
-                o.v[0][a] = force_z<float>(o.v[0][a], m.x, p.x);
-                o.v[1][a] = force_z<float>(o.v[1][a], m.y, p.y);
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            o.v[0][a] = force_xy<float>(o.v[0][a], l[a], px[a].y, ym[a].x, yp[a].x);
-            o.v[1][a] = force_xy<float>(o.v[1][a], px[a].x, r[a], ym[a].y, yp[a].y);
+            const float* sz = stress + ((6 + a) * V + c);
+            const float2 px = ld(sx), ym = ld(sy + w.ym), yp = ld(sy + w.yp), zm = ld(sz + w.zm), zp = ld(sz + w.zp);
+            const float2 ua = ld(u + (a * V + c)), er = ld(F + (a * V + c));
+            const float l = sx[w.xm], r = sx[xr];
+            o.v[0][a] = sum(l, px.y, ym.x, yp.x, zm.x, zp.x, nmu, ua.x, er.x);
+            o.v[1][a] = sum(px.x, r, ym.y, yp.y, zm.y, zp.y, nmu, ua.y, er.y);
         }
         if (last) {
 #pragma unroll
@@ -771,16 +764,16 @@ __global__ void __launch_bounds__(kPointThreads)
 
 // The same for FP16 storage without walls and an even nx, packed arithmetic:
 // two cells per thread (aa_even_h2, aa_odd_h2), because 2-byte accesses of one
-// cell leave the load-store path, not HBM, as the bound.  256^3, even / odd step:
-// one cell 363 / 401 us, two cells 323 / 379 us.
+// cell leave the load-store path, not HBM, as the bound.  Whole 256^3 step: one
+// cell 760 us, two cells 703 us.
 template <bool DEV, bool ODD>
 __global__ void __launch_bounds__(256, 3)
-    lbm_aa_point_h2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, int zm, __half* f,
+    lbm_aa_point_h2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, __half* f,
                            const float* __restrict__ stress, float* F, float* __restrict__ rho_buf, float* u, int last) {
     const int c = 2 * (int)(blockIdx.x * 256 + threadIdx.x);
     pdl_begin();
     if (c >= (int)P.V) return;
-    const PairPointForce force{P, zm, stress, F, last};
+    const PairPointForce force{P, stress, u, F, last};
     const CellPos q = cell_pos<int>(P, c, dnx, dnxy);
     if constexpr (ODD) aa_odd_h2<DEV, int>(P, c, q, f, force, rho_buf, u, last);
     else aa_even_h2<DEV, int>(P, c, q, f, force, rho_buf, u, last);
