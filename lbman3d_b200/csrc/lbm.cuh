@@ -425,10 +425,11 @@ __device__ __forceinline__ CellPos cell_pos(const SimParams& P, I c, const FastD
 }
 
 // Even and odd in-place step of cell c; force(c, position, F) gives the body
-// force (read from memory, or formed from the stress in qpoint.cuh).
+// force (read from memory, or formed from the stress in qpoint.cuh).  uout is not
+// __restrict__: a force formed here reads the same array, the cell's own velocity.
 template <class R, class S, bool DEV, int WM, class I, class Force>
 __device__ __forceinline__ void aa_even_cell(const SimParams& P, const FastDiv& dnx, const FastDiv& dnxy, I c, S* F,
-                                             const Force& force, R* __restrict__ rho_buf, R* __restrict__ uout,
+                                             const Force& force, R* __restrict__ rho_buf, R* uout,
                                              int write_rho_all) {
     const I V = (I)P.V;
     const Phys<R>& K = phys_ref<R>(P);
@@ -459,7 +460,7 @@ __device__ __forceinline__ void aa_even_cell(const SimParams& P, const FastDiv& 
 
 template <class R, class S, bool DEV, int WM, class I, class Force>
 __device__ __forceinline__ void aa_odd_cell(const SimParams& P, const FastDiv& dnx, const FastDiv& dnxy, I c, S* F,
-                                            const Force& force, R* __restrict__ rho_buf, R* __restrict__ uout,
+                                            const Force& force, R* __restrict__ rho_buf, R* uout,
                                             int write_rho_all) {
     const I V = (I)P.V;
     const Phys<R>& K = phys_ref<R>(P);
@@ -592,7 +593,7 @@ struct LoadForce2 {
 
 template <bool DEV, class I, class Force>
 __device__ __forceinline__ void aa_even_h2(const SimParams& P, I c, const CellPos& q, __half* F, const Force& force,
-                                           float* __restrict__ rho_buf, float* __restrict__ uout, int write_rho_all) {
+                                           float* __restrict__ rho_buf, float* uout, int write_rho_all) {
     const I V = (I)P.V;
     const Phys<float>& K = phys_ref<float>(P);
     __half2 w[15];
@@ -637,7 +638,7 @@ __device__ __forceinline__ void aa_even_h2(const SimParams& P, I c, const CellPo
 
 template <bool DEV, class I, class Force>
 __device__ __forceinline__ void aa_odd_h2(const SimParams& P, I c, const CellPos& q, __half* F, const Force& force,
-                                          float* __restrict__ rho_buf, float* __restrict__ uout, int write_rho_all) {
+                                          float* __restrict__ rho_buf, float* uout, int write_rho_all) {
     const I V = (I)P.V;
     const Phys<float>& K = phys_ref<float>(P);
     const AxisOff<I> o0 = axis_off<I>(P, q);  // cell c (x even)
