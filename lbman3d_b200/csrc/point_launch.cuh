@@ -31,19 +31,23 @@ void with_mask(int m, F&& f) {
     else f(std::integral_constant<int, 15>{});
 }
 
+constexpr int kMaxGridY = 65535;
+
 // Planes per thread (a power of two): the longest walk that still gives every
 // SM a few blocks.  At most 4 planes, where the gain of reusing the centre
 // values ends, and 16 blocks per SM; packed kernels on planes with long walks
 // (long_walks), where a walk also saves the z terms' trip through memory, at
 // most 16 planes and 6 blocks per SM.  Steps with 1 / 2 / 4 / 8 / 16 planes there:
 // 128^3 138 / 135 / 131 / 127 / 131 us (the rule: 8), 160^3 274 / 261 / 254 / 249 /
-// 247 us (16).
+// 247 us (16).  A box of so many planes that its chunks would pass the launch's y
+// dimension walks further.
 inline int point_walk(const SimParams& P, bool pair, int num_sms) {
     const bool longer = pair && long_walks(P);
     const int per_block = kPointThreads * (pair ? 2 : 1);
     const int64_t cols = (P.nxy + per_block - 1) / per_block, blocks = (int64_t)(longer ? 6 : 16) * num_sms;
     int zc = longer ? 16 : 4;
     while (zc > 1 && cols * ((P.nz + zc - 1) / zc) < blocks) zc /= 2;
+    while ((P.nz + zc - 1) / zc > kMaxGridY) zc *= 2;
     return zc;
 }
 
