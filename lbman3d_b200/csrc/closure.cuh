@@ -292,7 +292,7 @@ __host__ __device__ inline bool dhalo_ok(int nx, int ny) { return nx % 8 == 0 &&
 // Copies plane zz (-1 <= zz <= nz, periodic) of the column at (x0, y0) into
 // its ring slot S (worker threads).
 template <int CIN, int WORKERS>
-__device__ __forceinline__ void dhalo_load_plane(const Grid3& g, const __nv_bfloat16* __restrict__ in, int x0,
+__device__ __forceinline__ void dhalo_load_plane(const Grid3& g, const __nv_bfloat16* in, int x0,
                                                  int y0, int zz, unsigned char* S) {
     constexpr int N = (CIN / 8) * kHX * kHY;
     const int64_t zoff = (int64_t)wrapi(zz, g.nz) * g.ny;
@@ -344,7 +344,7 @@ __device__ __forceinline__ void conv_epilogue(uint32_t tacc, int64_t c, int64_t 
 // Block b marches column b % cols over planes [zc * (b / cols), + zc).
 // Smem: B image, then the plane ring.
 template <int CIN, int COUT, int MODE>
-__global__ void __launch_bounds__(conv_threads(COUT)) conv_dhalo_kernel(Grid3 g, int zc, const __nv_bfloat16* __restrict__ in,
+__global__ void __launch_bounds__(conv_threads(COUT)) conv_dhalo_kernel(Grid3 g, int zc, const __nv_bfloat16* in,
                                                                const uint4* __restrict__ bimg,
                                                                const float* __restrict__ bias,
                                                                const __nv_bfloat16* __restrict__ pre_below,
@@ -664,8 +664,8 @@ struct WGradMarch {
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const __nv_bfloat16* __restrict__ act,
-                                                                const __nv_bfloat16* __restrict__ grad,
+__global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const __nv_bfloat16* act,
+                                                                const __nv_bfloat16* grad,
                                                                 float* __restrict__ partials, int* __restrict__ err,
                                                                 uint32_t wait_limit) {
     using WM = WGradMarch<CIN, COUT>;
@@ -837,7 +837,7 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
 // thread per j summing all P serially left most SMs idle.)  Launch with
 // kFoldThreads threads and ceil(n / 32) blocks.
 constexpr int kFoldThreads = 256;
-__global__ void __launch_bounds__(kFoldThreads) sum_partials_kernel(const float* __restrict__ partials, int P, int n,
+__global__ void __launch_bounds__(kFoldThreads) sum_partials_kernel(const float* partials, int P, int n,
                                                                      float* __restrict__ out) {
     __shared__ float slice[kFoldThreads / 32][32];
     const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
@@ -932,8 +932,8 @@ __device__ __forceinline__ float hash_normal(uint64_t key, uint64_t i) {
 // Network input from 9 FP32 channel blocks (rho, u, Q; [9][V]):
 // act0[c][j] = (x_j - shift_j) * inv_scale_j (+ noise_std N(0,1) when
 // training with input noise) for j < 9, 0 for j in 9..15.
-__global__ void features_kernel(const float* __restrict__ rho, const float* __restrict__ u3,
-                                const float* __restrict__ q5, int64_t V, const float* __restrict__ shift,
+__global__ void features_kernel(const float* rho, const float* u3,
+                                const float* q5, int64_t V, const float* __restrict__ shift,
                                 const float* __restrict__ inv_scale, __nv_bfloat16* __restrict__ act0,
                                 float noise_std, uint64_t noise_key) {
     pdl_begin();
@@ -962,7 +962,7 @@ __global__ void features_kernel(const float* __restrict__ rho, const float* __re
 // Mean-squared error of the 8 outputs against the raw targets [8][V]
 // normalised by inv_scale, its gradient gout[c][16] (BF16, channels 8..15
 // zero) and per-block partial sums of the squared error.
-__global__ void __launch_bounds__(kThreads) loss_kernel(const float* __restrict__ out, const float* __restrict__ tgt,
+__global__ void __launch_bounds__(kThreads) loss_kernel(const float* out, const float* tgt,
                                                         const float* __restrict__ inv_scale, int64_t V,
                                                         __nv_bfloat16* __restrict__ gout,
                                                         double* __restrict__ partials) {
@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(kThreads) loss_kernel(const float* __restrict_
 
 // Correction of a coarse state after its step: Q_k += gain out[k][c] s_k
 // (k < 5), u_d += gain out[5+d][c] s_{5+d}.
-__global__ void apply_kernel(const float* __restrict__ out, const float* __restrict__ out_scale, int64_t V,
+__global__ void apply_kernel(const float* out, const float* __restrict__ out_scale, int64_t V,
                              float gain, float* __restrict__ u3, float* __restrict__ q5) {
     pdl_begin();
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < V; c += (int64_t)gridDim.x * blockDim.x) {

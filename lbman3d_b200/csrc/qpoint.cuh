@@ -136,7 +136,7 @@ struct ColumnRules {
 
 template <class R, bool UPWIND, int QW>
 __device__ __forceinline__ void point_update(const SimParams& P, const Phys<R>& K, const ColumnRules& r, int z,
-                                             const R* __restrict__ qin, const R* __restrict__ uin, int c,
+                                             const R* qin, const R* uin, int c,
                                              const R (&qm)[5], const R (&qc)[5], const R (&qp)[5], const R (&um)[2],
                                              const R (&uc)[3], const R (&up)[3], R qn[5], R sg[5], R ta[3], R er[3]) {
     constexpr bool COMB = sizeof(R) == 4;
@@ -231,7 +231,7 @@ __device__ __forceinline__ void point_store(const Phys<R>& K, int V, int c, cons
 // Column `col` (index within the plane) of planes [z0, z1).
 template <class R, bool UPWIND, int QW>
 __device__ __forceinline__ void qpoint_column(const SimParams& P, int x, int y, int col, int z0, int z1, bool live,
-                                              const R* __restrict__ qin, const R* __restrict__ uin,
+                                              const R* qin, const R* uin,
                                               R* __restrict__ qout, R* __restrict__ stress, R* __restrict__ F) {
     const Phys<R>& K = phys_ref<R>(P);
     const int V = (int)P.V, nxy = (int)P.nxy, nz = P.nz;
@@ -296,8 +296,8 @@ constexpr int kPairPointMinBlocks = 3;
 // Block (bx, bz): cells [128 bx, 128 bx + 128) of each plane of z chunk bz.
 template <class R, bool UPWIND, int QW>
 __global__ void __launch_bounds__(kPointThreads, point_min_blocks<R>())
-    qpoint_kernel(const __grid_constant__ SimParams P, FastDiv dnx, int zc, const R* __restrict__ qin,
-                  const R* __restrict__ uin, R* __restrict__ qout, R* __restrict__ stress, R* __restrict__ F) {
+    qpoint_kernel(const __grid_constant__ SimParams P, FastDiv dnx, int zc, const R* qin,
+                  const R* uin, R* __restrict__ qout, R* __restrict__ stress, R* __restrict__ F) {
     const int n = (int)P.nxy;
     int col = blockIdx.x * kPointThreads + threadIdx.x;
     const bool live = col < n;
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<R>())
 // bit): a thread updates the cells x, x + 1 (x even; nx a multiple of 4), so
 // every field moves as one 8-byte access except the two x neighbours outside
 // the pair.  F holds g (or W) negated.
-__device__ __forceinline__ F2 ldg2(const float* p) { return {__ldg(reinterpret_cast<const float2*>(p))}; }
+__device__ __forceinline__ F2 ldg2(const float* p) { return {*reinterpret_cast<const float2*>(p)}; }
 __device__ __forceinline__ void stg2(float* p, F2 v) { *reinterpret_cast<float2*>(p) = v.v; }
 
 // The warp's 64 cells of plane z + 2 are asked into the second-level cache two
@@ -341,7 +341,7 @@ enum : int { WALK_SHORT = 0, WALK_LONG = 1, WALK_FORCE = 2 };
 
 template <bool UPWIND, int QW, int WALK>
 __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y, int col, int z0, int z1, bool live,
-                                               const float* __restrict__ qin, const float* __restrict__ uin,
+                                               const float* qin, const float* uin,
                                                float* __restrict__ qout, float* __restrict__ stress,
                                                float* __restrict__ F) {
     constexpr bool WALKS = WALK == WALK_FORCE;
@@ -400,7 +400,7 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
             const float* a = qin + (k * V + c);
             qp[k] = ldg2(qin + (k * V + p));
             const F2 cc = qc[k];
-            float l = __ldg(a + rq.xl), r = __ldg(a + rq.xr);
+            float l = a[rq.xl], r = a[rq.xr];
             F2 ym = ldg2(a + rq.o.ym), yp = ldg2(a + rq.o.yp), zm = qm[k], zp = qp[k];
             if constexpr (QW & QW_ANCHOR) {
                 float t = 0.0f;  // the neighbour inside the pair is never a ghost
@@ -428,7 +428,7 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
             const float* a = uin + (comp * V + c);
             up[comp] = ldg2(uin + (comp * V + p));
             const F2 cc = uc[comp];
-            const float l = __ldg(a + ru.xl), r = __ldg(a + ru.xr);
+            const float l = a[ru.xl], r = a[ru.xr];
             const F2 ym = ldg2(a + ru.o.ym), yp = ldg2(a + ru.o.yp);
             if constexpr (QW & QW_X)
                 gr[comp * 3] = f2(v_diff<float>(K, vx0, 0, comp, l, cc.v.x, cc.v.y), v_diff<float>(K, vx1, 0, comp, cc.v.x, cc.v.y, r));
@@ -504,8 +504,8 @@ __device__ __forceinline__ void qpoint2_column(const SimParams& P, int x, int y,
 // Block (bx, bz): cells [256 bx, 256 bx + 256) of each plane of z chunk bz.
 template <bool UPWIND, int QW, int WALK>
 __global__ void __launch_bounds__(kPointThreads, kPairPointMinBlocks)
-    qpoint2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, int zc, const float* __restrict__ qin,
-                   const float* __restrict__ uin, float* __restrict__ qout, float* __restrict__ stress,
+    qpoint2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, int zc, const float* qin,
+                   const float* uin, float* __restrict__ qout, float* __restrict__ stress,
                    float* __restrict__ F) {
     const int n = (int)P.nxy;
     int col = 2 * (blockIdx.x * kPointThreads + threadIdx.x);
@@ -529,8 +529,8 @@ struct PointForce {
     static constexpr bool kNeedsPos = true;
     const SimParams& P;
     int zm;
-    const R* __restrict__ qn;
-    const R* __restrict__ stress;
+    const R* qn;
+    const R* stress;
     const R* u;
     const R* F;
     __device__ __forceinline__ void operator()(int c, const CellPos& q, R out[3]) const {
@@ -670,8 +670,8 @@ struct PointForce {
 
 template <class R, int QW, bool PAIR = false, bool WALKS = false>
 __global__ void __launch_bounds__(256)
-    point_force_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, int zm, const R* __restrict__ qn,
-                       const R* __restrict__ stress, const R* u, R* F) {
+    point_force_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, int zm, const R* qn,
+                       const R* stress, const R* u, R* F) {
     const int c = (int)(blockIdx.x * 256 + threadIdx.x);
     pdl_begin();
     if (c >= (int)P.V) return;
@@ -753,7 +753,7 @@ struct PairPointForce {
 template <class R, class S, bool DEV, int WM, int QW, bool ODD, bool PAIR = false, bool WALKS = false>
 __global__ void __launch_bounds__(kPointThreads)
     lbm_aa_point_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, int zm, S* f,
-                        const R* __restrict__ qn, const R* __restrict__ stress, R* F, R* __restrict__ rho_buf, R* u, int last) {
+                        const R* qn, const R* stress, R* F, R* __restrict__ rho_buf, R* u, int last) {
     const int c = (int)(blockIdx.x * kPointThreads + threadIdx.x);
     pdl_begin();
     if (c >= (int)P.V) return;
@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(kPointThreads)
 template <bool DEV, bool ODD>
 __global__ void __launch_bounds__(256, 3)
     lbm_aa_point_h2_kernel(const __grid_constant__ SimParams P, FastDiv dnx, FastDiv dnxy, __half* f,
-                           const float* __restrict__ stress, float* F, float* __restrict__ rho_buf, float* u, int last) {
+                           const float* stress, float* F, float* __restrict__ rho_buf, float* u, int last) {
     const int c = 2 * (int)(blockIdx.x * 256 + threadIdx.x);
     pdl_begin();
     if (c >= (int)P.V) return;
