@@ -25,8 +25,8 @@
         if (cudaError_t e = cudaMemsetAsync(count, 0, sizeof(*count), st)) return e;                           \
         const int gx = (P.nx + kDefX - 1) / kDefX, gy = (P.ny + kDefY - 1) / kDefY;                            \
         const int zc = diag_planes((int64_t)gx * gy, P.nz);                                                    \
-        defect_kernel<R><<<dim3(gx, gy, (P.nz + zc - 1) / zc), kDefThreads, 0, st>>>(P, zc, (const R*)q,       \
-                                                                                     flags, count);            \
+        const int64_t blocks = (int64_t)gx * gy * ((P.nz + zc - 1) / zc);                                      \
+        defect_kernel<R><<<(unsigned)blocks, kDefThreads, 0, st>>>(P, zc, (const R*)q, flags, count);          \
         return cudaGetLastError();                                                                             \
     }                                                                                                          \
     }

@@ -279,6 +279,8 @@ __device__ __forceinline__ bool plaquette_flip(const R d1[3], const R d2[3], con
 // (each is formed 1.1 times), where a director pass and a pass over its 24-byte
 // records took 567 us for 256^3 FP32.  The periodic seam faces are not visited,
 // as in the reference.
+// Block (bx, by, bz) of tiles and z chunks is one of the launch's x dimension:
+// long or tall boxes have more than the 65535 the others take.
 //   count: receives the number of flagged plaquettes (added atomically);
 //   flags: if not null, the flags in the reference's DefectFields layout
 //   (src/analysis/defect_fields.h:16-29): def_x nx*(ny-1)*(nz-1), then def_y
@@ -294,8 +296,10 @@ __global__ void __launch_bounds__(kDefThreads) defect_kernel(const __grid_consta
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const int64_t nfx = (int64_t)nx * (ny - 1) * (nz - 1), nfy = (int64_t)(nx - 1) * ny * (nz - 1);
     const int lx = threadIdx.x % kDefTX, ly = threadIdx.x / kDefTX;
-    const int x = blockIdx.x * kDefX + lx, y = blockIdx.y * kDefY + ly;
-    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);  // def_z planes of this block
+    const int gx = (nx + kDefX - 1) / kDefX, gy = (ny + kDefY - 1) / kDefY;
+    const int bx = blockIdx.x % gx, by = blockIdx.x / gx % gy, bz = blockIdx.x / gx / gy;
+    const int x = bx * kDefX + lx, y = by * kDefY + ly;
+    const int z0 = bz * zc, z1 = min(z0 + zc, nz);  // def_z planes of this block
     const bool in = x < nx && y < ny;
     const bool own = in && lx < kDefX && ly < kDefY;
     const int64_t col = (int64_t)y * nx + x;

@@ -32,3 +32,18 @@ def test_point_kernels_step_a_tall_box(grid, precision, kernels, tile):
             out.append(s.download(force=True))
     for n in out[0]:
         np.testing.assert_array_equal(out[0][n], out[1][n], err_msg=n)
+
+
+# more than 65535 of the 15-row tiles, of the 32-plane marches
+@pytest.mark.parametrize("grid", [(2, 983100, 2), (2, 2, 2097200)], ids=["long_y", "tall"])
+def test_defects_of_a_long_box(grid):
+    from cases import BC
+    from oracle import oracle as O
+    nx, ny, nz = grid
+    p = L.Params(nx=nx, ny=ny, nz=nz)
+    with L.Simulation(p, L.FullyPeriodicConfig(), L.Precision.FP64) as s:
+        s.upload(*_state(p.V))
+        d = s.reduce(N.DIAG_DEFECTS)
+        q = s.download()["q"]
+    op = O.make_params(nx, ny, nz, BC["periodic"])
+    assert d["defect_faces"] == O.winding(op, O.order_director(op, q)[1])[0]
