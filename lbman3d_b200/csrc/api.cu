@@ -250,6 +250,13 @@ constexpr int64_t kPointFusedCells = (int64_t)6 << 20;
 // two-phase stress, snapshots, statistics), so that none of them fails for it.
 constexpr int64_t kPointSpareWords = 48;
 
+// The z-marching kernels from here on; the point kernels' scratch is given back.
+void drop_point(lbman_solver* s) {
+    s->point = false;
+    cudaFree(s->pstress);
+    s->pstress = nullptr;
+}
+
 // Default z-marching tile before any autotuning: the widest compiled tile
 // up to 32 cells whose last partial tile pads x by at most 10% (wide rows
 // keep the global stores of a block in full sectors); otherwise the one with
@@ -997,8 +1004,7 @@ int lbman_get_shape(lbman_solver* s, lbman_shape* out) {
     return LBMAN_OK;
 }
 
-int lbman_set_shape(lbman_solver* s, const lbman_shape* sh) {
-    if (!s || !sh) return fail(LBMAN_ERR_ARG, "null argument");
+static int check_shape(lbman_solver* s, const lbman_shape* sh, QTile* tile) {
     if (sh->kernels != LBMAN_KERNELS_SPLIT && sh->kernels != LBMAN_KERNELS_FUSED &&
         sh->kernels != LBMAN_KERNELS_SPLIT_PAIR)
         return fail(LBMAN_ERR_ARG, "kernels must be LBMAN_KERNELS_SPLIT, LBMAN_KERNELS_FUSED or LBMAN_KERNELS_SPLIT_PAIR");
@@ -1012,10 +1018,26 @@ int lbman_set_shape(lbman_solver* s, const lbman_shape* sh) {
     if (s->ops().qforce_smem(t) == 0)
         return fail(LBMAN_ERR_ARG, "tile %dx%d is not compiled for this precision%s", sh->tile_x, sh->tile_y,
                     t.pair ? " and organisation" : "");
+    *tile = t;
+    return LBMAN_OK;
+}
+
+// Steps with the z-marching launch sh names; the point kernels' scratch stays.
+static int use_shape(lbman_solver* s, const lbman_shape* sh) {
+    QTile t;
+    LB_TRY(check_shape(s, sh, &t));
     s->kernels = sh->kernels;
-    s->point = false;  // a shape names a z-marching launch
+    s->point = false;
     s->shape.tile = t;
     s->shape.qthreads = s->ops().qforce_threads(t);
+    return LBMAN_OK;
+}
+
+int lbman_set_shape(lbman_solver* s, const lbman_shape* sh) {
+    if (!s || !sh) return fail(LBMAN_ERR_ARG, "null argument");
+    LB_TRY(use_shape(s, sh));
+    LB_TRY(set_device(s));
+    drop_point(s);
     return LBMAN_OK;
 }
 
@@ -1096,7 +1118,7 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
                     for (int zj = 0; zj < zi; ++zj) seen = seen || zs[zj] == zs[zi];
                     if (seen || (zi >= 6 && zs[zi] >= nzo)) continue;
                     cur = {k, t[0], t[1], zs[zi], 0, 0.0};
-                    if (lbman_set_shape(s, &cur) != LBMAN_OK) continue;
+                    if (use_shape(s, &cur) != LBMAN_OK) continue;
                     if ((status = time_trial(s, steps_per_trial, e0, e1, &cur.ms_per_step)) != LBMAN_OK) break;
                     ++count;
                     trials.push_back(cur);
@@ -1110,7 +1132,7 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
                   [](const lbman_shape& a, const lbman_shape& b) { return a.ms_per_step < b.ms_per_step; });
         for (size_t i = 0; i < trials.size() && i < 4 && status == LBMAN_OK; ++i) {
             cur = trials[i];
-            if (lbman_set_shape(s, &cur) != LBMAN_OK) continue;
+            if (use_shape(s, &cur) != LBMAN_OK) continue;
             if ((status = time_trial(s, 3 * steps_per_trial, e0, e1, &cur.ms_per_step)) != LBMAN_OK) break;
             ++count;
             if (cur.ms_per_step < win.ms_per_step) win = cur;
@@ -1124,16 +1146,17 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
     if (e1) cudaEventDestroy(e1);
     cudaFree(snap);
     if (status != LBMAN_OK) {
-        lbman_set_shape(s, &orig);
+        use_shape(s, &orig);
         s->point = point0;
         return status;
     }
-    if (point_ms <= win.ms_per_step) {
-        win = orig;
+    if (point0 && point_ms <= win.ms_per_step) {
+        use_shape(s, &orig);
+        s->point = true;
         win.ms_per_step = point_ms;
+    } else {
+        lbman_set_shape(s, &win);
     }
-    lbman_set_shape(s, &win);
-    s->point = point_ms <= win.ms_per_step;
     lbman_get_shape(s, best);
     best->ms_per_step = win.ms_per_step;
     if (ntrials) *ntrials = count;
@@ -1162,9 +1185,7 @@ int lbman_create_slab(const lbman_config* cfg, int nz_global, int z_offset, lbma
     lbman_solver* s = nullptr;
     LB_TRY(lbman_create(&c, &s));
     s->slab = true;
-    s->point = false;  // the point kernels cover whole boxes
-    cudaFree(s->pstress);
-    s->pstress = nullptr;
+    drop_point(s);  // the point kernels cover whole boxes
     s->nz_global = nz_global;
     s->z_offset = z_offset;
     SimParams& P = s->P;
