@@ -60,8 +60,9 @@ extern "C" {
 /* Kernel organisation. */
 /* AUTO: the split organisation (two points per thread where its 30-wide tiles
  * fit); a whole box in the size range where they are faster is stepped with
- * the shared-memory-free kernels, which do the same arithmetic bit for bit,
- * until a shape is set.                                                     */
+ * the shared-memory-free kernels, which do the same arithmetic bit for bit.
+ * Such a handle names them by the shape it was created with (lbman_get_shape);
+ * any other shape selects the z-marching kernels and gives their scratch back. */
 #define LBMAN_KERNELS_AUTO 0
 #define LBMAN_KERNELS_SPLIT 1 /* Q+force kernel, then LBM kernel               */
 #define LBMAN_KERNELS_FUSED 2 /* one kernel per time step                      */
@@ -229,14 +230,15 @@ typedef struct lbman_shape {
 int lbman_get_shape(lbman_solver* s, lbman_shape* out);
 /* Select a shape (tile_x x tile_y must be one of the compiled tiles: 30x6,
  * 32x6, 14x14, 32x8, and for FP32/FP16 also 30x14, 62x6, 32x14, 64x6;
- * zchunk >= -8).                                                           */
+ * zchunk >= -8).  The shape an AUTO handle was created with selects the
+ * shared-memory-free kernels again where it started with them and their scratch
+ * (9 words per cell, 8 in FP64) still fits.                                 */
 int lbman_set_shape(lbman_solver* s, const lbman_shape* shape);
 /* Autotuner (no counterpart in the reference): times steps_per_trial steps
  * of every kernel organisation x compiled tile x z-chunk candidate, and of the
- * shared-memory-free kernels of an AUTO handle (for which best holds the
- * handle's own shape), on the current state with CUDA events, keeps the
- * fastest and restores the state
- * it started from bit for bit (a temporary device copy of the fields is
+ * shared-memory-free kernels of an AUTO handle (named by the shape it was
+ * created with), on the current state with CUDA events, keeps the fastest and
+ * restores the state it started from bit for bit (a temporary device copy of the fields is
  * taken for that).  ntrials (may be NULL) receives the number of candidates
  * timed.                                                                    */
 int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int* ntrials);

@@ -166,8 +166,10 @@ struct lbman_solver {
     void* rho = nullptr;
     void* F = nullptr;
     // Point organisation (qpoint.cuh): steps run without the z-marching Q
-    // kernel; pstress holds the stress between its two kernels.
-    bool point = false;
+    // kernel; pstress holds the stress between its two kernels.  A handle it
+    // can step (point_able) names it by the shape it was created with.
+    bool point = false, point_able = false;
+    lbman_shape untuned{};
     void* pstress = nullptr;
     void* stress = nullptr;  // Sigma (5) and tau (3) of the two-phase Q stage, allocated on first use
     double* staging = nullptr;
@@ -249,6 +251,20 @@ constexpr int64_t kPointFusedCells = (int64_t)6 << 20;
 // kernels' scratch: the buffers it may ask for later (second population buffer,
 // two-phase stress, snapshots, statistics), so that none of them fails for it.
 constexpr int64_t kPointSpareWords = 48;
+
+// Scratch of the point kernels: 9 row-stress words (FP32) or Sigma and tau
+// (FP64) per cell.  A box that has no room for them keeps the z-marching kernels.
+bool take_point(lbman_solver* s) {
+    const size_t words = s->prec == LBMAN_FP64 ? 8 : 9;
+    size_t free_bytes = 0, total = 0;
+    if (!s->pstress && (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess ||
+                        (words + kPointSpareWords) * s->P.V * s->rbytes > free_bytes ||
+                        cudaMalloc(&s->pstress, words * s->P.V * s->rbytes) != cudaSuccess)) {
+        cudaGetLastError();
+        s->pstress = nullptr;
+    }
+    return s->point = s->pstress != nullptr;
+}
 
 // The z-marching kernels from here on; the point kernels' scratch is given back.
 void drop_point(lbman_solver* s) {
@@ -481,20 +497,10 @@ int lbman_create(const lbman_config* cfg, lbman_solver** out) {
         if (int st = alloc(&s->q[b], 5 * V * s->rbytes)) return bail(st);
         if (int st = alloc(&s->u[b], 3 * V * s->rbytes)) return bail(st);
     }
-    if (cfg->kernels == LBMAN_KERNELS_AUTO && cfg->tile_x == 0 && cfg->tile_y == 0 && cfg->zchunk == 0 &&
-        V <= kPointCells) {
-        // 9 row-stress words (FP32) or Sigma and tau (FP64) per cell; a box that
-        // has no room for them keeps the z-marching kernels
-        const size_t words = s->prec == LBMAN_FP64 ? 8 : 9;
-        size_t free_bytes = 0, total = 0;
-        if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess &&
-            (words + kPointSpareWords) * V * s->rbytes <= free_bytes)
-            s->point = cudaMalloc(&s->pstress, words * V * s->rbytes) == cudaSuccess;
-        if (!s->point) {
-            cudaGetLastError();
-            s->pstress = nullptr;
-        }
-    }
+    s->point_able = cfg->kernels == LBMAN_KERNELS_AUTO && cfg->tile_x == 0 && cfg->tile_y == 0 && cfg->zchunk == 0 &&
+                    V <= kPointCells;
+    s->untuned = {kern, s->shape.tile.tcx, s->shape.tile.tcy, s->shape.tile.zc, 0, 0.0, 0};
+    if (s->point_able) take_point(s);
     if (int st = alloc(&s->rho, V * s->rbytes)) return bail(st);
     if (int st = alloc(&s->F, 3 * V * s->rbytes)) return bail(st);
     // FP64 host staging too: downloads of an in-place-layout state gather
@@ -1033,11 +1039,18 @@ static int use_shape(lbman_solver* s, const lbman_shape* sh) {
     return LBMAN_OK;
 }
 
+// Does the shape name the point kernels?
+static bool names_point(const lbman_solver* s, const lbman_shape* sh) {
+    return s->point_able && sh->kernels == s->untuned.kernels && sh->tile_x == s->untuned.tile_x &&
+           sh->tile_y == s->untuned.tile_y && sh->zchunk == s->untuned.zchunk;
+}
+
 int lbman_set_shape(lbman_solver* s, const lbman_shape* sh) {
     if (!s || !sh) return fail(LBMAN_ERR_ARG, "null argument");
     LB_TRY(use_shape(s, sh));
     LB_TRY(set_device(s));
-    drop_point(s);
+    if (names_point(s, sh)) take_point(s);
+    else drop_point(s);
     return LBMAN_OK;
 }
 
@@ -1083,7 +1096,7 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
     int status = LBMAN_OK, count = 0;
     lbman_shape orig, cur{}, win{};
     std::vector<lbman_shape> trials;
-    const bool point0 = s->point;
+    bool point = false;
     double point_ms = 1e30;
     lbman_get_shape(s, &orig);
     win = orig;
@@ -1091,7 +1104,8 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
     if (copy_state(true) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
         status = fail(LBMAN_ERR_CUDA, "autotune set-up failed");
     } else {
-        if (point0) {  // the point kernels have no shape: one trial, at the length of the final ones
+        point = s->point_able && use_shape(s, &s->untuned) == LBMAN_OK && take_point(s);
+        if (point) {  // the point kernels: one trial, at the length of the final ones
             status = time_trial(s, 3 * steps_per_trial, e0, e1, &point_ms);
             ++count;
         }
@@ -1118,6 +1132,7 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
                     for (int zj = 0; zj < zi; ++zj) seen = seen || zs[zj] == zs[zi];
                     if (seen || (zi >= 6 && zs[zi] >= nzo)) continue;
                     cur = {k, t[0], t[1], zs[zi], 0, 0.0};
+                    if (point && names_point(s, &cur)) continue;
                     if (use_shape(s, &cur) != LBMAN_OK) continue;
                     if ((status = time_trial(s, steps_per_trial, e0, e1, &cur.ms_per_step)) != LBMAN_OK) break;
                     ++count;
@@ -1146,17 +1161,14 @@ int lbman_autotune(lbman_solver* s, int steps_per_trial, lbman_shape* best, int*
     if (e1) cudaEventDestroy(e1);
     cudaFree(snap);
     if (status != LBMAN_OK) {
-        use_shape(s, &orig);
-        s->point = point0;
+        lbman_set_shape(s, &orig);
         return status;
     }
-    if (point0 && point_ms <= win.ms_per_step) {
-        use_shape(s, &orig);
-        s->point = true;
+    if (point && point_ms <= win.ms_per_step) {
+        win = s->untuned;
         win.ms_per_step = point_ms;
-    } else {
-        lbman_set_shape(s, &win);
     }
+    lbman_set_shape(s, &win);
     lbman_get_shape(s, best);
     best->ms_per_step = win.ms_per_step;
     if (ntrials) *ntrials = count;
@@ -1186,6 +1198,7 @@ int lbman_create_slab(const lbman_config* cfg, int nz_global, int z_offset, lbma
     LB_TRY(lbman_create(&c, &s));
     s->slab = true;
     drop_point(s);  // the point kernels cover whole boxes
+    s->point_able = false;
     s->nz_global = nz_global;
     s->z_offset = z_offset;
     SimParams& P = s->P;
