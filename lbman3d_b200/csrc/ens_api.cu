@@ -92,6 +92,7 @@ struct lbman_ensemble {
     bool small = true;               // every box within the split kernels' 32-bit indices
     int par = 0, fcur = 0, fphase = F_PRE;
     bool uploaded = false, stepped = false;
+    bool held = false;               // the organisation's own buffers are there
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaGraphExec_t graph = nullptr;
@@ -109,26 +110,30 @@ void drop_graph(lbman_ensemble* e) {
     e->graph_par = -1;
 }
 
-// Second population and velocity buffers of the fused organisation, or the
-// stress of the split one, on first use (build_work uploads the pointers).
-int ensure_buffers(lbman_ensemble* e) {
-    const bool fused = e->kernels == LBMAN_KERNELS_FUSED;
+// The buffers only one organisation uses: the fused one's second populations or
+// the split one's stress.  Gives the other's back first, so an ensemble never
+// needs the memory of both; false if there is no room (build_work uploads the
+// pointers).
+bool hold_buffers(lbman_ensemble* e, bool fused) {
     const size_t words = e->prec == LBMAN_FP64 ? point_stress_words<double>() : point_stress_words<float>();
+    e->held = false;
     for (EnsBox& B : e->host) {
-        const int64_t V = B.P.V;
-        struct { void** p; size_t n; bool want; } want[] = {
-            {&B.f[1], 15 * V * e->sbytes, fused}, {&B.stress, words * V * e->rbytes, !fused}};
-        for (auto& w : want) {
-            if (!w.want || *w.p) continue;
-            if (cudaMalloc(w.p, w.n) != cudaSuccess) {
-                cudaGetLastError();
-                *w.p = nullptr;
-                return efail(LBMAN_ERR_NOMEM, "cudaMalloc of an ensemble buffer failed");
-            }
-            e->allocs.push_back(*w.p);
+        if (!fused && e->fcur) std::swap(B.f[0], B.f[1]);
+        void*& other = fused ? B.stress : B.f[1];
+        cudaFree(other);
+        other = nullptr;
+    }
+    if (!fused) e->fcur = 0;
+    for (EnsBox& B : e->host) {
+        void*& p = fused ? B.f[1] : B.stress;
+        const size_t n = fused ? 15 * e->sbytes : words * e->rbytes;
+        if (!p && cudaMalloc(&p, n * B.P.V) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+            return false;
         }
     }
-    return LBMAN_OK;
+    return e->held = true;
 }
 
 template <class T>
@@ -149,7 +154,6 @@ int upload_list(lbman_ensemble* e, const std::vector<T>& v, T** d) {
 // kEnsLbmCells cells (split).
 int build_work(lbman_ensemble* e) {
     constexpr int kWalk = 4;  // planes per thread, as in a large single box
-    if (int st = ensure_buffers(e)) return st;
     std::vector<EnsQWork> q;
     std::vector<EnsPointWork> p;
     std::vector<EnsLbmWork> l;
@@ -351,10 +355,15 @@ int lbman_ensemble_create(const lbman_config* cfgs, int nboxes, lbman_ensemble**
         for (int k = 0; k < 7; ++k) {
             if (cudaMalloc(slots[k], sizes[k]) != cudaSuccess)
                 return bail(efail(LBMAN_ERR_NOMEM, "cudaMalloc of an ensemble box failed"));
-            e->allocs.push_back(*slots[k]);
+            if (k != 4) e->allocs.push_back(*slots[k]);  // f[0] and f[1] may change places
         }
     }
     if (!e->small) e->kernels = LBMAN_KERNELS_FUSED;
+    // where only the second populations fit (FP16 storage: 30 bytes per cell for
+    // the stress's 36), the ensemble steps with the fused kernels (the same results)
+    if (e->kernels == LBMAN_KERNELS_SPLIT && !hold_buffers(e, false)) e->kernels = LBMAN_KERNELS_FUSED;
+    if (e->kernels == LBMAN_KERNELS_FUSED && !hold_buffers(e, true))
+        return bail(efail(LBMAN_ERR_NOMEM, "cudaMalloc of an ensemble buffer failed"));
     if (cudaMalloc(&e->staging, e->maxV * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&e->dboxes, nboxes * sizeof(EnsBox)) != cudaSuccess)
         return bail(efail(LBMAN_ERR_NOMEM, "cudaMalloc failed"));
@@ -372,6 +381,11 @@ int lbman_ensemble_destroy(lbman_ensemble* e) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     drop_graph(e);
     for (void* p : e->allocs) cudaFree(p);
+    for (EnsBox& B : e->host) {
+        cudaFree(B.f[0]);
+        cudaFree(B.f[1]);
+        cudaFree(B.stress);
+    }
     cudaFree(e->staging);
     cudaFree(e->dboxes);
     cudaFree(e->qwork);
@@ -490,6 +504,7 @@ int lbman_ensemble_download(lbman_ensemble* e, int box, double* rho, double* u3,
     if (f15) {
         const void* src = B.f[e->fcur];
         if (e->fphase == F_POST) {
+            if (!e->held) return efail(LBMAN_ERR_NOMEM, "the ensemble's buffers did not fit");
             if (e->ops().stream_only(P, src, B.f[1 - e->fcur], B.rho, e->stream) != cudaSuccess)
                 return efail(LBMAN_ERR_CUDA, "stream failed");
             src = B.f[1 - e->fcur];
@@ -513,6 +528,7 @@ int lbman_ensemble_download(lbman_ensemble* e, int box, double* rho, double* u3,
 int lbman_ensemble_step(lbman_ensemble* e, int nsteps) {
     if (!e || nsteps < 0) return efail(LBMAN_ERR_ARG, "bad arguments");
     if (!e->uploaded) return efail(LBMAN_ERR_STATE, "step before initialisation");
+    if (!e->held) return efail(LBMAN_ERR_NOMEM, "the ensemble's buffers did not fit");
     E_CUDA(cudaSetDevice(e->device));
     int done = 0;
     // rho everywhere is refreshed by the final step of each call; the first
@@ -551,12 +567,8 @@ int lbman_ensemble_set_shape(lbman_ensemble* e, int kernels, int tile_x, int til
         return efail(LBMAN_ERR_ARG, "kernels must be SPLIT or FUSED");
     if (e->ops().qforce_smem(QTile{tile_x, tile_y, 1}) == 0)
         return efail(LBMAN_ERR_ARG, "tile is not compiled for this precision");
+    E_CUDA(cudaSetDevice(e->device));
     if (!e->small) kernels = LBMAN_KERNELS_FUSED;
-    const int before = e->kernels;
-    e->kernels = kernels;
-    const int have = ensure_buffers(e);
-    e->kernels = before;
-    if (have != LBMAN_OK) return have;
     if (e->stepped && kernels != e->kernels) {
         // the split organisation keeps u in u[0]; the fused one ping-pongs
         const int p = e->par;
@@ -567,6 +579,15 @@ int lbman_ensemble_set_shape(lbman_ensemble* e, int kernels, int tile_x, int til
                 E_CUDA(cudaMemcpyAsync(B.u[0], B.u[p], 3 * B.P.V * e->rbytes, cudaMemcpyDeviceToDevice, e->stream));
         }
         E_CUDA(cudaStreamSynchronize(e->stream));
+    }
+    // before the second population buffer goes: reading back the two-buffer
+    // layout needs it
+    if (kernels == LBMAN_KERNELS_SPLIT && e->fphase == F_POST)
+        if (int st = ens_layout(e, F_SWAP)) return st;
+    if (!hold_buffers(e, kernels == LBMAN_KERNELS_FUSED)) {
+        if (hold_buffers(e, e->kernels == LBMAN_KERNELS_FUSED))
+            if (int st = build_work(e)) return st;  // the buffers moved
+        return efail(LBMAN_ERR_NOMEM, "cudaMalloc of an ensemble buffer failed");
     }
     e->kernels = kernels;
     e->tcx = tile_x;
@@ -599,9 +620,9 @@ int lbman_ensemble_autotune(lbman_ensemble* e, int steps_per_trial, lbman_shape*
                                    15 * V * e->sbytes, V * e->rbytes,     3 * V * e->rbytes};
         return s[k];
     };
-    const int fcur0 = e->fcur, fphase0 = e->fphase;
+    const int fphase0 = e->fphase;
     auto ptr_of = [&](EnsBox& B, int k) -> void* {
-        void* p[kFields] = {B.q[0], B.q[1], B.u[0], B.u[1], B.f[fcur0], B.rho, B.F};
+        void* p[kFields] = {B.q[0], B.q[1], B.u[0], B.u[1], B.f[e->fcur], B.rho, B.F};
         return p[k];
     };
     for (auto& B : e->host)
@@ -655,6 +676,7 @@ int lbman_ensemble_autotune(lbman_ensemble* e, int steps_per_trial, lbman_shape*
     }
     // restore: fields, parity and the velocity organisation of the original shape
     e->kernels = kern0;
+    e->fcur = 0;
     int i = 0;
     for (auto& B : e->host)
         for (int k = 0; k < kFields; ++k, ++i)
@@ -664,7 +686,6 @@ int lbman_ensemble_autotune(lbman_ensemble* e, int steps_per_trial, lbman_shape*
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     e->par = par0;
-    e->fcur = fcur0;
     e->fphase = fphase0;
     e->stepped = stepped0;
     e->steps = steps0;
