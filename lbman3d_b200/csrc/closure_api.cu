@@ -292,12 +292,12 @@ __global__ void __launch_bounds__(kFoldLossThreads) fold_loss_kernel(const doubl
 
 // Device copies of the host arrays of lbman_closure_forward / _gradient, kept
 // between calls (allocating and freeing them cost more than the kernels of a
-// 64^3 gradient).
-int ensure_io(lbman_closure* c) {
+// 64^3 gradient); a call takes those it uses.
+int ensure_io(lbman_closure* c, bool gradient) {
     const size_t V = (size_t)c->V;
     if (!c->x_in) CL_CUDA(cudaMalloc(&c->x_in, 9 * V * sizeof(float)));
-    if (!c->t_in) CL_CUDA(cudaMalloc(&c->t_in, 8 * V * sizeof(float)));
-    if (!c->loss_out) CL_CUDA(cudaMalloc(&c->loss_out, sizeof(double)));
+    if (gradient && !c->t_in) CL_CUDA(cudaMalloc(&c->t_in, 8 * V * sizeof(float)));
+    if (gradient && !c->loss_out) CL_CUDA(cudaMalloc(&c->loss_out, sizeof(double)));
     return LBMAN_OK;
 }
 
@@ -487,7 +487,7 @@ int lbman_closure_forward(lbman_closure* c, const float* feat9, float* out8) {
     if (!c || !feat9 || !out8) return failc(LBMAN_ERR_ARG, "closure: null argument");
     CL_CUDA(cudaSetDevice(c->device));
     const int64_t V = c->V;
-    CL_TRY(ensure_io(c));
+    CL_TRY(ensure_io(c, false));
     float* dx = c->x_in;
     CL_CUDA(cudaMemcpyAsync(dx, feat9, 9 * V * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     CL_TRY(features(c, c->stream, dx, dx + V, dx + 4 * V));
@@ -502,7 +502,7 @@ int lbman_closure_gradient(lbman_closure* c, const float* feat9, const float* ta
     if (!c || !feat9 || !target8) return failc(LBMAN_ERR_ARG, "closure: null argument");
     CL_CUDA(cudaSetDevice(c->device));
     const int64_t V = c->V;
-    CL_TRY(ensure_io(c));
+    CL_TRY(ensure_io(c, true));
     float* dx = c->x_in;
     CL_CUDA(cudaMemcpyAsync(dx, feat9, 9 * V * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     CL_TRY(features(c, c->stream, dx, dx + V, dx + 4 * V));
