@@ -635,32 +635,37 @@ __global__ void __launch_bounds__(kThreads) wgrad_kernel(Grid3 g, const __nv_bfl
 // and one block per 8-channel group:
 //   unit(slot, g, hy, x) at slot*SLOT + (g*18 + hy)*8 + x,  g = (dx+1)*CIN/8 + kg,
 // so 16 consecutive groups at one stride are the M = 128 rows of an operand:
-// the 3 CIN rows of the three dx taps, a group whose channel 0 is the constant
-// 1 (its row of the product is the bias gradient), and groups of the next slot
-// whose rows are not read back.  dy moves the start by one row (128 bytes), dz
-// picks the slot, and the K groups (y rows) are 128 bytes apart.  A tile is 9
-// (dy, dz) x 8 K-steps of MMAs and costs one new plane and one gradient tile;
-// nothing is copied inside shared memory.  (Assembling a 32 KB operand per 4
-// taps in shared memory instead took 179 us per 32 -> 32 layer at 64^3, and the
-// bias gradient 25 us in kernels of its own.)
+// the 3 CIN rows of the three dx taps, and groups of the next slot whose rows
+// are not read back.  dy moves the start by one row (128 bytes), dz picks the
+// slot, and the K groups (y rows) are 128 bytes apart.  A tile is 9 (dy, dz) x 8
+// K-steps of MMAs and costs one new plane and one gradient tile; nothing is
+// copied inside shared memory.  (Assembling a 32 KB operand per 4 taps in shared
+// memory instead took 179 us per 32 -> 32 layer at 64^3, and the bias gradient
+// 25 us in kernels of its own.)
 //
 // One block per SM takes an equal share of the column-major sequence of tiles.
 // Warps 0-7 copy (two planes ahead, ring of 5 planes and 3 gradient tiles),
 // warp 8 issues the MMAs; one block barrier per tile.  The nine accumulators
-// (COUT columns each) stay in TMEM for the whole share.
+// (COUT columns each) stay in TMEM for half of the share: the tensor core's FP32
+// sums drift with their length, and the halves, added in FP32, are as long as
+// the sums of two blocks per SM.  The bias gradient, which needs no product, is
+// summed by the copying warps from the staged tiles in FP32.  Error against 64
+// bits at 80^3, of the sum of the terms' magnitudes, weights / biases: 1.8e-6 /
+// 7e-8; whole shares with the biases as a row of the product 5.0e-6 / 4.4e-7, in
+// 57 us for the 72 us a 32 -> 32 layer takes at 64^3.
 constexpr int kWRing = 5, kWGrads = 3;
 template <int CIN, int COUT>
 struct WGradMarch {
     static constexpr int KGN = CIN / 8;
     static constexpr int GROUP = kHY * 8 * 16;             // bytes of one channel group
-    static constexpr int SLOTG = 3 * KGN + 1;              // groups per plane, the constant one last
+    static constexpr int SLOTG = 3 * KGN;                  // groups per plane
     static constexpr int SLOT = SLOTG * GROUP;
     static constexpr int PAD = (16 - SLOTG) * GROUP;       // the last slot's operand ends here
     static constexpr int GB = (COUT / 8) * 2048;           // output-gradient tile
     static constexpr int SMEM = kWRing * SLOT + PAD + kWGrads * GB;
     static constexpr int TCOLS = 9 * COUT <= 256 ? 256 : 512;
     static constexpr int NOUT = 27 * CIN * COUT + COUT;    // weights, then biases
-    static_assert(SLOTG <= 16, "the constant group lies inside the 128 operand rows");
+    static_assert(SLOTG <= 16, "a plane's groups lie inside the 128 operand rows");
 };
 
 template <int CIN, int COUT>
@@ -681,11 +686,6 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
         tc::mbar_fence_init();
     }
     if (t < 32) tc::tmem_alloc(&tslot, WM::TCOLS);
-    for (int i = t; i < kWRing * kHY * 8; i += kZThreads) {  // channel 0 = 1.0 in BF16
-        const int slot = i / (kHY * 8), u = i % (kHY * 8);
-        *reinterpret_cast<uint4*>(sm + slot * SLOT + 3 * KGN * WM::GROUP + u * 16) = make_uint4(0x3F80u, 0, 0, 0);
-    }
-    tc::fence_smem_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -696,15 +696,48 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
     const bool worker = t < kZWorkers;
     const int bx = g.nx / 8;
     const int64_t ntiles = (int64_t)bx * (g.ny / 16) * g.nz;
-    int64_t tile = ntiles * blockIdx.x / gridDim.x;
+    const int64_t tile0 = ntiles * blockIdx.x / gridDim.x;  // gridDim.x <= ntiles: no share is empty
     const int64_t tile1 = ntiles * (blockIdx.x + 1) / gridDim.x;
+    const int64_t mid = tile0 + (tile1 - tile0 + 1) / 2;
+    int64_t tile = tile0;
     int n = 0;  // tiles issued by this block
     bool ok = true;
+    float* const dst = partials + (int64_t)blockIdx.x * WM::NOUT;
+    // The accumulators into this block's partials, or added to them (workers).
+    // Lane m of an accumulator: channel group m / 8, channel m % 8; warps w and
+    // w + 4 read the same lanes and take alternate accumulators.
+    auto flush = [&](bool add) {
+        const int w = t >> 5, m = t & 127, gr = m / 8;
+        const int dx = gr / KGN, ci = (gr % KGN) * 8 + m % 8;
+        for (int gi = w >> 2; gi < 9; gi += 2) {
+            float v[COUT];
+#pragma unroll
+            for (int c0 = 0; c0 < COUT; c0 += 16)
+                tc::tmem_ld16(tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(gi * COUT + c0), v + c0);
+            if (gr < 3 * KGN) {
+                float4* o = reinterpret_cast<float4*>(dst + ((gi * 3 + dx) * CIN + ci) * COUT);
+#pragma unroll
+                for (int q = 0; q < COUT / 4; ++q) {
+                    float4 s = add ? o[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    s.x += v[4 * q];
+                    s.y += v[4 * q + 1];
+                    s.z += v[4 * q + 2];
+                    s.w += v[4 * q + 3];
+                    o[q] = s;
+                }
+            }
+            __syncwarp();  // the next load is a whole warp's
+        }
+    };
+    // Bias gradient: warp w sums channel group w % NG of a gradient tile
+    constexpr int NG = COUT / 8, BC = (kZWorkers / 32) / NG;  // groups; warps per group
+    float bsum[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     while (tile < tile1 && ok) {
         // one column segment: planes [za, za + len)
         const int64_t col = tile / g.nz;
         const int za = (int)(tile - col * g.nz);
-        const int len = (int)min((int64_t)(g.nz - za), tile1 - tile);
+        const int len = (int)min((int64_t)(g.nz - za), (tile < mid ? mid : tile1) - tile);
+        const bool fresh = tile == tile0 || tile == mid;  // starts new sums
         const int x0 = (int)(col % bx) * 8, y0 = (int)(col / bx) * 16;
         // plane za + r (-1 <= r <= len) into slot (r + 1) % ring, gradient tile
         // za + r into slot r % 3
@@ -741,6 +774,10 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
                     load_grad(1);
                 }
                 asm volatile("cp.async.commit_group;\n" ::: "memory");
+                if (fresh && n > 0) {  // the first half's sums are final
+                    tc::fence_after_sync();
+                    flush(false);
+                }
                 asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             }
             tc::fence_smem_async();
@@ -762,11 +799,24 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks)
                         tc::mma_bf16(tmem + gi * COUT, da0 + (uint32_t)(ks * 256 / 16), db0 + (uint32_t)(ks * 256 / 16),
-                                     idesc, (n > 0 || ks > 0) ? 1u : 0u);
+                                     idesc, (!fresh || i > 0 || ks > 0) ? 1u : 0u);
                 }
                 tc::mma_commit(&bar[n & 1]);
             }
             if (worker) {
+                // this tile's gradient was complete at the last barrier and keeps its
+                // slot until the next one
+                const unsigned char* D = Gs + (i % kWGrads) * WM::GB + ((t >> 5) % NG) * 2048;
+                for (int k = (t >> 5) / NG * 32 + (t & 31); k < kTileM; k += 32 * BC) {
+                    const uint4 u = *reinterpret_cast<const uint4*>(D + k * 16);
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 f = __bfloat1622float2(h[j]);
+                        bsum[2 * j] += f.x;
+                        bsum[2 * j + 1] += f.y;
+                    }
+                }
                 // tile n - 1 done: plane i - 2 (its slot takes plane i + 3) and
                 // the gradient of tile i - 1 are no longer read
                 if (n > 0) lost = !tc::mbar_wait(&bar[(n - 1) & 1], ((n - 1) >> 1) & 1, err, wait_limit);
@@ -795,31 +845,21 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
         ok = !__syncthreads_or(lost);
     }
     tc::fence_after_sync();
+    __shared__ float bsh[kZWorkers / 32][8];
     if (ok && worker) {
-        // lane m of an accumulator: channel group m / 8, channel m % 8; warps w
-        // and w + 4 read the same lanes and take alternate accumulators
-        const int w = t >> 5, m = t & 127, gr = m / 8;
-        const int dx = gr / KGN, ci = (gr % KGN) * 8 + m % 8;
-        float* dst = partials + (int64_t)blockIdx.x * WM::NOUT;
-        for (int gi = w >> 2; gi < 9; gi += 2) {
-            float v[COUT];
-            if (n == 0) {
+        flush(mid < tile1);
 #pragma unroll
-                for (int co = 0; co < COUT; ++co) v[co] = 0.0f;  // no tiles: zero partial
-            } else {
-#pragma unroll
-                for (int c0 = 0; c0 < COUT; c0 += 16)
-                    tc::tmem_ld16(tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(gi * COUT + c0), v + c0);
-            }
-            float* o = nullptr;
-            if (gr < 3 * KGN) o = dst + ((gi * 3 + dx) * CIN + ci) * COUT;
-            else if (gi == 4 && m == 24 * KGN) o = dst + 27 * CIN * COUT;  // the constant row, undisplaced
-            if (o) {
-#pragma unroll
-                for (int co = 0; co < COUT; co += 4)
-                    *reinterpret_cast<float4*>(o + co) = make_float4(v[co], v[co + 1], v[co + 2], v[co + 3]);
-            }
+        for (int j = 0; j < 8; ++j) {
+            float v = bsum[j];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if ((t & 31) == 0) bsh[t >> 5][j] = v;
         }
+    }
+    __syncthreads();
+    if (ok && t < COUT) {
+        float v = 0.0f;
+        for (int w = t / 8; w < kZWorkers / 32; w += NG) v += bsh[w][t % 8];
+        dst[27 * CIN * COUT + t] = v;
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");  // no copy outlives the block
     if (t == 0) {  // drain: the newest commit on each barrier
