@@ -233,19 +233,27 @@ int default_zchunk(int nx, int ny, int nz, int tcx, int tcy, int num_sms) {
 // Largest box (cells) an untuned AUTO handle steps with the point kernels
 // (qpoint.cuh): they index 15 V in 32 bits.  Below that they were the faster
 // ones at every size tried.  Whole steps on B200, z-marching kernels -> these:
-//   FP64             32^3 67 -> 8 us, 256^3 2865 -> 2100 us
+//   FP64             32^3 67 -> 8 us, 256^3 2865 -> 2070 us
 //   FP32, one point  64x256x256 slit 282 -> 243 us, 256^3 slit 981 -> 834 us,
 //                    301x300x300 channel 2914 -> 1766 us
-//   FP32, packed     128^3 139 -> 126 us, 256^3 944 -> 803 us, 512x512x256
-//                    3547 -> 3216 us
-//   FP16, packed     256^3 844 -> 664 us, 512x512x256 3136 -> 2745 us
+//   FP32, packed     240x160x165 350 -> 310 us, 256^3 909 -> 784 us, 512x512x256
+//                    3470 -> 3162 us, 512^3 6918 -> 6423 us
+//   FP16, packed     240x240x60 189 -> 161 us, 256^3 811 -> 704 us, 512x512x256
+//                    3055 -> 2848 us
 constexpr int64_t kPointCells = (((int64_t)1 << 31) - 1) / 15;
 
-// FP64: up to this size the LBM kernel forms the body force itself (one launch
-// and the force's round trip less); above it a force kernel runs before the LBM
-// step.  FP32 forms it there at every size
-// (256^3 slit, a force kernel / formed there: 858 / 834 us, FP16 801 / 746 us).
+// FP64 boxes with z walls or anchoring (whose kernels carry every wall rule)
+// form the body force in a kernel of its own above this size: 200^3 1485 us per
+// step, 1533 us with the force formed by the LBM kernel.  All others form it
+// there, a launch and the force's round trip less: FP64 200^3 1001 us for 1073,
+// 256^3 2070 for 2216, 256^3 slit 2165 for 2343, 301x200x150 channel 1300 for
+// 1333; FP32 256^3 slit 834 for 858.
 constexpr int64_t kPointFusedCells = (int64_t)6 << 20;
+bool force_apart(const SimParams& P) {
+    bool general = !(P.qper[4] && P.qper[5] && P.uper[4] && P.uper[5]);
+    for (const Face& f : P.face) general = general || f.qbc == Q_ANCHORING;
+    return general && P.V > kPointFusedCells;
+}
 
 // Memory (words per cell) a handle must leave free when it takes the point
 // kernels' scratch: the buffers it may ask for later (second population buffer,
@@ -446,7 +454,9 @@ int lbman_create(const lbman_config* cfg, lbman_solver** out) {
     // tried, and the two-points-per-thread Q kernel is the faster of the two
     // where its 30-wide tiles pad x by at most 10% (512^3: 19.3 against 18.2
     // GLUPS untuned); so those are the defaults until lbman_autotune says
-    // otherwise.
+    // otherwise.  The point kernels have no tiles, but take their arithmetic
+    // (one point or packed) from the same rule, so that a box has the same bits
+    // with and without them.
     int kern = cfg->kernels;
     if (kern == LBMAN_KERNELS_AUTO) {
         const bool pair_fits = cfg->precision != LBMAN_FP64 && cfg->nx % 4 == 0 && cfg->tile_x == 0 &&
@@ -757,7 +767,7 @@ static int one_step(lbman_solver* s, bool last) {
         s->ucur ^= 1;
         s->fcur ^= 1;
         s->fphase = F_POST;
-    } else if (s->point && (s->prec != LBMAN_FP64 || s->P.V <= kPointFusedCells)) {
+    } else if (s->point && (s->prec != LBMAN_FP64 || !force_apart(s->P))) {
         LB_TRY(q_stage(s, false));
         LB_TRY(aa_layout(s));
         const bool odd = s->fphase == F_SWAP;
