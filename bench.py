@@ -162,21 +162,46 @@ def time_device(sim, steps, warmup, stream):
     return e0.elapsed_time(e1), sim.launch_count() - l0
 
 
-def kernel_breakdown(sim, kernels, precision, V, stream, n):
+POINT_CELLS = (2 ** 31 - 1) // 15    # largest box the shared-memory-free kernels index
+LONG_WALK_PLANE = 1 << 15            # packed FP32: planes on which the update finishes the force's z terms
+
+
+def steps_without_shared_memory(shape, own, auto, V):
+    """Does a handle step with the shared-memory-free kernels?  An AUTO handle
+    that can names them by the shape it was created with."""
+    return auto and V <= POINT_CELLS and all(shape[k] == own[k] for k in ("kernels", "tile_x", "tile_y", "zchunk"))
+
+
+def point_bytes_per_cell(precision, packed, plane):
+    """Bytes the shared-memory-free step must move per cell: Q and u in, Q_new,
+    the stress and the local force out; these, the populations and u in the
+    LBM kernel."""
+    rb = 8 if precision == "fp64" else 4
+    sb = {"fp64": 8, "fp32": 4, "fp16": 2}[precision]
+    if precision == "fp64":
+        return rb * (8 + 5 + 8 + 3) + rb * (8 + 5 + 3 + 3) + 30 * sb + 3 * rb
+    stress, u = (6, 0) if packed and precision == "fp32" and plane >= LONG_WALK_PLANE else (9, 3)
+    return rb * (8 + 5 + stress + 3) + rb * (stress + 3 + u) + 30 * sb + 3 * rb
+
+
+def kernel_breakdown(sim, kernels, precision, V, stream, n, plane=0, packed=False):
     """Average duration of each kernel of the step, CUDA events around each
     launch on the solver's stream, with the algorithmic bytes per cell each
-    one must move (state words read + written, body force included)."""
+    one must move (state words read + written, body force included).  The two
+    kernels of the shared-memory-free step overlap at their ends and run only
+    together, so they are one entry, as the fused kernel is."""
     import torch
     rb = 8 if precision == "fp64" else 4
     sb = {"fp64": 8, "fp32": 4, "fp16": 2}[precision]
-    if kernels == "fused":
+    if kernels in ("fused", "point"):
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         sim.step(2)
         e0.record(stream)
         sim.step(n)
         e1.record(stream)
         e1.synchronize()
-        return {"fused_step": {"ms": e0.elapsed_time(e1) / n, "bytes_per_cell": 30 * sb + 16 * rb}}
+        nbytes = 30 * sb + 16 * rb if kernels == "fused" else point_bytes_per_cell(precision, packed, plane)
+        return {f"{kernels}_step": {"ms": e0.elapsed_time(e1) / n, "bytes_per_cell": nbytes}}
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True),
            torch.cuda.Event(enable_timing=True)) for _ in range(n)]
     sim.step(2)
@@ -640,13 +665,16 @@ def main():
     tile = tuple(int(v) for v in a.tile.split(",")) if a.tile else None
     sim, p = make_sim(a.workload, a.precision, local, a.kernels, tile)
     sim.set_stream(stream.cuda_stream)
-    if a.kernels == "auto" and not tile:
+    auto, own = a.kernels == "auto" and not tile, sim.shape()
+    if auto:
         sim.init_seeded(SEED, S0, SIGMA)
         tuned = sim.autotune(steps_per_trial=8 if V > 5e7 else 10)
         config["autotuned"] = {k: tuned[k] for k in ("kernels", "tile_x", "tile_y", "zchunk", "trials")}
     sh = sim.shape()
     config["kernels"] = {1: "split", 2: "fused", 3: "split_pair"}[sh["kernels"]]
     config["tile"] = [sh["tile_x"], sh["tile_y"], sh["zchunk"]]
+    if steps_without_shared_memory(sh, own, auto, V):
+        config["kernels"] = "point"  # the tile is that of the z slabs below
     if world > 1:
         dist.barrier()
     torch.cuda.synchronize()
@@ -658,7 +686,8 @@ def main():
     peak, peak_kind = measured_peaks()
     bpc = BYTES_PER_CELL[a.precision]
     step_achieved = bpc * V / (ms_step * 1e-3) / 1e9
-    kern = kernel_breakdown(sim, config["kernels"], a.precision, V, stream, 30 if V > 5e7 else 200)
+    kern = kernel_breakdown(sim, config["kernels"], a.precision, V, stream, 30 if V > 5e7 else 200, nx * ny,
+                            sh["kernels"] == 3)
     dom = max(kern, key=lambda k: kern[k]["ms"])
     achieved = kern[dom]["bytes_per_cell"] * V / (kern[dom]["ms"] * 1e-3) / 1e9
     for k in kern:
@@ -704,7 +733,7 @@ def main():
         line["other_workloads"] = side_workloads([w for w in ("slit64", "channel20") if w != a.workload], local,
                                                  stream)
         line["ensemble"] = ensemble_vs_sequential(local, stream)
-        kern_id = {"split": 1, "split_pair": 3}.get(config["kernels"], 1)
+        kern_id = sh["kernels"] if sh["kernels"] != 2 else 1
         line["slab_split"] = slab_split(a.workload, a.precision, local, stream, kern_id, tuple(config["tile"]))
         line["slab_split"]["vs_single_box"] = line["slab_split"]["value"] / mlups
         torch.cuda.empty_cache()
