@@ -4,8 +4,10 @@
 // Every box is described by an EnsBox in device memory (its own SimParams
 // and field pointers).  The host flattens all boxes into work lists, and each
 // launch covers every box, running the code of the single-box kernels on the
-// item's box, so the results are the single-box ones bit for bit.  There is no
-// communication between boxes.
+// item's box: one point per thread, so the results are bit for bit those of a
+// single box with the one-point kernels (FP64, LBMAN_KERNELS_SPLIT, and AUTO
+// where its 30-wide tiles do not fit; the packed arithmetic of the other FP32 and
+// FP16 boxes rounds differently).  There is no communication between boxes.
 //
 //   split   ens_qpoint_kernel, then ens_lbm_point_kernel (the time step of
 //           qpoint.cuh, in-place streaming): one block per work item;

@@ -35,12 +35,13 @@ constexpr int kMaxGridY = 65535;
 
 // Planes per thread (a power of two): the longest walk that still gives every
 // SM a few blocks.  At most 4 planes, where the gain of reusing the centre
-// values ends, and 16 blocks per SM; packed kernels on planes with long walks
-// (long_walks), where a walk also saves the z terms' trip through memory, at
-// most 16 planes and 6 blocks per SM.  Steps with 1 / 2 / 4 / 8 / 16 planes there:
-// 128^3 138 / 135 / 131 / 127 / 131 us (the rule: 8), 160^3 274 / 261 / 254 / 249 /
-// 247 us (16).  A box of so many planes that its chunks would pass the launch's y
-// dimension walks further.
+// values ends, and 16 blocks per SM; packed kernels on planes of 2^15 cells and
+// more (long_walks), where the walk prefetches and in FP32 saves the z terms' trip
+// through memory, at most 16 planes and 6 blocks per SM.  FP32 steps with walks
+// of at most 4 / 8 / 16 planes there: 256x256x64 226 / 220 / 217 us, 240x160x165
+// 356 / 331 / 331 us, 256^3 909 / 855 / 840 us, 512x512x128 1780 / 1680 / 1670 us.
+// A box of so many planes that its chunks would pass the launch's y dimension
+// walks further.
 inline int point_walk(const SimParams& P, bool pair, int num_sms) {
     const bool longer = pair && long_walks(P);
     const int per_block = kPointThreads * (pair ? 2 : 1);

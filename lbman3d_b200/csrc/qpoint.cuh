@@ -13,32 +13,35 @@
 //                        collide-and-stream, so it never goes to memory.
 //
 // The arithmetic is that of the z-marching kernels, value for value (what those
-// keep in shared memory is what qpoint_kernel stores), so both organisations
-// give the same bits.
+// keep in shared memory is what qpoint_kernel stores): one point per thread as
+// qforce.cuh, packed as qpair.cuh, each with the bits of its counterpart.
 //
 // A thread of qpoint_kernel walks a chunk of planes of one (x, y) column and
 // keeps the centre values of three planes in registers, so a plane costs its x
 // and y neighbours (first-level cache) and one new centre value per field.  No
 // point is updated twice and no warp waits for another; the price is the
 // stress's trip through the second-level cache, or HBM for large boxes.  The
-// packed kernels
-// (qpoint2_kernel) on planes with long walks (long_walks, qpair.cuh) finish the z
-// terms of the force in the walk, for all but a chunk's first and last plane:
-// per cell 6 stress words and 3 of force go to the LBM kernel instead of 9
-// stress words, 3 of Ericksen force and the 3 of the old velocity.
+// packed FP32 kernels (qpoint2_kernel) on planes with long walks (force_in_walk,
+// qpair.cuh) finish the z terms of the force in the walk, for all but a chunk's
+// first and last plane: per cell 6 stress words and 3 of force go to the LBM
+// kernel instead of 9 stress words, 3 of Ericksen force and the 3 of the old
+// velocity.
 //
 // What bounds it: launches below about 10^5 cells, registers and latency up to
-// a few 10^6 (12-20 warps per SM), then HBM: packed on long walks 94 B per cell in
-// the update (256^3: 298 us against a 244 us floor; 330 us without the prefetch,
-// 318 us with 4-plane walks) and 174 B in the LBM step (449 / 490 us even / odd
-// against 440 us; FP16 storage 114 B, 323 / 379 us against 290 us), and, in
-// FP64, the FP64 pipe.  Whole steps before (z-marching Q kernel, then LBM) and
-// with these kernels:
-//   32^3 FP64             67 ->  8 us      20x100x100 FP64    150 -> 26 us
-//   67x101x131 FP32      161 ->  61 us     64^3 FP32           39 -> 16 us
-//   64x256x256 slit FP32 282 -> 243 us     same, FP64         898 -> 515 us
-//   256^3 slit FP32      981 -> 834 us     256^3 FP64        2865 -> 2100 us
-//   256^3 FP32 / FP16    944 -> 803, 844 -> 664 us
+// a few 10^6 (11-18 warps per SM in the update), then HBM.  256^3 packed, DRAM
+// bytes per cell as counted and the time they take at the copy rate (6463 GB/s):
+//   FP32 update 90 B, 298 us for 234 (11 warps per SM; 330 us without the
+//     prefetch, 318 us with 4-plane walks); LBM 168 B, 449 / 490 us even / odd
+//     for 436 (the odd step's x-shifted accesses are unaligned)
+//   FP16 update 98 B, 309 us for 255; LBM 130 B, 348 / 397 us for 337
+// FP64 (64x256x256 slit): update 179 B, 192 us for 116, the FP64 pipe 62% active;
+// LBM 406 B, 266 / 305 us for 263.  Whole steps before (z-marching Q kernel, then
+// LBM) and with these kernels:
+//   32^3 FP64             67 ->  8 us      20x100x100 FP64    150 -> 23 us
+//   67x101x131 FP32      161 ->  60 us     64^3 FP32           39 -> 16 us
+//   64x256x256 slit FP32 282 -> 244 us     same, FP64         898 -> 490 us
+//   256^3 slit FP32      981 -> 834 us     256^3 FP64        2865 -> 2070 us
+//   256^3 FP32 / FP16    909 -> 784, 811 -> 704 us
 #pragma once
 
 #include "lbm.cuh"

@@ -129,6 +129,8 @@ __device__ __forceinline__ int qx_off(int a, int n, int per_lo, int per_hi) {
 // next plane's values are loaded while this one is worked on.  256^3 FP32:
 // 331 us one thread per cell, 252 us now at 3 blocks per SM (293 at 2, 294 at
 // 4, which spills); FP64, which converts nothing: 343-352 us at 2 blocks, 369 at 3.
+// Neither HBM (1.4 TB/s) nor the FP64 pipe (29% active) bounds it: issue slots are
+// 55% used, at 23 warps per SM and one barrier per plane.
 constexpr int kEnX = 32, kEnY = 8;
 static_assert(kEnX * kEnY == kRedThreads, "one thread per column of a tile");
 template <class R>
