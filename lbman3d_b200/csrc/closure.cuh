@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(kThreads) wgrad_kernel(Grid3 g, const __nv_bfl
 // summed by the copying warps from the staged tiles in FP32.  Error against 64
 // bits at 80^3, of the sum of the terms' magnitudes, weights / biases: 1.8e-6 /
 // 7e-8; whole shares with the biases as a row of the product 5.0e-6 / 4.4e-7, in
-// 57 us for the 72 us a 32 -> 32 layer takes at 64^3.
+// 57 us for the 64 us a 32 -> 32 layer takes at 64^3.
 constexpr int kWRing = 5, kWGrads = 3;
 template <int CIN, int COUT>
 struct WGradMarch {
@@ -703,27 +703,26 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
     int n = 0;  // tiles issued by this block
     bool ok = true;
     float* const dst = partials + (int64_t)blockIdx.x * WM::NOUT;
-    // The accumulators into this block's partials, or added to them (workers).
-    // Lane m of an accumulator: channel group m / 8, channel m % 8; warps w and
-    // w + 4 read the same lanes and take alternate accumulators.
+    // The accumulators into this block's partials (MarchOrder), or added to them
+    // (workers).  Warps w and w + 4 read the same lanes and take alternate
+    // accumulators.
     auto flush = [&](bool add) {
-        const int w = t >> 5, m = t & 127, gr = m / 8;
-        const int dx = gr / KGN, ci = (gr % KGN) * 8 + m % 8;
+        const int w = t >> 5, m = t & 127;
         for (int gi = w >> 2; gi < 9; gi += 2) {
             float v[COUT];
 #pragma unroll
             for (int c0 = 0; c0 < COUT; c0 += 16)
                 tc::tmem_ld16(tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(gi * COUT + c0), v + c0);
-            if (gr < 3 * KGN) {
-                float4* o = reinterpret_cast<float4*>(dst + ((gi * 3 + dx) * CIN + ci) * COUT);
+            if (m < 3 * CIN) {
+                float4* o = reinterpret_cast<float4*>(dst) + gi * (COUT / 4) * 3 * CIN + m;
 #pragma unroll
                 for (int q = 0; q < COUT / 4; ++q) {
-                    float4 s = add ? o[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    float4 s = add ? o[q * 3 * CIN] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     s.x += v[4 * q];
                     s.y += v[4 * q + 1];
                     s.z += v[4 * q + 2];
                     s.w += v[4 * q + 3];
-                    o[q] = s;
+                    o[q * 3 * CIN] = s;
                 }
             }
             __syncwarp();  // the next load is a whole warp's
@@ -871,12 +870,28 @@ __global__ void __launch_bounds__(kZThreads) wgrad_march_kernel(Grid3 g, const _
     if (t < 32) tc::tmem_dealloc(tmem, WM::TCOLS);
 }
 
-// out[j] = sum over p < P of partials[p * n + j] in a fixed order: a block
+// Order of a block's partials: the gradient's own, [tap][ci][co] and then the
+// biases, or wgrad_march_kernel's, where the lanes of an accumulator store
+// neighbouring float4: accumulator (dy, dz), 4 columns, lane (dx, ci), column.
+struct GradOrder {
+    __device__ __forceinline__ int operator()(int j) const { return j; }
+};
+template <int CIN, int COUT>
+struct MarchOrder {
+    __device__ __forceinline__ int operator()(int j) const {
+        if (j >= 27 * CIN * COUT) return j;
+        const int e = j % 4, m = j / 4 % (3 * CIN), k = j / (12 * CIN), q = k % (COUT / 4), gi = k / (COUT / 4);
+        return ((gi * 3 + m / CIN) * CIN + m % CIN) * COUT + 4 * q + e;
+    }
+};
+
+// out[order(j)] = sum over p < P of partials[p * n + j] in a fixed order: a block
 // takes 32 consecutive j; its warp s sums the partials p = s, s + 8, ... in
 // increasing p, then the 8 slice sums are added in increasing s.  (One
 // thread per j summing all P serially left most SMs idle.)  Launch with
 // kFoldThreads threads and ceil(n / 32) blocks.
 constexpr int kFoldThreads = 256;
+template <class Order>
 __global__ void __launch_bounds__(kFoldThreads) sum_partials_kernel(const float* partials, int P, int n,
                                                                      float* __restrict__ out) {
     __shared__ float slice[kFoldThreads / 32][32];
@@ -892,7 +907,7 @@ __global__ void __launch_bounds__(kFoldThreads) sum_partials_kernel(const float*
         float t = slice[0][lane];
 #pragma unroll
         for (int k = 1; k < kFoldThreads / 32; ++k) t += slice[k][lane];
-        out[j] = t;
+        out[Order()(j)] = t;
     }
 }
 

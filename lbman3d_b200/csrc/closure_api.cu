@@ -192,7 +192,7 @@ int run_wgrad(lbman_closure* c, cudaStream_t st, const __nv_bfloat16* a, const _
         const int grid = (int)std::min<int64_t>(c->num_sms, c->V / cl::kTileM);
         CL_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, WM::SMEM));
         CL_CUDA(launch_dependent(K, dim3(grid), cl::kZThreads, WM::SMEM, st, g3, a, gr, c->wpart, c->err, c->wait_limit));
-        CL_CUDA(launch_dependent(cl::sum_partials_kernel, dim3((WM::NOUT + 31) / 32), cl::kFoldThreads, 0, st,
+        CL_CUDA(launch_dependent(cl::sum_partials_kernel<cl::MarchOrder<CIN, COUT>>, dim3((WM::NOUT + 31) / 32), cl::kFoldThreads, 0, st,
                                  (const float*)c->wpart, grid, (int)WM::NOUT, c->g + w_off(layer)));
         return LBMAN_OK;
     }
@@ -201,11 +201,11 @@ int run_wgrad(lbman_closure* c, cudaStream_t st, const __nv_bfloat16* a, const _
     CL_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, WS::SMEM));
     K<<<c->Gw, cl::kThreads, WS::SMEM, st>>>(g3, a, gr, c->wpart, c->err, c->wait_limit);
     CL_CUDA(cudaGetLastError());
-    cl::sum_partials_kernel<<<(n + 31) / 32, cl::kFoldThreads, 0, st>>>(c->wpart, c->Gw, n, c->g + w_off(layer));
+    cl::sum_partials_kernel<cl::GradOrder><<<(n + 31) / 32, cl::kFoldThreads, 0, st>>>(c->wpart, c->Gw, n, c->g + w_off(layer));
     CL_CUDA(cudaGetLastError());
     cl::bias_grad_kernel<COUT><<<c->Gb, cl::kThreads, 0, st>>>(gr, c->V, c->bpart);
     CL_CUDA(cudaGetLastError());
-    cl::sum_partials_kernel<<<(COUT + 31) / 32, cl::kFoldThreads, 0, st>>>(c->bpart, c->Gb, COUT, c->g + b_off(layer));
+    cl::sum_partials_kernel<cl::GradOrder><<<(COUT + 31) / 32, cl::kFoldThreads, 0, st>>>(c->bpart, c->Gb, COUT, c->g + b_off(layer));
     CL_CUDA(cudaGetLastError());
     return LBMAN_OK;
 }
